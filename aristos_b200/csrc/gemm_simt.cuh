@@ -1,9 +1,8 @@
 // Expert-FFN GEMM on the FP32 pipes: 128x128x16 block tile, 256 threads, 8x8 register tile.
 //
-// This is the path for torch_dtype 0 (float): the reference also runs float on scalar FMA,
-// not on tensor cores (os/processor/mmaConfig.cuh:19-26), and fp32 FMA is what keeps the
-// layer output within 1e-5 of the fp64 oracle.  It is also instantiated for bf16 as a
-// debugging cross-check of the tensor-core kernel.
+// The reference runs float layers this way, on scalar FMA and not on tensor cores
+// (os/processor/mmaConfig.cuh:19-26).  Here it is the cross-check of the tensor-core kernels, for every
+// element type, selected with KLEOS_DEBUG_SIMT_GEMM=1.
 #pragma once
 
 #include "gemm_common.cuh"

@@ -22,6 +22,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include "config.hpp"
+#include "gemm_f32.cuh"
 #include "gemm_simt.cuh"
 #include "gemm_tc2.cuh"
 #include "gemm_tf32.cuh"
@@ -54,6 +55,8 @@ struct State {
     uint32_t epoch = 0;
     long long wait_cycles = 20000000000LL;  // about ten seconds of SM clock (ranks may start far apart)
     bool use_tc = false;       // 16-bit layers: tcgen05 router and FFN GEMMs
+    bool use_f32_tc = false;   // float layers: tcgen05 FFN GEMMs on split operands (the router stays on FP32 FMA)
+    int f32_bn[2] = {};        // ... and their tile widths
     bool use_tf32_tc = false;  // TF32 layers: tcgen05 kind::tf32 FFN GEMMs (the router stays on FP32 FMA)
     // num_experts == 1: the layer is a plain FFN over this rank's tokens (the reference switches
     // to its fffn kernel, moe/moe.cuh:174-177,197-204): no gate, no exchange, and the packed
@@ -292,11 +295,20 @@ Sections slice(const void* iP, void* oP) {
 }
 
 int ensure_maps(const Sections& s) {
-    if ((!g.use_tc && !g.use_tf32_tc) || g.maps_for_iP == s.A) return KLEOS_OK;
+    if ((!g.use_tc && !g.use_tf32_tc && !g.use_f32_tc) || g.maps_for_iP == s.A) return KLEOS_OK;
     const LayerConfig& c = g.cfg;
     // the dense layer multiplies the activations where they lie: S rows instead of the cells
     const uint64_t cell_rows = g.dense ? (uint64_t)c.S : (uint64_t)g.world * g.nLx * c.pEC;
     int rc;
+    if (g.use_f32_tc) {
+        const uint32_t rk = gemm_f32::BK;
+        if ((rc = make_map(&g.map_x, g.dense ? s.A : g.arena + g.lay.xcell, cell_rows, c.H, gemm_f32::BM, rk))) return rc;
+        if ((rc = make_map(&g.map_w1, s.W1, (uint64_t)g.nLx * c.I, c.H, g.f32_bn[0] / 2, rk))) return rc;
+        if ((rc = make_map(&g.map_y1, g.y1, cell_rows, c.I, gemm_f32::BM, rk))) return rc;
+        if ((rc = make_map(&g.map_w2, s.W2, (uint64_t)g.nLx * c.H, c.I, g.f32_bn[1] / 2, rk))) return rc;
+        g.maps_for_iP = s.A;
+        return KLEOS_OK;
+    }
     if (g.use_tf32_tc) {
         const uint32_t bk = gemm_tf32::BK;
         if ((rc = make_map(&g.map_x, g.dense ? s.A : g.arena + g.lay.xcell, cell_rows, c.H, gemm_tf32::BM, bk))) return rc;
@@ -379,6 +391,25 @@ void launch_tf32(int epi, cudaStream_t st, const CUtensorMap& map_a, const CUten
     else { ++g.launches; ffn_gemm_tf32<2><<<grid, 256, smem, st>>>(map_a, map_b, ga); }
 }
 
+// Float layers: tile width of the split-operand GEMM with N output columns: the one whose rounds of
+// tiles over the block pairs take least time, with the rows an expert gets when the tokens spread
+// evenly.  A 32-wide K slice took 1400 cycles at 128 columns and 950 at 64 (4096 tokens, 16 experts,
+// H = I = 2048: 368 and 490 us per launch; 256 tokens, 8 experts, 512 columns: 40 and 32 us).
+int f32_tile_width(int N) {
+    const LayerConfig& c = g.cfg;
+    const long long rows = g.dense ? c.S : std::min<long long>((long long)g.world * c.EC, ((long long)c.S * c.K + g.nLx - 1) / g.nLx);
+    const long long pairs = (long long)g.nLx * ((rows + 2 * kTileM - 1) / (2 * kTileM)), clusters = g.sm_count / 2;
+    auto cost = [&](int width, int cycles) { return (pairs * ((N + width - 1) / width) + clusters - 1) / clusters * cycles; };
+    return cost(128, 1400) <= cost(64, 950) ? 128 : 64;
+}
+
+void launch_f32(int bn, cudaStream_t st, const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmArgs& ga) {
+    const int grid = g.sm_count & ~1, thr = gemm_f32::kThreads;
+    ++g.launches;
+    if (bn == 128) ffn_gemm_f32<128><<<grid, thr, gemm_f32::Shape<128>::SMEM_BYTES, st>>>(map_a, map_b, ga);
+    else ffn_gemm_f32<64><<<grid, thr, gemm_f32::Shape<64>::SMEM_BYTES, st>>>(map_a, map_b, ga);
+}
+
 // Optional replacement of the activation input and the layer-output destination of one
 // forward (used by the pipelined host path, whose staging buffers live outside iP / oP).
 struct Staging {
@@ -424,6 +455,10 @@ int forward_dense(const Sections& s, const CUtensorMap* map_a, cudaStream_t st, 
         launch_tf32(c.hidden_act, st, *map_a, g.map_w1, g1);
         KLEOS_CUDA(mark());
         launch_tf32(2, st, g.map_y1, g.map_w2, g2);
+    } else if (g.use_f32_tc) {
+        launch_f32(g.f32_bn[0], st, *map_a, g.map_w1, g1);
+        KLEOS_CUDA(mark());
+        launch_f32(g.f32_bn[1], st, g.map_y1, g.map_w2, g2);
     } else {
         { ++g.launches; ffn_gemm_simt<T><<<g.sm_count * 2, 256, 0, st>>>(g1); }
         KLEOS_CUDA(mark());
@@ -602,6 +637,11 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
         KLEOS_CUDA(mark());
         launch_tf32(2, st, g.map_y1, g.map_w2, g2);
         KLEOS_CUDA(mark());
+    } else if (g.use_f32_tc) {
+        launch_f32(g.f32_bn[0], st, g.map_x, g.map_w1, g1);
+        KLEOS_CUDA(mark());
+        launch_f32(g.f32_bn[1], st, g.map_y1, g.map_w2, g2);
+        KLEOS_CUDA(mark());
     } else {
         { ++g.launches; ffn_gemm_simt<T><<<g.sm_count * 2, 256, 0, st>>>(g1); }
         KLEOS_CUDA(mark());
@@ -698,8 +738,8 @@ int ensure_host_pipe() {
         if (g.use_tc && c.PX <= 128) {
             int rc = make_map(&hp.map_act[b], hp.act[b], c.S, c.H, route_tc::BM);
             if (rc) return rc;
-        } else if (g.use_tf32_tc && (g.dense || c.PX <= 128)) {
-            // same box (128 rows x 32 words) serves the tf32 router and the dense layer's GEMM1
+        } else if ((g.use_tf32_tc && (g.dense || c.PX <= 128)) || (g.use_f32_tc && g.dense)) {
+            // same box (128 rows x 32 words) serves the tf32 router and the dense layers' GEMM1
             int rc = make_map(&hp.map_act[b], hp.act[b], c.S, c.H, gemm_tf32::BM, gemm_tf32::BK);
             if (rc) return rc;
         }
@@ -850,6 +890,7 @@ static int initialize_impl(const char* config_json_path, int rank, int world, co
     }
     const char* simt = std::getenv("KLEOS_DEBUG_SIMT_GEMM");
     g.use_tc = (cfg.torch_dtype == 2 || cfg.torch_dtype == 3) && !(simt && simt[0] == '1');
+    g.use_f32_tc = cfg.torch_dtype == 0 && !(simt && simt[0] == '1');
     g.use_tf32_tc = cfg.torch_dtype == 1 && !(simt && simt[0] == '1');
 
     const size_t eb = cfg.elem_bytes;
@@ -897,6 +938,13 @@ static int initialize_impl(const char* config_json_path, int rank, int world, co
         if (cfg.torch_dtype == 2) rc = set_tc_attributes<__nv_bfloat16>();
         else rc = set_tc_attributes<__half>();
         if (rc) return rc;
+    }
+    if (g.use_f32_tc) {
+        const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_f32<64>, dyn, gemm_f32::Shape<64>::SMEM_BYTES));
+        KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_f32<128>, dyn, gemm_f32::Shape<128>::SMEM_BYTES));
+        g.f32_bn[0] = f32_tile_width(cfg.I);
+        g.f32_bn[1] = f32_tile_width(cfg.H);
     }
     if (g.use_tf32_tc) {
         const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;

@@ -46,7 +46,7 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, uint32_t pari
     }
     return true;
 }
-// Same, adding the cycles spent waiting to *acc (used by the optional per-role stall counters).
+// mbar_wait, adding the cycles spent waiting to *acc (used by the optional per-role stall counters).
 __device__ __forceinline__ bool mbar_wait_timed(unsigned long long* bar, uint32_t parity,
                                                 long long budget, volatile int* abort,
                                                 long long* acc) {
@@ -205,6 +205,14 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
                  : "memory");
 }
+// The same arrival with release semantics of this block only, which does not wait for the thread's
+// global memory traffic (the cluster-wide form took 1100 to 1950 cycles in the split-operand GEMM's
+// loop, this one under 100).  Enough when what it announces stays inside this block's SM: operand
+// tiles in its own shared memory, already handed to the async proxy by a proxy fence, or an
+// accumulator in its own tensor memory, already read.
+__device__ __forceinline__ void mbar_arrive_pair(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.release.cta.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -227,6 +235,42 @@ __device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a,
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// One lane of a converged warp, the same one every time.  The MMA warps run their loops as a whole and
+// let the elected lane issue: operand descriptors and addresses then live in uniform registers, where
+// the instruction wants them.  (From a loop that only lane 0 runs, each instruction cost about 64
+// cycles of moves into uniform registers, which is what N = 128 tiles and the gate GEMM ran at.)
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t e;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(e));
+    return e;
+}
+// The value of lane 0, known to the compiler as warp-uniform.
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ void umma_bf16_pair_if(uint32_t issue, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
+                                                  uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(issue)
+        : "memory");
+}
+// Arrives on the mbarrier at shared address `bar` of BOTH blocks of the pair once the pair's MMAs issued
+// so far have completed.
+__device__ __forceinline__ void umma_commit_both_if(uint32_t issue, uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t.reg .b16 m;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "mov.b16 m, 3;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}"
+        ::"r"(bar), "r"(issue)
         : "memory");
 }
 // Arrives on the mbarrier at `bar_cluster` once the pair's MMAs issued so far have completed.

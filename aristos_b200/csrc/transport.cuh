@@ -331,7 +331,8 @@ struct ReturnFlagArgs {
     int suppress;  // test hook: do not raise the flags (exercises the bounded wait in combine)
 };
 
-__device__ __forceinline__ void publish_return_flags(const ReturnFlagArgs& r, bool* smem_last) {
+template <typename Flag>
+__device__ __forceinline__ void publish_return_flags(const ReturnFlagArgs& r, Flag* smem_last) {
     __threadfence_system();
     __syncthreads();
     if (threadIdx.x == 0) {

@@ -1,0 +1,63 @@
+"""Float layers: the split-operand tensor-core GEMM at the edges of its tiles, and on operands whose
+sums are not finite, where it has to give what fp32 multiply-adds give."""
+import numpy as np
+import pytest
+
+from aristos_b200 import synth
+from aristos_b200.config import KleosConfig
+from oracle import c_oracle, moe_oracle
+from tests import moe_harness as hz
+
+pytestmark = pytest.mark.gpu
+
+
+def _cfg(**kw):
+    return KleosConfig(**{**dict(sequence_len=256, hidden_size=512, intermediate_size=1024, num_experts=8, torch_dtype=0), **kw})
+
+
+@pytest.mark.parametrize("kw", [
+    dict(sequence_len=128, hidden_size=64, intermediate_size=64, num_experts=4),       # one tile, two K slices
+    dict(sequence_len=384, hidden_size=192, intermediate_size=320, num_experts=2),     # odd panel count, 64-column tail
+    dict(sequence_len=2048, hidden_size=256, intermediate_size=2112, num_experts=2, hidden_act=1),  # wide tiles, tail, GELU
+    dict(sequence_len=1024, hidden_size=704, intermediate_size=448, num_experts=64),   # more experts than block pairs / 2
+], ids=["smallest", "odd-panels", "wide-tail-gelu", "many-experts"])
+def test_tile_edges(kw):
+    cfg = _cfg(**kw)
+    packed, views = hz.make_inputs(cfg, 1, bias_scale=0.5)
+    ref = moe_oracle.moe_forward(cfg, 1, views)[0]
+    probs, out, routing = hz.run_layer_single_gpu(cfg, packed[0], forwards=2)
+    hz.check_against_oracle(cfg, ref, probs, out, routing)
+
+
+def test_operands_of_very_different_size():
+    """Rows scaled by 1e-30 .. 1e30: relative accuracy does not depend on a row's size."""
+    cfg = _cfg(num_experts=1, expert_top_k=1)
+    packed, views = hz.make_inputs(cfg, 1)
+    scale = np.float32(10.0) ** np.linspace(-30, 30, cfg.S).astype(np.float32)
+    a = packed[0][:cfg.S * cfg.H].reshape(cfg.S, cfg.H)
+    a *= scale[:, None]
+    ref = c_oracle.dense_ffn(cfg, synth.split_packed(cfg, packed[0], 1))
+    _, out, _ = hz.run_layer_single_gpu(cfg, packed[0])
+    err = np.abs(out - ref).max(axis=1) / np.abs(ref).max(axis=1)
+    assert err.max() <= hz.TOL[0]
+
+
+@pytest.mark.parametrize("act", [0, 1], ids=["relu", "gelu"])
+def test_values_that_are_not_finite(monkeypatch, act):
+    """Infinities, NaN and sums that overflow: the same values as from the FP32 FMA kernel."""
+    cfg = _cfg(num_experts=1, expert_top_k=1, hidden_act=act)
+    packed, _ = hz.make_inputs(cfg, 1, bias_scale=0.5)
+    a = packed[0][:cfg.S * cfg.H].reshape(cfg.S, cfg.H)
+    a[3, 5], a[40, 511], a[70, 0] = np.inf, -np.inf, np.nan
+    a[130] *= np.float32(1e38)
+    a[200, :4] = np.float32(3.4e38)
+    got = hz.run_layer_single_gpu(cfg, packed[0])[1]
+    monkeypatch.setenv("KLEOS_DEBUG_SIMT_GEMM", "1")
+    want = hz.run_layer_single_gpu(cfg, packed[0])[1]
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
+    assert not np.isfinite(want[[3, 40, 70]]).all()
+    plain = np.ones(cfg.S, bool)
+    plain[[3, 40, 70, 130, 200]] = False
+    # two fp32 results, each within the layer's bound of the 64-bit one
+    assert np.abs(got[plain] - want[plain]).max() <= 2 * hz.TOL[0] * np.abs(want[plain]).max()

@@ -219,51 +219,54 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer (leader only)
-        if (leader && lane == 0) {
-            uint32_t it = 0, tile_n = 0;
+        // (the whole warp runs the loop and the elected lane issues, see tc::elect_one)
+        if (leader) {
+            const uint32_t elected = elect_one();
+            const uint32_t slices = smem_u32(tiles), bars = smem_u32(ctl), tmem = (uint32_t)uniform((int)tmem_base);
+            const int n_tiles = uniform(total);
+            uint32_t s = 0, ph = 0, tile_n = 0;
             long long w_acc = 0, w_full = 0;
             const long long t_begin = clock64();
-            for (int t = cluster_id; t < total && !*abort_flag; t += n_clusters, ++tile_n) {
+            for (int t = cluster_id; t < n_tiles; t += n_clusters, ++tile_n) {
                 const uint32_t buf = tile_n & 1, use = tile_n >> 1;
                 if (!mbar_wait_timed(&ctl->acc_empty[buf], (use & 1) ^ 1, g.wait_cycles, abort_flag, &w_acc)) {
-                    report_error(g.status, KLEOS_AT_GEMM_MMA, t, (int)g.epoch);
+                    if (lane == 0) report_error(g.status, KLEOS_AT_GEMM_MMA, t, (int)g.epoch);
                     *abort_flag = 1;
                     break;
                 }
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_base + buf * BN;
+                const uint32_t d_tmem = tmem + buf * BN;
                 bool ok = true;
-                for (int kb = 0; kb < KB; ++kb, ++it) {
-                    const int s = it % NST;
-                    const uint32_t ph = (it / NST) & 1;
+                for (int kb = 0; kb < KB; ++kb) {
                     if (!mbar_wait_timed(&ctl->full[s], ph, g.wait_cycles, abort_flag, &w_full)) {
-                        report_error(g.status, KLEOS_AT_GEMM_MMA, t, (int)g.epoch);
+                        if (lane == 0) report_error(g.status, KLEOS_AT_GEMM_MMA, t, (int)g.epoch);
                         *abort_flag = 1;
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t sa = smem_u32(tiles + s * STAGE_BYTES);
-                    const int nsub = min(SUB, KS - kb * SUB);
-                    for (int sub = 0; sub < nsub; ++sub) {
+                    const uint32_t sa = slices + s * STAGE_BYTES;
+#pragma unroll
+                    for (int sub = 0; sub < SUB; ++sub) {
+                        if (sub > 0 && kb * SUB + sub >= KS) break;  // the last deep stage may be half full
                         const uint64_t da = make_smem_desc(sa + sub * SLICE_BYTES);
                         const uint64_t db = make_smem_desc(sa + sub * SLICE_BYTES + A_STAGE_BYTES);
 #pragma unroll
                         for (int k = 0; k < BK / UMMA_K; ++k)
-                            umma_bf16_pair(d_tmem, da + 2 * k, db + 2 * k, kInstrDesc,
-                                           (kb | sub | k) != 0 ? 1u : 0u);
+                            umma_bf16_pair_if(elected, d_tmem, da + 2 * k, db + 2 * k, kInstrDesc,
+                                              (sub | k) != 0 ? 1u : (uint32_t)(kb != 0));
                     }
                     // the stage is free in both blocks once these MMAs have read it
-                    const uint32_t e_local = smem_u32(&ctl->empty[s]);
-                    umma_commit_pair(map_to_cta(e_local, 0));
-                    umma_commit_pair(map_to_cta(e_local, 1));
+                    umma_commit_both_if(elected, bars + (uint32_t)offsetof(Control, empty) + 8 * s);
+                    if (++s == NST) {
+                        s = 0;
+                        ph ^= 1;
+                    }
                 }
                 if (!ok) break;
-                const uint32_t f_local = smem_u32(&ctl->acc_full[buf]);
-                umma_commit_pair(map_to_cta(f_local, 0));
-                umma_commit_pair(map_to_cta(f_local, 1));
+                umma_commit_both_if(elected, bars + (uint32_t)offsetof(Control, acc_full) + 8 * buf);
             }
-            if (g.stats) {
+            if (g.stats && lane == 0) {
                 g.stats[blockIdx.x * kStatSlots + 2] = w_acc;
                 g.stats[blockIdx.x * kStatSlots + 3] = w_full;
                 g.stats[blockIdx.x * kStatSlots + 4] = clock64() - t_begin;
@@ -318,7 +321,7 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
             if (rows_w <= 0) {
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl->acc_empty[buf]), 0));
+                if (lane == 0) mbar_arrive_pair(map_to_cta(smem_u32(&ctl->acc_empty[buf]), 0));
                 continue;
             }
             TE* obase = out_ptr<TE>(g, p, q * 32, n0);
@@ -340,7 +343,7 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                     // the whole accumulator is in registers: hand it back to the MMA issuer
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl->acc_empty[buf]), 0));
+                    if (lane == 0) mbar_arrive_pair(map_to_cta(smem_u32(&ctl->acc_empty[buf]), 0));
                 }
                 const uint32_t* rc = r[c & 1];
                 const float4* bq = reinterpret_cast<const float4*>(&ctl->bias_s[q][c * 32]);

@@ -141,6 +141,16 @@ __device__ __forceinline__ bool wait_flag(const unsigned long long* flag, uint32
     }
 }
 
+// ---------------------------------------------------------------- programmatic launches
+// The kernels of a forward are launched with programmatic stream serialisation: a kernel's blocks may
+// become resident, and set up their barriers and tensor memory, while the kernel before it is still
+// draining.  pdl_wait() returns once that kernel has completed and its writes are visible.  EVERY
+// kernel calls it, before it touches any global memory that a kernel writes, so that completion is
+// transitive along the stream; pdl_trigger() lets the next kernel's blocks start to arrive.  Both do
+// nothing in a kernel that was launched without the attribute.  (A launch boundary cost 2 to 3 us.)
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // 16-byte global accesses.  Loads of data a peer may have written go through L2 (.cg).
 __device__ __forceinline__ uint4 ld_cg_v4(const void* p) {
     uint4 v;

@@ -180,7 +180,6 @@ ffn_gemm_f32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
     const uint32_t cta_rank = cluster_ctarank();
     volatile int* abort_flag = &ctl->abort;
 
-    for (int i = tid; i <= g.nLx; i += kThreads) ctl->le_start[i] = g.le_start[i];
     if (tid == 0) {
         for (int s = 0; s < Sh::RING; ++s) {
             mbar_init(&ctl->ring_full[s], 1);
@@ -203,6 +202,9 @@ ffn_gemm_f32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
+    pdl_wait();
+    pdl_trigger();
+    for (int i = tid; i <= g.nLx; i += kThreads) ctl->le_start[i] = g.le_start[i];
     tc_fence_before();
     __syncthreads();
     cluster_sync_all();  // both blocks' barriers exist before anything remote touches them

@@ -18,6 +18,8 @@ __global__ void __launch_bounds__(256) ffn_gemm_simt(GemmArgs g) {
     __shared__ bool last_block;
 
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    pdl_trigger();
+    pdl_wait();
     for (int i = tid; i <= g.nLx; i += 256) le_start_s[i] = g.le_start[i];
     __syncthreads();
     const int NT = (g.N + BN - 1) / BN;

@@ -59,7 +59,6 @@ ffn_gemm_tf32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     volatile int* abort_flag = &ctl->abort;
 
-    for (int i = tid; i <= g.nLx; i += blockDim.x) ctl->le_start[i] = g.le_start[i];
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&ctl->full[s], 1);
@@ -78,6 +77,9 @@ ffn_gemm_tf32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    pdl_wait();
+    pdl_trigger();
+    for (int i = tid; i <= g.nLx; i += blockDim.x) ctl->le_start[i] = g.le_start[i];
     tc_fence_before();
     __syncthreads();
     tc_fence_after();

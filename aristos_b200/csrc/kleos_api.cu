@@ -338,13 +338,31 @@ int ensure_maps(const Sections& s) {
     return KLEOS_OK;
 }
 
+// One kernel of a forward, launched so that its blocks may arrive while the kernel before it drains
+// (see pdl_wait()).
+template <typename... P, typename... A>
+void launch(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3((unsigned)grid);
+    lc.blockDim = dim3((unsigned)threads);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = &at;
+    lc.numAttrs = 1;
+    ++g.launches;
+    cudaLaunchKernelEx(&lc, kernel, args...);  // failures: cudaGetLastError() at the end of the forward
+}
+
 template <typename T>
 int launch_route(const RouteArgs& ra, cudaStream_t st) {
     const int grid = (ra.S + 63) / 64;
     if (ra.PX == 64) {
-        { ++g.launches; route_kernel<T, 64><<<grid, 256, route_smem_bytes<64>(), st>>>(ra); }
+        launch(route_kernel<T, 64>, grid, 256, route_smem_bytes<64>(), st, ra);
     } else if (ra.PX == 128) {
-        { ++g.launches; route_kernel<T, 128><<<grid, 256, route_smem_bytes<128>(), st>>>(ra); }
+        launch(route_kernel<T, 128>, grid, 256, route_smem_bytes<128>(), st, ra);
     } else if (ra.PX == 256) {
         static bool attr_set = false;
         if (!attr_set) {
@@ -353,11 +371,11 @@ int launch_route(const RouteArgs& ra, cudaStream_t st) {
                                             (int)route_smem_bytes<256>()));
             attr_set = true;
         }
-        { ++g.launches; route_kernel<T, 256><<<grid, 256, route_smem_bytes<256>(), st>>>(ra); }
+        launch(route_kernel<T, 256>, grid, 256, route_smem_bytes<256>(), st, ra);
     } else {
         return fail(KLEOS_E_UNSUPPORTED, "more than 256 experts are not supported by the router");
     }
-    { ++g.launches; refine_kernel<T><<<148, 256, 0, st>>>(ra); }
+    launch(refine_kernel<T>, 148, 256, 0, st, ra);
     return KLEOS_OK;
 }
 
@@ -367,28 +385,28 @@ template <typename TE, int kEpi>
 void launch_tc2(bool deep, int grid, cudaStream_t st, const CUtensorMap& map_a, const CUtensorMap& map_b,
                 const GemmArgs& ga) {
     if (deep)
-        { ++g.launches; ffn_gemm_tc2<TE, kEpi, 2><<<grid, 256, gemm_tc2::SMEM_BYTES, st>>>(map_a, map_b, ga); }
+        launch(ffn_gemm_tc2<TE, kEpi, 2>, grid, 256, gemm_tc2::SMEM_BYTES, st, map_a, map_b, ga);
     else
-        { ++g.launches; ffn_gemm_tc2<TE, kEpi, 1><<<grid, 256, gemm_tc2::SMEM_BYTES, st>>>(map_a, map_b, ga); }
+        launch(ffn_gemm_tc2<TE, kEpi, 1>, grid, 256, gemm_tc2::SMEM_BYTES, st, map_a, map_b, ga);
 }
 
 // The persistent kernel, instantiated per activation and per compile-time top-k of the combine.
 template <typename TE>
 void launch_flow(int act, int K, cudaStream_t st, const flow::Args& fa, const CUtensorMap* fa_act) {
     const int grid = g.flow_grid, smem = flow::SMEM_BYTES, thr = flow::kThreads;
-    if (act == 0 && K == 2) { ++g.launches; moe_flow_kernel<TE, 0, 2><<<grid, thr, smem, st>>>(g.map_x, g.map_w1h, g.map_y1, g.map_w2h, *fa_act, g.map_wgh, fa); }
-    else if (act == 0) { ++g.launches; moe_flow_kernel<TE, 0, 0><<<grid, thr, smem, st>>>(g.map_x, g.map_w1h, g.map_y1, g.map_w2h, *fa_act, g.map_wgh, fa); }
-    else if (K == 2) { ++g.launches; moe_flow_kernel<TE, 1, 2><<<grid, thr, smem, st>>>(g.map_x, g.map_w1h, g.map_y1, g.map_w2h, *fa_act, g.map_wgh, fa); }
-    else { ++g.launches; moe_flow_kernel<TE, 1, 0><<<grid, thr, smem, st>>>(g.map_x, g.map_w1h, g.map_y1, g.map_w2h, *fa_act, g.map_wgh, fa); }
+    if (act == 0 && K == 2) launch(moe_flow_kernel<TE, 0, 2>, grid, thr, smem, st, g.map_x, g.map_w1h, g.map_y1, g.map_w2h, *fa_act, g.map_wgh, fa);
+    else if (act == 0) launch(moe_flow_kernel<TE, 0, 0>, grid, thr, smem, st, g.map_x, g.map_w1h, g.map_y1, g.map_w2h, *fa_act, g.map_wgh, fa);
+    else if (K == 2) launch(moe_flow_kernel<TE, 1, 2>, grid, thr, smem, st, g.map_x, g.map_w1h, g.map_y1, g.map_w2h, *fa_act, g.map_wgh, fa);
+    else launch(moe_flow_kernel<TE, 1, 0>, grid, thr, smem, st, g.map_x, g.map_w1h, g.map_y1, g.map_w2h, *fa_act, g.map_wgh, fa);
 }
 
 // TF32 layers: one launch of the kind::tf32 GEMM with the epilogue chosen at compile time.
 void launch_tf32(int epi, cudaStream_t st, const CUtensorMap& map_a, const CUtensorMap& map_b,
                  const GemmArgs& ga) {
     const int grid = g.sm_count, smem = gemm_tf32::SMEM_BYTES;
-    if (epi == 0) { ++g.launches; ffn_gemm_tf32<0><<<grid, 256, smem, st>>>(map_a, map_b, ga); }
-    else if (epi == 1) { ++g.launches; ffn_gemm_tf32<1><<<grid, 256, smem, st>>>(map_a, map_b, ga); }
-    else { ++g.launches; ffn_gemm_tf32<2><<<grid, 256, smem, st>>>(map_a, map_b, ga); }
+    if (epi == 0) launch(ffn_gemm_tf32<0>, grid, 256, smem, st, map_a, map_b, ga);
+    else if (epi == 1) launch(ffn_gemm_tf32<1>, grid, 256, smem, st, map_a, map_b, ga);
+    else launch(ffn_gemm_tf32<2>, grid, 256, smem, st, map_a, map_b, ga);
 }
 
 // Float layers: tile width of the split-operand GEMM with N output columns: the one whose rounds of
@@ -405,9 +423,8 @@ int f32_tile_width(int N) {
 
 void launch_f32(int bn, cudaStream_t st, const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmArgs& ga) {
     const int grid = g.sm_count & ~1, thr = gemm_f32::kThreads;
-    ++g.launches;
-    if (bn == 128) ffn_gemm_f32<128><<<grid, thr, gemm_f32::Shape<128>::SMEM_BYTES, st>>>(map_a, map_b, ga);
-    else ffn_gemm_f32<64><<<grid, thr, gemm_f32::Shape<64>::SMEM_BYTES, st>>>(map_a, map_b, ga);
+    if (bn == 128) launch(ffn_gemm_f32<128>, grid, thr, gemm_f32::Shape<128>::SMEM_BYTES, st, map_a, map_b, ga);
+    else launch(ffn_gemm_f32<64>, grid, thr, gemm_f32::Shape<64>::SMEM_BYTES, st, map_a, map_b, ga);
 }
 
 // Optional replacement of the activation input and the layer-output destination of one
@@ -460,9 +477,9 @@ int forward_dense(const Sections& s, const CUtensorMap* map_a, cudaStream_t st, 
         KLEOS_CUDA(mark());
         launch_f32(g.f32_bn[1], st, g.map_y1, g.map_w2, g2);
     } else {
-        { ++g.launches; ffn_gemm_simt<T><<<g.sm_count * 2, 256, 0, st>>>(g1); }
+        launch(ffn_gemm_simt<T>, g.sm_count * 2, 256, 0, st, g1);
         KLEOS_CUDA(mark());
-        { ++g.launches; ffn_gemm_simt<T><<<g.sm_count * 2, 256, 0, st>>>(g2); }
+        launch(ffn_gemm_simt<T>, g.sm_count * 2, 256, 0, st, g2);
     }
     KLEOS_CUDA(mark());
     KLEOS_CUDA(mark());  // combine: nothing to do
@@ -526,12 +543,10 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
         if constexpr (!std::is_same<T, float>::value) {
             const int grid = (c.S + route_tc::BM - 1) / route_tc::BM;
             if (c.PX == 64)
-                { ++g.launches; route_tc_kernel<T, 64><<<grid, 256, route_tc::Shape<64>::SMEM_BYTES, st>>>(
-                    *act_map, g.map_wg, ra, g.status, g.wait_cycles, (int)g.epoch); }
+                launch(route_tc_kernel<T, 64>, grid, 256, route_tc::Shape<64>::SMEM_BYTES, st, *act_map, g.map_wg, ra, g.status, g.wait_cycles, (int)g.epoch);
             else
-                { ++g.launches; route_tc_kernel<T, 128><<<grid, 256, route_tc::Shape<128>::SMEM_BYTES, st>>>(
-                    *act_map, g.map_wg, ra, g.status, g.wait_cycles, (int)g.epoch); }
-            { ++g.launches; refine_kernel<T><<<148, 256, 0, st>>>(ra); }
+                launch(route_tc_kernel<T, 128>, grid, 256, route_tc::Shape<128>::SMEM_BYTES, st, *act_map, g.map_wg, ra, g.status, g.wait_cycles, (int)g.epoch);
+            launch(refine_kernel<T>, 148, 256, 0, st, ra);
         }
     } else if ((rc = launch_route<T>(ra, st))) {
         return rc;
@@ -546,10 +561,10 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     sa.cflag_offset = g.lay.cflag; sa.rank = g.rank; sa.nLx = g.nLx; sa.epoch = g.epoch;
     sa.tile_hist = g.tile_hist;
     if (!routed_in_kernel) {
-        { ++g.launches; tile_hist_kernel<<<(c.S + kSlotTile - 1) / kSlotTile, 256, 0, st>>>(sa); }
-        { ++g.launches; slot_kernel<<<(c.S + kSlotTile - 1) / kSlotTile, 256, 0, st>>>(sa); }
+        launch(tile_hist_kernel, (c.S + kSlotTile - 1) / kSlotTile, 256, 0, st, sa);
+        launch(slot_kernel, (c.S + kSlotTile - 1) / kSlotTile, 256, 0, st, sa);
         if (g.col_partial)
-            { ++g.launches; gate_stats_kernel<<<1, 256, 0, st>>>(g.col_partial, route_blocks, c.PX, g.counts, c.S, c.E, g.gate_stats); }
+            launch(gate_stats_kernel, 1, 256, 0, st, g.col_partial, route_blocks, c.PX, g.counts, c.S, c.E, g.gate_stats);
         KLEOS_CUDA(mark());
     }
 
@@ -592,7 +607,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     da.lay = g.lay; da.done_counter = g.done_dispatch; da.H = c.H; da.E = c.E; da.EC = c.EC;
     da.pEC = c.pEC; da.nLx = g.nLx; da.rank = g.rank; da.world = g.world; da.epoch = g.epoch;
     da.elem_bytes = c.elem_bytes; da.le_begin = 0; da.le_end = g.nLx;
-    { ++g.launches; dispatch_kernel<<<g.sm_count * 4, 256, 0, st>>>(da); }
+    launch(dispatch_kernel, g.sm_count * 4, 256, 0, st, da);
     KLEOS_CUDA(mark());
     // 4. plan: wait for every source's rows, list the panels
     PlanArgs pa{};
@@ -600,7 +615,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     pa.cell_counts = g.cell_counts; pa.status = g.status; pa.world = g.world; pa.nLx = g.nLx;
     pa.pEC = c.pEC; pa.epoch = g.epoch; pa.wait_cycles = g.wait_cycles; pa.rank = g.rank;
     pa.le_begin = 0; pa.le_end = g.nLx;
-    { ++g.launches; plan_kernel<<<1, 1024, 0, st>>>(pa); }
+    launch(plan_kernel, 1, 1024, 0, st, pa);
     KLEOS_CUDA(mark());
 
     // 5./6. expert FFN
@@ -643,9 +658,9 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
         launch_f32(g.f32_bn[1], st, g.map_y1, g.map_w2, g2);
         KLEOS_CUDA(mark());
     } else {
-        { ++g.launches; ffn_gemm_simt<T><<<g.sm_count * 2, 256, 0, st>>>(g1); }
+        launch(ffn_gemm_simt<T>, g.sm_count * 2, 256, 0, st, g1);
         KLEOS_CUDA(mark());
-        { ++g.launches; ffn_gemm_simt<T><<<g.sm_count * 2, 256, 0, st>>>(g2); }
+        launch(ffn_gemm_simt<T>, g.sm_count * 2, 256, 0, st, g2);
         KLEOS_CUDA(mark());
     }
 
@@ -656,11 +671,11 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     ca.PX = c.PX; ca.pEC = c.pEC; ca.world = g.world; ca.epoch = g.epoch;
     ca.wait_cycles = g.wait_cycles;
     if (c.K == 2)
-        { ++g.launches; combine_kernel<T, 2><<<g.sm_count * 4, 256, 0, st>>>(ca); }
+        launch(combine_kernel<T, 2>, g.sm_count * 4, 256, 0, st, ca);
     else if (c.K == 1)
-        { ++g.launches; combine_kernel<T, 1><<<g.sm_count * 4, 256, 0, st>>>(ca); }
+        launch(combine_kernel<T, 1>, g.sm_count * 4, 256, 0, st, ca);
     else
-        { ++g.launches; combine_kernel<T, 0><<<g.sm_count * 4, 256, 0, st>>>(ca); }
+        launch(combine_kernel<T, 0>, g.sm_count * 4, 256, 0, st, ca);
     KLEOS_CUDA(mark());
     KLEOS_CUDA(cudaGetLastError());
     return KLEOS_OK;

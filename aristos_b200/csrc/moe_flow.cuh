@@ -461,7 +461,6 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     Counters* ctr = a.ctr + (a.epoch & 1u);
     const long long budget = a.wait_cycles;
     long long* stamp = a.stamps ? a.stamps + (size_t)blockIdx.x * kStampSlots : nullptr;
-    if (stamp && tid == 0) stamp[kStart] = global_ns();
     long long* stall = a.stalls ? a.stalls + (size_t)blockIdx.x * kStallSlots : nullptr;
     // waits of the tile stream, timed only when the caller asked for the counters
     auto timed_wait = [&](unsigned long long* bar, uint32_t parity, long long* acc) -> bool {
@@ -502,6 +501,9 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
+    pdl_wait();
+    pdl_trigger();
+    if (stamp && tid == 0) stamp[kStart] = global_ns();
     if (blockIdx.x == 0) {
         // the forward after this one finds its copy of the scheduler state cleared
         unsigned* nxt = reinterpret_cast<unsigned*>(a.ctr + ((a.epoch + 1u) & 1u));

@@ -118,6 +118,8 @@ __global__ void __launch_bounds__(256) route_kernel(RouteArgs a) {
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
     const int row0 = blockIdx.x * BM;
     const int H = a.H;
+    pdl_trigger();
+    pdl_wait();
 
     float acc[4][TN];
 #pragma unroll
@@ -216,6 +218,8 @@ __global__ void __launch_bounds__(256) gate_stats_kernel(const float* col_partia
                                                          int PX, const unsigned* counts, int S,
                                                          int E, float* out) {
     __shared__ float term[256];
+    pdl_trigger();
+    pdl_wait();
     const int e = threadIdx.x;
     float t = 0.f;
     if (e < E) {
@@ -250,6 +254,8 @@ __global__ void __launch_bounds__(256) refine_kernel(RouteArgs a) {
     constexpr int VEC = 16 / sizeof(T);
     const T* A = static_cast<const T*>(a.A);
     const T* Wg = static_cast<const T*>(a.Wg);
+    pdl_trigger();
+    pdl_wait();
     const int n = *a.refine_count;
     const int lane = threadIdx.x & 31;
     const int warps = gridDim.x * (blockDim.x >> 5);
@@ -373,6 +379,8 @@ constexpr int kSlotTile = 128;
 
 __global__ void __launch_bounds__(256) tile_hist_kernel(SlotArgs a) {
     __shared__ int hist[256];  // E <= 256
+    pdl_trigger();
+    pdl_wait();
     const int tid = threadIdx.x, tok0 = blockIdx.x * kSlotTile;
     for (int e = tid; e < a.E; e += blockDim.x) hist[e] = 0;
     __syncthreads();
@@ -385,6 +393,8 @@ __global__ void __launch_bounds__(256) tile_hist_kernel(SlotArgs a) {
 __global__ void __launch_bounds__(256) slot_kernel(SlotArgs a) {
     __shared__ int base[256];
     const int tid = threadIdx.x, b = blockIdx.x;
+    pdl_trigger();
+    pdl_wait();
     const int tok0 = b * kSlotTile;
     const bool last = b == (int)gridDim.x - 1;
     // base slot of every expert = sum of the earlier tiles' histograms; the tiles are split

@@ -43,6 +43,8 @@ __global__ void __launch_bounds__(256) dispatch_kernel(DispatchArgs a) {
     __shared__ unsigned prefix[257];  // E <= 256
     __shared__ bool last_block;
     const int tid = threadIdx.x;
+    pdl_trigger();
+    pdl_wait();
     // Rows are sent in this order: local expert index first, and for each of them the owner
     // ranks starting with the one after this rank.  At any moment the source ranks therefore
     // write to DIFFERENT owners, instead of all pushing into the same GPU's NVLink ingress.
@@ -142,6 +144,8 @@ __global__ void __launch_bounds__(1024) plan_kernel(PlanArgs a) {
     __shared__ int failed;
     __shared__ int cnt_s[2048];  // world * nLx <= 8 * 256; a count can reach pEC, which has no 16-bit limit
     const int cells = a.world * a.nLx;
+    pdl_trigger();
+    pdl_wait();
     if (threadIdx.x == 0) failed = 0;
     __syncthreads();
     const unsigned long long* flags =
@@ -212,6 +216,8 @@ struct CombineArgs {
 template <typename T, int KT>
 __global__ void __launch_bounds__(256) combine_kernel(CombineArgs a) {
     __shared__ int failed;
+    pdl_trigger();
+    pdl_wait();
     if (threadIdx.x == 0) failed = 0;
     __syncthreads();
     if (threadIdx.x < a.world) {

@@ -505,6 +505,9 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     auto mark = [&]() -> cudaError_t { return timed ? cudaEventRecord(g.ev[evi++], st) : cudaSuccess; };
     KLEOS_CUDA(mark());
 
+    // One rank owns every expert: the router writes the panel list, and the rows only move inside this
+    // GPU's memory, with no flags to raise or to wait for.
+    const bool local = g.world == 1 && !g.use_flow;
     bool routed_in_kernel = g.use_flow && g.fuse_route;
     if (routed_in_kernel) {
         KLEOS_CUDA(mark());
@@ -521,6 +524,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
             fr.pEC = c.pEC; fr.nLx = g.nLx; fr.rank = g.rank; fr.world = g.world; fr.epoch = g.epoch;
             fr.sub = 1; fr.unit_rows = flow::kUnitRows; fr.fuse_route = 1; fr.route_only = 1;
             fr.Wg = s.Wg; fr.gate_bias = g.bias; fr.tile_hist = g.tile_hist; fr.tie_eps = 1e-4f;
+            if (local) { fr.panels = g.panels; fr.le_start = g.le_start; }
             launch_flow<T>(c.hidden_act, c.K, st, fr, act_map);
         }
         KLEOS_CUDA(mark());
@@ -560,6 +564,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     for (int r = 0; r < kMaxWorld; ++r) sa.peer_arena[r] = g.peers.arena[r];
     sa.cflag_offset = g.lay.cflag; sa.rank = g.rank; sa.nLx = g.nLx; sa.epoch = g.epoch;
     sa.tile_hist = g.tile_hist;
+    if (local) { sa.panels = g.panels; sa.le_start = g.le_start; }
     if (!routed_in_kernel) {
         launch(tile_hist_kernel, (c.S + kSlotTile - 1) / kSlotTile, 256, 0, st, sa);
         launch(slot_kernel, (c.S + kSlotTile - 1) / kSlotTile, 256, 0, st, sa);
@@ -607,7 +612,8 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     da.lay = g.lay; da.done_counter = g.done_dispatch; da.H = c.H; da.E = c.E; da.EC = c.EC;
     da.pEC = c.pEC; da.nLx = g.nLx; da.rank = g.rank; da.world = g.world; da.epoch = g.epoch;
     da.elem_bytes = c.elem_bytes; da.le_begin = 0; da.le_end = g.nLx;
-    launch(dispatch_kernel, g.sm_count * 4, 256, 0, st, da);
+    if (local) launch(dispatch_local_kernel, (c.S + kDispatchTokens - 1) / kDispatchTokens, kDispatchTokens * 32, 0, st, LocalDispatchArgs{s.A, g.topk, g.slots, g.arena + g.lay.xcell, c.S, c.K, c.pEC, (unsigned)((size_t)c.H * c.elem_bytes / 16)});
+    else launch(dispatch_kernel, g.sm_count * 4, 256, 0, st, da);
     KLEOS_CUDA(mark());
     // 4. plan: wait for every source's rows, list the panels
     PlanArgs pa{};
@@ -615,7 +621,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     pa.cell_counts = g.cell_counts; pa.status = g.status; pa.world = g.world; pa.nLx = g.nLx;
     pa.pEC = c.pEC; pa.epoch = g.epoch; pa.wait_cycles = g.wait_cycles; pa.rank = g.rank;
     pa.le_begin = 0; pa.le_end = g.nLx;
-    launch(plan_kernel, 1, 1024, 0, st, pa);
+    if (!local) launch(plan_kernel, 1, 1024, 0, st, pa);
     KLEOS_CUDA(mark());
 
     // 5./6. expert FFN

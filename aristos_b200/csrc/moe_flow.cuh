@@ -176,6 +176,8 @@ struct Args {
     const float* gate_bias;  // [E]
     int* tile_hist;          // [S/128][E] per-tile histogram of the chosen experts
     float tie_eps;
+    PanelEntry* panels;      // route_only on one rank: the panel list is written here (else null)
+    int* le_start;
 };
 
 struct Tile {
@@ -886,6 +888,13 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                                    make_flag(a.epoch, (unsigned)min(total, a.EC)));
                 }
             };
+            auto write_plan = [&](int last_tile_too) {
+                if (a.panels == nullptr) return;
+                int* cnt = ctl->cnt_s;
+                for (int e = tid; e < a.E; e += kThreads)
+                    cnt[e] = min(base[e] + (last_tile_too ? __ldcg(a.tile_hist + (size_t)(n_tiles - 1) * a.E + e) : 0), a.EC);
+                write_local_plan(cnt, reinterpret_cast<int*>(ctl->prefix_s), a.E, a.pEC, a.rank, a.panels, a.le_start);
+            };
             // When the last block pair routed no tile it has nothing to do here: its second block
             // adds up ALL tiles and publishes the counts, off the path of the blocks that write
             // slots.  Otherwise the block of the last tile does it on top of its own work.
@@ -893,6 +902,7 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             if (spare && blockIdx.x == gridDim.x - 1) {
                 sum_tiles_before(n_tiles);
                 publish_counts(0);
+                write_plan(0);
             }
             for (int rt = cluster_id; rt < n_rt; rt += n_clusters) {
                 const int tile = rt * 2 + (int)cta_rank;
@@ -901,7 +911,10 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 for (int i = tid; i < 8 * 256; i += kThreads) (&wcount[0][0])[i] = 0;
                 sum_tiles_before(tile);
                 if (stamp && tid == 0) stamp[kSlotBase] = global_ns();
-                if (!spare && tile == n_tiles - 1) publish_counts(1);
+                if (!spare && tile == n_tiles - 1) {
+                    publish_counts(1);
+                    write_plan(1);
+                }
                 const int n_own = min(BM, a.S - tok0) * a.K;
                 for (int i0 = 0; i0 < n_own; i0 += 256) {
                     const int i = i0 + tid;

@@ -9,7 +9,7 @@
 // are re-evaluated in fp64 so the selected set does not depend on accumulation order.
 #pragma once
 
-#include "common.cuh"
+#include "transport.cuh"
 
 namespace kleos {
 
@@ -365,6 +365,9 @@ struct SlotArgs {
     size_t cflag_offset;
     int rank, nLx;
     uint32_t epoch;
+    // one rank: the last block also writes the panel list (else null)
+    PanelEntry* panels;
+    int* le_start;
 };
 
 // Slots in ascending token order (the reference hands them out in atomicAdd arrival order,
@@ -417,6 +420,7 @@ __global__ void __launch_bounds__(256) slot_kernel(SlotArgs a) {
         }
         __syncthreads();
     }
+    __shared__ int routed[256], off[257];
     for (int e = tid; e < a.E; e += blockDim.x) {
         const int run = base[e];
         if (last) {
@@ -426,8 +430,10 @@ __global__ void __launch_bounds__(256) slot_kernel(SlotArgs a) {
             st_release_sys(reinterpret_cast<unsigned long long*>(a.peer_arena[owner] + a.cflag_offset) +
                                ((size_t)a.rank * a.nLx + le),
                            make_flag(a.epoch, (unsigned)min(total, a.EC)));
+            routed[e] = min(total, a.EC);
         }
     }
+    if (last && a.panels != nullptr) write_local_plan(routed, off, a.E, a.pEC, a.rank, a.panels, a.le_start);
     // Rank of every (token, choice) entry among the earlier entries of the tile that chose the
     // same expert.  Entries are taken in order, 256 at a time: inside a warp the rank comes from
     // a match mask, across the eight warps from a per-warp count table, and `base` carries the

@@ -356,27 +356,23 @@ void launch(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream
     cudaLaunchKernelEx(&lc, kernel, args...);  // failures: cudaGetLastError() at the end of the forward
 }
 
+// Router on the FP32 pipes, for the layer's padded expert count.  `prepare` only sets the kernel up.
 template <typename T>
-int launch_route(const RouteArgs& ra, cudaStream_t st) {
-    const int grid = (ra.S + 63) / 64;
-    if (ra.PX == 64) {
-        launch(route_kernel<T, 64>, grid, 256, route_smem_bytes<64>(), st, ra);
-    } else if (ra.PX == 128) {
-        launch(route_kernel<T, 128>, grid, 256, route_smem_bytes<128>(), st, ra);
-    } else if (ra.PX == 256) {
-        static bool attr_set = false;
-        if (!attr_set) {
-            KLEOS_CUDA(cudaFuncSetAttribute(route_kernel<T, 256>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)route_smem_bytes<256>()));
-            attr_set = true;
+int launch_route(const RouteArgs& ra, cudaStream_t st, bool prepare = false) {
+    const int grid = (ra.S + route_fma::TM - 1) / route_fma::TM;
+    auto one = [&](void (*kernel)(RouteArgs), int smem) -> int {
+        if (prepare) {
+            KLEOS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            return KLEOS_OK;
         }
-        launch(route_kernel<T, 256>, grid, 256, route_smem_bytes<256>(), st, ra);
-    } else {
-        return fail(KLEOS_E_UNSUPPORTED, "more than 256 experts are not supported by the router");
-    }
-    launch(refine_kernel<T>, 148, 256, 0, st, ra);
-    return KLEOS_OK;
+        launch(kernel, grid, 256, smem, st, ra);
+        launch(refine_kernel<T>, 148, 256, 0, st, ra);
+        return KLEOS_OK;
+    };
+    if (ra.PX == 64) return one(route_kernel<T, 64>, route_fma::smem_bytes<T, 64>());
+    if (ra.PX == 128) return one(route_kernel<T, 128>, route_fma::smem_bytes<T, 128>());
+    if (ra.PX == 256) return one(route_kernel<T, 256>, route_fma::smem_bytes<T, 256>());
+    return fail(KLEOS_E_UNSUPPORTED, "more than 256 experts are not supported by the router");
 }
 
 // The paired GEMM comes in two pipeline shapes (see gemm_tc2.cuh): deep = three 128-wide stages,
@@ -539,7 +535,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     ra.refine_logits = g.refine_logits; ra.refine_done = g.refine_done;
     ra.S = c.S; ra.H = c.H; ra.E = c.E; ra.K = c.K; ra.PX = c.PX; ra.tie_eps = 1e-4f;
     ra.col_partial = g.col_partial;  // null unless is_training
-    int route_blocks = (c.S + 63) / 64;
+    int route_blocks = (c.S + route_fma::TM - 1) / route_fma::TM;
     if (routed_in_kernel) {
         // nothing to launch here
     } else if ((g.use_tc || g.use_tf32_tc) && c.PX <= 128) {
@@ -947,7 +943,7 @@ static int initialize_impl(const char* config_json_path, int rank, int world, co
     if ((rc = dev_alloc(&g.panels, (size_t)cfg.E * cfg.pEC / kTileM))) return rc;
     if ((rc = dev_alloc(&g.status, 1))) return rc;
     if (cfg.is_training && !dense) {
-        if ((rc = dev_alloc(&g.col_partial, (size_t)((cfg.S + 63) / 64) * cfg.PX))) return rc;
+        if ((rc = dev_alloc(&g.col_partial, (size_t)((cfg.S + route_fma::TM - 1) / route_fma::TM) * cfg.PX))) return rc;
         if ((rc = dev_alloc(&g.gate_stats, (size_t)2 * cfg.E + 1))) return rc;
     }
     for (auto& e : g.ev) KLEOS_CUDA(cudaEventCreate(&e));
@@ -955,6 +951,15 @@ static int initialize_impl(const char* config_json_path, int rank, int world, co
     if (const char* gs = std::getenv("KLEOS_GEMM_STATS"))
         if (gs[0] == '1' && (rc = dev_alloc(&g.gemm_stats, (size_t)2 * g.sm_count * kStatSlots))) return rc;
 
+    if (!dense && !((g.use_tc || g.use_tf32_tc) && cfg.PX <= 128) && cfg.PX != 192) {
+        RouteArgs ra{};
+        ra.PX = cfg.PX;
+        rc = cfg.torch_dtype == 0   ? launch_route<float>(ra, 0, true)
+             : cfg.torch_dtype == 1 ? launch_route<tf32_t>(ra, 0, true)
+             : cfg.torch_dtype == 2 ? launch_route<__nv_bfloat16>(ra, 0, true)
+                                    : launch_route<__half>(ra, 0, true);
+        if (rc) return rc;
+    }
     if (g.use_tc) {
         if (cfg.torch_dtype == 2) rc = set_tc_attributes<__nv_bfloat16>();
         else rc = set_tc_attributes<__half>();

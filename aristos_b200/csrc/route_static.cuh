@@ -71,9 +71,12 @@ extern "C" int kleos_route_static(const void* A, const void* Wg, const float* ga
     if (!g_scratch_ptr[dev]) {
         // one-time set-up for this device (do the first call outside any stream capture)
         void* p = nullptr;
-        const cudaError_t e = cudaGetSymbolAddress(&p, g_route_scratch);
+        cudaError_t e = cudaGetSymbolAddress(&p, g_route_scratch);
+        const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(route_kernel<float, 64>, dyn, route_fma::smem_bytes<float, 64>());
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(route_kernel<__nv_bfloat16, 64>, dyn, route_fma::smem_bytes<__nv_bfloat16, 64>());
         if (e != cudaSuccess || !p) {
-            std::fprintf(stderr, "[kleos_b200] cudaGetSymbolAddress failed: %s\n",
+            std::fprintf(stderr, "[kleos_b200] setting up kleos_route_static failed: %s\n",
                          cudaGetErrorString(e));
             return KLEOS_E_CUDA;
         }
@@ -104,12 +107,12 @@ extern "C" int kleos_route_static(const void* A, const void* Wg, const float* ga
     ra.K = K;
     ra.PX = 64;
     ra.tie_eps = 1e-4f;
-    const int grid = (S + 63) / 64;
+    const int grid = (S + route_fma::TM - 1) / route_fma::TM;
     if (torch_dtype == 0) {
-        route_kernel<float, 64><<<grid, 256, route_smem_bytes<64>(), st>>>(ra);
+        route_kernel<float, 64><<<grid, 256, route_fma::smem_bytes<float, 64>(), st>>>(ra);
         refine_kernel<float><<<148, 256, 0, st>>>(ra);
     } else {
-        route_kernel<__nv_bfloat16, 64><<<grid, 256, route_smem_bytes<64>(), st>>>(ra);
+        route_kernel<__nv_bfloat16, 64><<<grid, 256, route_fma::smem_bytes<__nv_bfloat16, 64>(), st>>>(ra);
         refine_kernel<__nv_bfloat16><<<148, 256, 0, st>>>(ra);
     }
     const cudaError_t e = cudaGetLastError();

@@ -8,14 +8,14 @@
 // 128-byte lines, also when the destination is a peer's cell.  No load is multicast: every block
 // fetches exactly the bytes it keeps.
 //
-// Per block, 256 threads:
+// Per block, 384 threads:
 //   warp 0      TMA producer (one lane): waits on its own `empty`, loads into its own shared
 //               memory, credits the bytes to the LEADER's `full` barrier
 //   warp 1      leader only: issues tcgen05.mma.cta_group::2, commits to `empty` and
 //               `acc_full` of BOTH blocks
 //   warp 2      tensor-memory allocation / release (both blocks, cta_group::2 forms)
-//   warps 4..7  epilogue of the block's own 128 accumulator rows; arrives on the LEADER's
-//               `acc_empty`
+//   warps 4..11 epilogue of the block's own 128 accumulator rows, half of the columns each; arrives
+//               on the LEADER's `acc_empty`
 // Work and epilogue semantics follow the reference's tile worker (os/processor/processor.cuh:
 // 350-489,706-741).  Every wait is bounded.  This kernel runs one GEMM over a finished panel
 // list (the dense single-expert layer, and the routed layer when its phases are launched one
@@ -35,6 +35,7 @@ constexpr int kSlices = 6;                        // 64-wide K slices of shared 
 constexpr int A_STAGE_BYTES = BM * BK * 2;        // 16 KiB: one K slice of this block's panel
 constexpr int B_STAGE_BYTES = (BN / 2) * BK * 2;  // 16 KiB: one K slice of this block's half weight tile
 constexpr int SLICE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
+constexpr int kBackWarps = 8, kThreads = (4 + kBackWarps) * 32;
 constexpr int TMEM_COLS = 512;  // two accumulators of 256 fp32 columns
 constexpr int SMEM_BYTES = kSlices * SLICE_BYTES + 1024 + 28672;
 
@@ -42,12 +43,12 @@ struct Control {
     unsigned long long full[kSlices];   // used on the leader (one per pipeline stage)
     unsigned long long empty[kSlices];  // one per block
     unsigned long long acc_full[2];    // one per block
-    unsigned long long acc_empty[2];   // used on the leader, 8 arrivals (4 warps x 2 blocks)
+    unsigned long long acc_empty[2];   // used on the leader, 16 arrivals (8 warps x 2 blocks)
     uint32_t tmem_base;
     int abort;
     int le_start[257];
-    __align__(16) float bias_s[4][256];      // bias of the tile being read back, per epilogue warp
-    __align__(16) uint4 stage_s[4][32 * 8];  // per epilogue warp: 32 rows x 128 bytes, swizzled
+    __align__(16) float bias_s[kBackWarps][BN / 2];   // bias of the columns being read back, per epilogue warp
+    __align__(16) uint4 stage_s[kBackWarps][16 * 8];  // per epilogue warp: 16 rows x 128 bytes, swizzled
 };
 
 static_assert(sizeof(Control) <= 28672, "control block must fit the shared memory set aside for it");
@@ -91,7 +92,7 @@ __device__ __forceinline__ int total_pair_tiles(const int* le_start, int le_begi
 // stream from HBM), 2 gives three deep stages and half the barrier round trips (best when the
 // operands come from L2 and the tensor pipe is the limit).
 template <typename TE, int kEpi, int kSub>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_tc2::kThreads, 1)
 ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
              GemmArgs g) {
     using namespace tc;
@@ -119,7 +120,7 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&ctl->acc_full[b], 1);
-            mbar_init(&ctl->acc_empty[b], 8);
+            mbar_init(&ctl->acc_empty[b], 2 * kBackWarps);
         }
         ctl->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -275,9 +276,12 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
             }
         }
         __syncwarp();
-    } else if (warp >= 4 && warp < 8) {
+    } else if (warp >= 4) {
         // ------------------------------------------------------------ epilogue (both blocks)
-        const int q = warp - 4;
+        // Eight warps, two per quadrant of the accumulator rows, and a rolled loop over 64-column groups.
+        // With four warps and the tile's 256 erff per thread unrolled, layers with GELU waited for their
+        // read-back and for instructions: 6016 tokens, H = 1472, I = 3008, dense: 166 -> 91 us.
+        const int q = warp & 3, half = (warp - 4) >> 2, w8 = warp - 4;
         const TE* bias = static_cast<const TE*>(g.bias);
         uint32_t tile_n = 0;
         long long w_accfull = 0, w_tmem = 0;
@@ -291,18 +295,16 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
             const uint32_t buf = tile_n & 1, use = tile_n >> 1;
             if (*abort_flag) break;
             {
-                // stage this tile's 256 bias values in shared memory (one private copy per warp,
-                // one 16-byte load per lane) while the main loop of the tile is still running:
-                // global loads issued later would queue behind the operand traffic streaming
-                // into this SM
-                const int nb = pt.nt * BN + 8 * lane;
-                float* bs = &ctl->bias_s[q][8 * lane];
+                // stage the bias of this warp's 128 columns in shared memory (one 8-byte load per lane)
+                // while the main loop of the tile is still running: global loads issued later would
+                // queue behind the operand traffic streaming into this SM
+                const int nb = pt.nt * BN + half * (BN / 2) + 4 * lane;
+                float* bs = &ctl->bias_s[w8][4 * lane];
                 if (nb < g.N) {
-                    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(
-                        bias + (size_t)pt.le * g.N + nb));
+                    const uint2 raw = __ldg(reinterpret_cast<const uint2*>(bias + (size_t)pt.le * g.N + nb));
                     const TE2* h2 = reinterpret_cast<const TE2*>(&raw);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
+                    for (int j = 0; j < 2; ++j) {
                         const float2 f = Pack2<TE>::to_f2(h2[j]);
                         bs[2 * j] = f.x;
                         bs[2 * j + 1] = f.y;
@@ -316,8 +318,8 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                 break;
             }
             tc_fence_after();
-            const int n0 = pt.nt * BN;
-            const uint32_t taddr = tmem_base + buf * BN + (static_cast<uint32_t>(q * 32) << 16);
+            const int n0 = pt.nt * BN + half * (BN / 2);
+            const uint32_t taddr = tmem_base + buf * BN + half * (BN / 2) + (static_cast<uint32_t>(q * 32) << 16);
             // this warp's 32 accumulator rows; rows_w of them carry tokens
             const int rows_w = min(32, rows - q * 32);
             if (rows_w <= 0) {
@@ -327,34 +329,32 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                 continue;
             }
             TE* obase = out_ptr<TE>(g, p, q * 32, n0);
-            uint4* stg = ctl->stage_s[q];
-            // Accumulator read-back, two 32-column chunks in flight.  Every 64 columns the warp
-            // transposes through a swizzled shared-memory tile so that each store instruction
-            // writes four complete 128-byte lines (one row segment per 8 lanes) instead of 32
-            // scattered 16-byte pieces: this is what the NVLink path to a peer's cell needs.
-            uint32_t r[2][32];
-            tmem_ld_32x32(taddr, r[0]);
-#pragma unroll
-            for (int c = 0; c < BN / 32; ++c) {
+            uint4* stg = ctl->stage_s[w8];
+            // Every 64 columns the warp transposes through a swizzled shared-memory tile, sixteen rows
+            // at a time, so that each store instruction writes four complete 128-byte lines (one row
+            // segment per 8 lanes) instead of 32 scattered 16-byte pieces: this is what the NVLink path
+            // to a peer's cell needs.
+#pragma unroll 1
+            for (int cc = 0; cc < BN / 2; cc += 64) {
+                uint32_t r[64];
+                tmem_ld_32x32(taddr + cc, r);
+                tmem_ld_32x32(taddr + cc + 32, r + 32);
                 const long long tq = clock64();
                 tmem_ld_wait();
                 w_tmem += clock64() - tq;
-                if (c + 1 < BN / 32) {
-                    tmem_ld_32x32(taddr + (c + 1) * 32, r[(c + 1) & 1]);
-                } else {
-                    // the whole accumulator is in registers: hand it back to the MMA issuer
+                if (cc + 64 == BN / 2) {
+                    // this warp's part of the accumulator is in registers: hand it back to the MMA issuer
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive_pair(map_to_cta(smem_u32(&ctl->acc_empty[buf]), 0));
                 }
-                const uint32_t* rc = r[c & 1];
-                const float4* bq = reinterpret_cast<const float4*>(&ctl->bias_s[q][c * 32]);
-                uint32_t packed[16];
+                if (n0 + cc >= g.N) continue;
+                const float4* bq = reinterpret_cast<const float4*>(&ctl->bias_s[w8][cc]);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
+                for (int j = 0; j < 32; ++j) {
                     const float4 bf = bq[j >> 1];
-                    float v0 = __uint_as_float(rc[2 * j]) + ((j & 1) ? bf.z : bf.x);
-                    float v1 = __uint_as_float(rc[2 * j + 1]) + ((j & 1) ? bf.w : bf.y);
+                    float v0 = __uint_as_float(r[2 * j]) + ((j & 1) ? bf.z : bf.x);
+                    float v1 = __uint_as_float(r[2 * j + 1]) + ((j & 1) ? bf.w : bf.y);
                     if constexpr (kEpi == 0) {
                         v0 = fmaxf(v0, 0.f);
                         v1 = fmaxf(v1, 0.f);
@@ -363,25 +363,24 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                         v1 = apply_act(v1, 1);
                     }
                     const TE2 h = Pack2<TE>::from_f2(v0, v1);
-                    packed[j] = *reinterpret_cast<const uint32_t*>(&h);
+                    r[j] = *reinterpret_cast<const uint32_t*>(&h);
                 }
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int ch = (c & 1) * 4 + j;  // 16-byte chunk inside the 128-byte row segment
-                    stg[lane * 8 + (ch ^ (lane & 7))] = make_uint4(
-                        packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
-                }
-                if (c & 1) {
+                for (int p0 = 0; p0 < 32; p0 += 16) {
+                    if (p0 >= rows_w) break;
+                    if ((lane & 16) == p0) {
+#pragma unroll
+                        for (int ch = 0; ch < 8; ++ch)
+                            stg[(lane & 15) * 8 + (ch ^ (lane & 7))] =
+                                make_uint4(r[4 * ch], r[4 * ch + 1], r[4 * ch + 2], r[4 * ch + 3]);
+                    }
                     __syncwarp();
-                    const int col0 = (c - 1) * 32;
-                    if (n0 + col0 < g.N) {
 #pragma unroll
-                        for (int it = 0; it < 8; ++it) {
-                            const int rr = it * 4 + (lane >> 3), ch = lane & 7;
-                            const uint4 v = stg[rr * 8 + (ch ^ (rr & 7))];
-                            if (rr < rows_w)
-                                *reinterpret_cast<uint4*>(obase + (size_t)rr * g.N + col0 + ch * 8) = v;
-                        }
+                    for (int it = 0; it < 4; ++it) {
+                        const int rr = it * 4 + (lane >> 3), ch = lane & 7;
+                        const uint4 v = stg[rr * 8 + (ch ^ (rr & 7))];
+                        if (p0 + rr < rows_w)
+                            *reinterpret_cast<uint4*>(obase + (size_t)(p0 + rr) * g.N + cc + ch * 8) = v;
                     }
                     __syncwarp();
                 }

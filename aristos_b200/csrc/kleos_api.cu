@@ -381,9 +381,9 @@ template <typename TE, int kEpi>
 void launch_tc2(bool deep, int grid, cudaStream_t st, const CUtensorMap& map_a, const CUtensorMap& map_b,
                 const GemmArgs& ga) {
     if (deep)
-        launch(ffn_gemm_tc2<TE, kEpi, 2>, grid, 256, gemm_tc2::SMEM_BYTES, st, map_a, map_b, ga);
+        launch(ffn_gemm_tc2<TE, kEpi, 2>, grid, gemm_tc2::kThreads, gemm_tc2::SMEM_BYTES, st, map_a, map_b, ga);
     else
-        launch(ffn_gemm_tc2<TE, kEpi, 1>, grid, 256, gemm_tc2::SMEM_BYTES, st, map_a, map_b, ga);
+        launch(ffn_gemm_tc2<TE, kEpi, 1>, grid, gemm_tc2::kThreads, gemm_tc2::SMEM_BYTES, st, map_a, map_b, ga);
 }
 
 // The persistent kernel, instantiated per activation and per compile-time top-k of the combine.

@@ -20,6 +20,11 @@
 // 350-489,706-741).  Every wait is bounded.  This kernel runs one GEMM over a finished panel
 // list (the dense single-expert layer, and the routed layer when its phases are launched one
 // by one); the persistent kernel in moe_flow.cuh reuses its tile shapes and pipeline.
+//
+// Element types: bf16, fp16, and TF32 words (kind::tf32, torch_dtype 1; the reference's mma.sync
+// m16n8k8 block GEMM, os/processor/mmaConfig.cuh:73-81).  A K slice is 128 bytes of a row and four
+// instructions in either case: 64 16-bit or 32 4-byte elements.
+// ~TF32NOW~
 #pragma once
 
 #include <cuda.h>
@@ -30,7 +35,8 @@
 namespace kleos {
 namespace gemm_tc2 {
 
-constexpr int BM = 128, BN = 256, BK = 64, UMMA_K = 16;
+constexpr int BM = 128, BN = 256, BK = 64, UMMA_K = 16;  // BK: of 16-bit elements
+constexpr int kSteps = BK / UMMA_K;                 // instructions per K slice, 32 bytes of a row each
 constexpr int kSlices = 6;                        // 64-wide K slices of shared memory in total
 constexpr int A_STAGE_BYTES = BM * BK * 2;        // 16 KiB: one K slice of this block's panel
 constexpr int B_STAGE_BYTES = (BN / 2) * BK * 2;  // 16 KiB: one K slice of this block's half weight tile
@@ -84,6 +90,12 @@ __device__ __forceinline__ int total_pair_tiles(const int* le_start, int le_begi
     return total;
 }
 
+template <typename TE>
+__host__ __device__ constexpr uint32_t instr_desc() {
+    if constexpr (sizeof(TE) == 4) return tc::make_instr_desc_tf32(2 * BM, BN);
+    else return tc::make_instr_desc_16b(2 * BM, BN, Pack2<TE>::kMmaFormat);
+}
+
 }  // namespace gemm_tc2
 
 // kEpi selects the fused epilogue at compile time (0: bias + ReLU, 1: bias + GELU, 2: bias only)
@@ -99,8 +111,9 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
     using namespace gemm_tc2;
     constexpr int SUB = kSub, STAGES = kSlices / kSub, STAGE_BYTES = kSub * SLICE_BYTES;
     constexpr int NST = STAGES;
-    constexpr uint32_t kInstrDesc = make_instr_desc_16b(2 * BM, BN, Pack2<TE>::kMmaFormat);
-    using TE2 = typename Pack2<TE>::type;
+    constexpr bool kWide = sizeof(TE) == 4;           // TF32
+    constexpr int BKE = 128 / (int)sizeof(TE);        // elements of a K slice
+    constexpr uint32_t kInstrDesc = instr_desc<TE>();
     const long long t_kernel = clock64();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>(
@@ -144,7 +157,7 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
 
     const int NT = (g.N + BN - 1) / BN;
     const int total = total_pair_tiles(ctl->le_start, g.le_begin, g.le_end, NT);
-    const int KS = g.Kd / BK;                 // 64-wide K slices
+    const int KS = g.Kd / BKE;                // K slices
     const int KB = (KS + SUB - 1) / SUB;      // pipeline stages per tile
     const int n_clusters = (int)gridDim.x >> 1, cluster_id = blockIdx.x >> 1;
 
@@ -175,7 +188,7 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                     const uint32_t full_leader = map_to_cta(smem_u32(&ctl->full[s]), 0);
                     uint8_t* sa = tiles + s * STAGE_BYTES;
                     for (int sub = 0; sub < nsub; ++sub) {
-                        const int kx = (kb * SUB + sub) * BK;
+                        const int kx = (kb * SUB + sub) * BKE;
                         tma_load_2d_pair(sa + sub * SLICE_BYTES, &map_a, kx, p.row_base, full_leader);
                     }
                 }
@@ -213,7 +226,7 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                     const uint32_t full_leader = map_to_cta(smem_u32(&ctl->full[s]), 0);
                     uint8_t* sa = tiles + s * STAGE_BYTES;
                     for (int sub = 0; sub < nsub; ++sub)
-                        tma_load_2d_pair(sa + sub * SLICE_BYTES + A_STAGE_BYTES, &map_b, (kb * SUB + sub) * BK, brow,
+                        tma_load_2d_pair(sa + sub * SLICE_BYTES + A_STAGE_BYTES, &map_b, (kb * SUB + sub) * BKE, brow,
                                          full_leader);
                 }
                 if (!ok) break;
@@ -255,9 +268,11 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                         const uint64_t da = make_smem_desc(sa + sub * SLICE_BYTES);
                         const uint64_t db = make_smem_desc(sa + sub * SLICE_BYTES + A_STAGE_BYTES);
 #pragma unroll
-                        for (int k = 0; k < BK / UMMA_K; ++k)
-                            umma_bf16_pair_if(elected, d_tmem, da + 2 * k, db + 2 * k, kInstrDesc,
-                                              (sub | k) != 0 ? 1u : (uint32_t)(kb != 0));
+                        for (int k = 0; k < kSteps; ++k) {
+                            const uint32_t more = (sub | k) != 0 ? 1u : (uint32_t)(kb != 0);
+                            if constexpr (kWide) umma_tf32_pair_if(elected, d_tmem, da + 2 * k, db + 2 * k, kInstrDesc, more);
+                            else umma_bf16_pair_if(elected, d_tmem, da + 2 * k, db + 2 * k, kInstrDesc, more);
+                        }
                     }
                     // the stage is free in both blocks once these MMAs have read it
                     umma_commit_both_if(elected, bars + (uint32_t)offsetof(Control, empty) + 8 * s);
@@ -295,19 +310,25 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
             const uint32_t buf = tile_n & 1, use = tile_n >> 1;
             if (*abort_flag) break;
             {
-                // stage the bias of this warp's 128 columns in shared memory (one 8-byte load per lane)
+                // stage the bias of this warp's 128 columns in shared memory (one load per lane)
                 // while the main loop of the tile is still running: global loads issued later would
                 // queue behind the operand traffic streaming into this SM
                 const int nb = pt.nt * BN + half * (BN / 2) + 4 * lane;
                 float* bs = &ctl->bias_s[w8][4 * lane];
                 if (nb < g.N) {
-                    const uint2 raw = __ldg(reinterpret_cast<const uint2*>(bias + (size_t)pt.le * g.N + nb));
-                    const TE2* h2 = reinterpret_cast<const TE2*>(&raw);
+                    const TE* src = bias + (size_t)pt.le * g.N + nb;
+                    if constexpr (kWide) {
+                        *reinterpret_cast<float4*>(bs) = __ldg(reinterpret_cast<const float4*>(src));
+                    } else {
+                        using TE2 = typename Pack2<TE>::type;
+                        const uint2 raw = __ldg(reinterpret_cast<const uint2*>(src));
+                        const TE2* h2 = reinterpret_cast<const TE2*>(&raw);
 #pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        const float2 f = Pack2<TE>::to_f2(h2[j]);
-                        bs[2 * j] = f.x;
-                        bs[2 * j + 1] = f.y;
+                        for (int j = 0; j < 2; ++j) {
+                            const float2 f = Pack2<TE>::to_f2(h2[j]);
+                            bs[2 * j] = f.x;
+                            bs[2 * j + 1] = f.y;
+                        }
                     }
                 }
                 __syncwarp();
@@ -330,19 +351,19 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
             }
             TE* obase = out_ptr<TE>(g, p, q * 32, n0);
             uint4* stg = ctl->stage_s[w8];
-            // Every 64 columns the warp transposes through a swizzled shared-memory tile, sixteen rows
-            // at a time, so that each store instruction writes four complete 128-byte lines (one row
-            // segment per 8 lanes) instead of 32 scattered 16-byte pieces: this is what the NVLink path
-            // to a peer's cell needs.
+            // Every 128 bytes of the rows (64 or 32 columns) the warp transposes through a swizzled
+            // shared-memory tile, sixteen rows at a time, so that each store instruction writes four
+            // complete 128-byte lines (one row segment per 8 lanes) instead of 32 scattered 16-byte
+            // pieces: this is what the NVLink path to a peer's cell needs.
 #pragma unroll 1
-            for (int cc = 0; cc < BN / 2; cc += 64) {
-                uint32_t r[64];
+            for (int cc = 0; cc < BN / 2; cc += BKE) {
+                uint32_t r[BKE];
                 tmem_ld_32x32(taddr + cc, r);
-                tmem_ld_32x32(taddr + cc + 32, r + 32);
+                if constexpr (!kWide) tmem_ld_32x32(taddr + cc + 32, r + 32);
                 const long long tq = clock64();
                 tmem_ld_wait();
                 w_tmem += clock64() - tq;
-                if (cc + 64 == BN / 2) {
+                if (cc + BKE == BN / 2) {
                     // this warp's part of the accumulator is in registers: hand it back to the MMA issuer
                     tc_fence_before();
                     __syncwarp();
@@ -351,7 +372,7 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                 if (n0 + cc >= g.N) continue;
                 const float4* bq = reinterpret_cast<const float4*>(&ctl->bias_s[w8][cc]);
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
+                for (int j = 0; j < BKE / 2; ++j) {
                     const float4 bf = bq[j >> 1];
                     float v0 = __uint_as_float(r[2 * j]) + ((j & 1) ? bf.z : bf.x);
                     float v1 = __uint_as_float(r[2 * j + 1]) + ((j & 1) ? bf.w : bf.y);
@@ -362,8 +383,13 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                         v0 = apply_act(v0, 1);
                         v1 = apply_act(v1, 1);
                     }
-                    const TE2 h = Pack2<TE>::from_f2(v0, v1);
-                    r[j] = *reinterpret_cast<const uint32_t*>(&h);
+                    if constexpr (kWide) {
+                        r[2 * j] = __float_as_uint(round_tf32(v0));
+                        r[2 * j + 1] = __float_as_uint(round_tf32(v1));
+                    } else {
+                        const auto h = Pack2<TE>::from_f2(v0, v1);
+                        r[j] = *reinterpret_cast<const uint32_t*>(&h);
+                    }
                 }
 #pragma unroll
                 for (int p0 = 0; p0 < 32; p0 += 16) {
@@ -380,7 +406,7 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                         const int rr = it * 4 + (lane >> 3), ch = lane & 7;
                         const uint4 v = stg[rr * 8 + (ch ^ (rr & 7))];
                         if (p0 + rr < rows_w)
-                            *reinterpret_cast<uint4*>(obase + (size_t)(p0 + rr) * g.N + cc + ch * 8) = v;
+                            *reinterpret_cast<uint4*>(obase + (size_t)(p0 + rr) * g.N + cc + ch * (16 / (int)sizeof(TE))) = v;
                     }
                     __syncwarp();
                 }

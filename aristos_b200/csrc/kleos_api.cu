@@ -25,7 +25,6 @@
 #include "gemm_f32.cuh"
 #include "gemm_simt.cuh"
 #include "gemm_tc2.cuh"
-#include "gemm_tf32.cuh"
 #include "moe_flow.cuh"
 #include "placement.hpp"
 #include "route.cuh"
@@ -102,8 +101,8 @@ struct State {
 
     // tensor maps (rebuilt when the caller's weight pointer changes)
     const void* maps_for_iP = nullptr;
-    // map_w1 / map_w2: whole 256-row weight tiles (TF32 GEMM); map_w1h / map_w2h: the half tile
-    // each block of a pair loads (16-bit GEMMs)
+    // map_w1 / map_w2: weight tiles of the float GEMM; map_w1h / map_w2h: the half tile each block of a
+    // pair loads (16-bit and TF32 GEMMs)
     CUtensorMap map_x{}, map_w1{}, map_y1{}, map_w2{}, map_act{}, map_wg{}, map_w1h{}, map_w2h{}, map_wgh{};
 
     // pipelined host-buffer path (kleos_forward_host_async): double-buffered staging of the
@@ -310,11 +309,11 @@ int ensure_maps(const Sections& s) {
         return KLEOS_OK;
     }
     if (g.use_tf32_tc) {
-        const uint32_t bk = gemm_tf32::BK;
-        if ((rc = make_map(&g.map_x, g.dense ? s.A : g.arena + g.lay.xcell, cell_rows, c.H, gemm_tf32::BM, bk))) return rc;
-        if ((rc = make_map(&g.map_w1, s.W1, (uint64_t)g.nLx * c.I, c.H, gemm_tf32::BN, bk))) return rc;
-        if ((rc = make_map(&g.map_y1, g.y1, cell_rows, c.I, gemm_tf32::BM, bk))) return rc;
-        if ((rc = make_map(&g.map_w2, s.W2, (uint64_t)g.nLx * c.H, c.I, gemm_tf32::BN, bk))) return rc;
+        const uint32_t bk = 32;  // 128 bytes
+        if ((rc = make_map(&g.map_x, g.dense ? s.A : g.arena + g.lay.xcell, cell_rows, c.H, gemm_tc2::BM, bk))) return rc;
+        if ((rc = make_map(&g.map_w1h, s.W1, (uint64_t)g.nLx * c.I, c.H, gemm_tc2::BN / 2, bk))) return rc;
+        if ((rc = make_map(&g.map_y1, g.y1, cell_rows, c.I, gemm_tc2::BM, bk))) return rc;
+        if ((rc = make_map(&g.map_w2h, s.W2, (uint64_t)g.nLx * c.H, c.I, gemm_tc2::BN / 2, bk))) return rc;
         if (c.PX <= 128 && !g.dense) {
             if ((rc = make_map(&g.map_act, s.A, c.S, c.H, route_tc::BM, bk))) return rc;
             if ((rc = make_map(&g.map_wg, s.Wg, c.PX, c.H, c.PX, bk))) return rc;
@@ -396,15 +395,6 @@ void launch_flow(int act, int K, cudaStream_t st, const flow::Args& fa, const CU
     else launch(moe_flow_kernel<TE, 1, 0>, grid, thr, smem, st, g.map_x, g.map_w1h, g.map_y1, g.map_w2h, *fa_act, g.map_wgh, fa);
 }
 
-// TF32 layers: one launch of the kind::tf32 GEMM with the epilogue chosen at compile time.
-void launch_tf32(int epi, cudaStream_t st, const CUtensorMap& map_a, const CUtensorMap& map_b,
-                 const GemmArgs& ga) {
-    const int grid = g.sm_count, smem = gemm_tf32::SMEM_BYTES;
-    if (epi == 0) launch(ffn_gemm_tf32<0>, grid, 256, smem, st, map_a, map_b, ga);
-    else if (epi == 1) launch(ffn_gemm_tf32<1>, grid, 256, smem, st, map_a, map_b, ga);
-    else launch(ffn_gemm_tf32<2>, grid, 256, smem, st, map_a, map_b, ga);
-}
-
 // Float layers: tile width of the split-operand GEMM with N output columns: the one whose rounds of
 // tiles over the block pairs take least time, with the rows an expert gets when the tokens spread
 // evenly.  A 32-wide K slice took 1400 cycles at 128 columns and 950 at 64 (4096 tokens, 16 experts,
@@ -453,8 +443,8 @@ int forward_dense(const Sections& s, const CUtensorMap* map_a, cudaStream_t st, 
     GemmArgs g2 = ga;
     g2.A = g.y1; g2.B = s.W2; g2.bias = s.b2; g2.y1 = s.out; g2.N = c.H; g2.Kd = c.I;
     g2.hidden_act = 2;  // identity
-    if (g.use_tc) {
-        if constexpr (sizeof(T) == 2) {
+    if (g.use_tc || g.use_tf32_tc) {
+        if constexpr (!std::is_same<T, float>::value) {
             const int grid = g.sm_count & ~1;
             const bool deep = c.S >= 512;
             if (c.hidden_act == 0)
@@ -464,10 +454,6 @@ int forward_dense(const Sections& s, const CUtensorMap* map_a, cudaStream_t st, 
             KLEOS_CUDA(mark());
             launch_tc2<T, 2>(deep, grid, st, g.map_y1, g.map_w2h, g2);
         }
-    } else if (g.use_tf32_tc) {
-        launch_tf32(c.hidden_act, st, *map_a, g.map_w1, g1);
-        KLEOS_CUDA(mark());
-        launch_tf32(2, st, g.map_y1, g.map_w2, g2);
     } else if (g.use_f32_tc) {
         launch_f32(g.f32_bn[0], st, *map_a, g.map_w1, g1);
         KLEOS_CUDA(mark());
@@ -637,8 +623,8 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
         g1.stats = g.gemm_stats;
         g2.stats = g.gemm_stats + (size_t)g.sm_count * kStatSlots;
     }
-    if (g.use_tc) {
-        if constexpr (sizeof(T) == 2) {
+    if (g.use_tc || g.use_tf32_tc) {
+        if constexpr (!std::is_same<T, float>::value) {
             const int grid = g.sm_count & ~1;
             const bool deep = (long long)g.world * c.EC >= 512;
             if (c.hidden_act == 0)
@@ -649,11 +635,6 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
             launch_tc2<T, 2>(deep, grid, st, g.map_y1, g.map_w2h, g2);
             KLEOS_CUDA(mark());
         }
-    } else if (g.use_tf32_tc) {
-        launch_tf32(c.hidden_act, st, g.map_x, g.map_w1, g1);
-        KLEOS_CUDA(mark());
-        launch_tf32(2, st, g.map_y1, g.map_w2, g2);
-        KLEOS_CUDA(mark());
     } else if (g.use_f32_tc) {
         launch_f32(g.f32_bn[0], st, g.map_x, g.map_w1, g1);
         KLEOS_CUDA(mark());
@@ -706,16 +687,23 @@ int sync_last_forward() {
 }
 
 template <typename TE>
-int set_tc_attributes() {
+int set_gemm_attributes() {
     const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    KLEOS_CUDA(cudaFuncSetAttribute(route_tc_kernel<TE, 64>, dyn, route_tc::Shape<64>::SMEM_BYTES));
-    KLEOS_CUDA(cudaFuncSetAttribute(route_tc_kernel<TE, 128>, dyn, route_tc::Shape<128>::SMEM_BYTES));
     KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 0, 1>, dyn, gemm_tc2::SMEM_BYTES));
     KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 0, 2>, dyn, gemm_tc2::SMEM_BYTES));
     KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 1, 1>, dyn, gemm_tc2::SMEM_BYTES));
     KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 1, 2>, dyn, gemm_tc2::SMEM_BYTES));
     KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 2, 1>, dyn, gemm_tc2::SMEM_BYTES));
     KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 2, 2>, dyn, gemm_tc2::SMEM_BYTES));
+    return KLEOS_OK;
+}
+
+template <typename TE>
+int set_tc_attributes() {
+    const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    KLEOS_CUDA(cudaFuncSetAttribute(route_tc_kernel<TE, 64>, dyn, route_tc::Shape<64>::SMEM_BYTES));
+    KLEOS_CUDA(cudaFuncSetAttribute(route_tc_kernel<TE, 128>, dyn, route_tc::Shape<128>::SMEM_BYTES));
+    if (const int rc = set_gemm_attributes<TE>()) return rc;
     KLEOS_CUDA(cudaFuncSetAttribute(moe_flow_kernel<TE, 0, 2>, dyn, flow::SMEM_BYTES));
     KLEOS_CUDA(cudaFuncSetAttribute(moe_flow_kernel<TE, 0, 0>, dyn, flow::SMEM_BYTES));
     KLEOS_CUDA(cudaFuncSetAttribute(moe_flow_kernel<TE, 1, 2>, dyn, flow::SMEM_BYTES));
@@ -757,7 +745,7 @@ int ensure_host_pipe() {
             if (rc) return rc;
         } else if ((g.use_tf32_tc && (g.dense || c.PX <= 128)) || (g.use_f32_tc && g.dense)) {
             // same box (128 rows x 32 words) serves the tf32 router and the dense layers' GEMM1
-            int rc = make_map(&hp.map_act[b], hp.act[b], c.S, c.H, gemm_tf32::BM, gemm_tf32::BK);
+            int rc = make_map(&hp.map_act[b], hp.act[b], c.S, c.H, gemm_tc2::BM, 32);
             if (rc) return rc;
         }
     }
@@ -974,9 +962,7 @@ static int initialize_impl(const char* config_json_path, int rank, int world, co
     }
     if (g.use_tf32_tc) {
         const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tf32<0>, dyn, gemm_tf32::SMEM_BYTES));
-        KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tf32<1>, dyn, gemm_tf32::SMEM_BYTES));
-        KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tf32<2>, dyn, gemm_tf32::SMEM_BYTES));
+        if ((rc = set_gemm_attributes<tf32_t>())) return rc;
         KLEOS_CUDA(cudaFuncSetAttribute(route_tc_kernel<tf32_t, 64>, dyn, route_tc::Shape<64>::SMEM_BYTES));
         KLEOS_CUDA(cudaFuncSetAttribute(route_tc_kernel<tf32_t, 128>, dyn, route_tc::Shape<128>::SMEM_BYTES));
     }

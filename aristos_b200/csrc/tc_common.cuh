@@ -262,6 +262,17 @@ __device__ __forceinline__ void umma_bf16_pair_if(uint32_t issue, uint32_t tmem_
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(issue)
         : "memory");
 }
+// 4-byte operands (fp32 words read as TF32), K = 8 per instruction
+__device__ __forceinline__ void umma_tf32_pair_if(uint32_t issue, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
+                                                  uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(issue)
+        : "memory");
+}
 // Arrives on the mbarrier at shared address `bar` of BOTH blocks of the pair once the pair's MMAs issued
 // so far have completed.
 __device__ __forceinline__ void umma_commit_both_if(uint32_t issue, uint32_t bar) {

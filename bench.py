@@ -507,7 +507,7 @@ def run_cuda(args):
         k_flops = 0.5 * ffn_flops
         k_bytes = (active_experts * cfg.I * cfg.H + pairs_per_rank * (cfg.H + cfg.I)) * float(eb)
         k_ms = max_over_ranks(0.5 * (phases["gemm1"] + phases["gemm2"]))
-        kernel_name = {0: "ffn_gemm_simt", 1: "ffn_gemm_tf32"}.get(cfg.torch_dtype, "ffn_gemm_tc2") + \
+        kernel_name = {0: "ffn_gemm_f32"}.get(cfg.torch_dtype, "ffn_gemm_tc2") + \
             " (mean of the GEMM1 and GEMM2 launches)"
     tflops = k_flops / (k_ms * 1e-3) / 1e12
     gbs = k_bytes / (k_ms * 1e-3) / 1e9

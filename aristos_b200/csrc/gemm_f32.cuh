@@ -2,40 +2,47 @@
 //
 // Every fp32 operand is the exact sum of three bf16 values, its leading, middle and trailing eight
 // significand bits (x = h + m + l, each part a truncation of what the parts before it leave), so
-// a product of two operands is nine bf16 products.  The six largest are computed -- l*h, h*l, m*m,
-// m*h, h*m, h*h -- and the three left out are below 2^-22 of the product.  (Splitting fp32 operands
-// over several low-precision products: Henry, Tang, Heinecke, "Leveraging the bfloat16 Artificial
-// Intelligence Datatype For Higher-Precision Computations", ARITH 2019; summing short runs on the
-// matrix unit and the runs in fp32 registers: Ootomo, Yokota, "Recovering single precision accuracy
-// from Tensor Cores", IJHPCA 2022.)  The matrix unit does not round its running sum to nearest, so
-// no sum stays in it for longer than one 32-wide K slice: within a slice the five small products
-// are added up first and the two h*h instructions last, and the slices are summed in registers with
-// ordinary fp32 additions.
+// a product of two operands is nine bf16 products.  All but l*l, which is below 2^-30 of the product,
+// are computed.  (Splitting fp32 operands over several low-precision products: Henry, Tang, Heinecke,
+// "Leveraging the bfloat16 Artificial Intelligence Datatype For Higher-Precision Computations", ARITH
+// 2019; summing short runs on the matrix unit and the runs in fp32 registers: Ootomo, Yokota,
+// "Recovering single precision accuracy from Tensor Cores", IJHPCA 2022.)  The matrix unit does not
+// round its running sum to nearest, so h*h is summed apart from the seven small products, which
+// together are below 2^-6 of it, and no sum stays there for long: the h*h sums are read back every two
+// K slices of 32 (a step) and the small sums every two steps, and both are added up in registers with
+// ordinary fp32 additions.  So a sum of one term is as exact as a rounded fp32 product (at most 2^-24
+// (1 + 2^-4) of it); six products in one accumulator left up to 5e-7.  With the small sums kept for
+// four steps a launch was 2 % faster, and sums of positive terms less exact (2.2e-7, now 1.9e-7).
+//
+// An infinity or NaN among the operands makes the h*h sums what fp32 multiply-adds give: the leading
+// part of such a value is one too.  The small sums beside it are NaN; they are limited to finite values
+// on the way to the registers and so leave an infinity or NaN there as it is.
 //
 // A cluster of two blocks computes a 256 x BN tile (cta_group::2), as in gemm_tc2.cuh.  The parts of the
 // panel go to tensor memory (the MMA's A operand may come from there), those of the weight rows to
-// shared memory: with both in shared memory the six products' operand reads made its bandwidth the
-// limit (per K slice and block at BN = 128: 72 KiB of them, 36 KiB of part stores and 24 KiB each way
-// for the fp32 rows, 1220 cycles at 128 bytes a cycle, against twelve instructions of 64 cycles; now
-// 84 KiB in all, 660 cycles).  BN = 64 is for layers with too few tiles to fill the chip.
+// shared memory: with both in shared memory the eight products' operand reads would make its bandwidth
+// the limit (per K slice and block at BN = 128: 96 KiB of them, 36 KiB of part stores and 24 KiB each way
+// for the fp32 rows, 1440 cycles at 128 bytes a cycle, against sixteen instructions of 64 cycles; this
+// way 92 KiB in all, 736 cycles).  BN = 64 is for layers with too few tiles to fill the chip.
 //
 // Per block, 512 threads:
-//   warps 0..7    drain: the accumulator of every slice is added to the warp's registers (32 rows x
-//                 BN / 2 columns); after a tile's last slice bias, activation and stores
+//   warps 0..7    drain: the sums of every step are added to the warp's registers (32 rows x
+//                 BN / 2 columns); after a tile's last step bias, activation and stores
 //   warps 8..11   split the panel: one row per thread, fp32 slice -> three parts in tensor memory
 //   warps 12, 13  split the weight rows: fp32 slice -> three part planes in shared memory, in the
 //                 swizzle the MMA reads
 //   warp 14       tensor-memory owner; in the leader block also the MMA issuer
 //   warp 15       TMA producer: fp32 rows, 32 columns at a time, into a ring
-// Measured (4096 tokens, 16 experts, H = I = 2048, one launch = 68.7 GFLOP): 368 us, where the FP32
-// FMA kernel (gemm_simt.cuh) took 1630; the layer's output is 7.9e-7 from the 64-bit result (relative
-// 2-norm), before 1.2e-6.  A slice takes 1400 cycles of the 768 its MMAs need.  Slower forms: rows
-// loaded into registers instead of staged by TMA 510 us (the stages leave little L1 for loads in
-// flight), panel parts in shared memory 388, two roles fewer (the same warps split and drain) 420.
-//
-// An output whose sum is not finite (an infinity or NaN among the operands, or an overflow) is
-// computed again as a chain of fp32 multiply-adds, so such values come out as they do in fp32.
+// Measured (4096 tokens, 16 experts, H = I = 2048, one launch = 68.7 GFLOP): 404 us, where the FP32
+// FMA kernel (gemm_simt.cuh) took 1630; the layer's output is 2.9e-7 from the 64-bit result (relative
+// 2-norm), with that kernel 1.2e-6.  A slice takes 1380 cycles of the 1024 its MMAs need.  Slower forms,
+// measured with six products: rows loaded into registers instead of staged by TMA 510 us (the stages
+// leave little L1 for loads in flight) where this form took 368, panel parts in shared memory 388, two
+// roles fewer (the same warps split and drain) 420.
 #pragma once
+
+#include <cfloat>
+#include <type_traits>
 
 #include "gemm_tc2.cuh"
 
@@ -48,7 +55,9 @@ constexpr int ROW = BK * 2;  // bytes of a part row: 64, the swizzle span
 constexpr int kDrain = 8, kSplitA = 4, kSplitB = 2, kSplit = kSplitA + kSplitB;  // warps
 constexpr int kMmaWarp = kDrain + kSplit, kTmaWarp = kMmaWarp + 1;
 constexpr int kThreads = (kTmaWarp + 1) * 32;  // 128 registers a thread
-constexpr int kStages = 4, kMaxRing = 6, kMaxAcc = 4;
+constexpr int kStages = 4, kMaxRing = 6;
+constexpr int kStep = 2;   // K slices whose h*h products share a read-back
+constexpr int kGroup = 2;  // steps whose small products share one
 constexpr int A_COLS = 3 * BK / 2;  // tensor-memory columns of a stage's panel parts, two bf16 a column
 
 struct Control {
@@ -56,8 +65,8 @@ struct Control {
     unsigned long long ring_empty[kMaxRing];  // the team of split warps has read the slot
     unsigned long long full[kStages];         // used on the leader: the slice's parts are in place, a team of both blocks
     unsigned long long done[kStages];         // one per block: the MMAs of the slice have completed
-    unsigned long long acc_full[kMaxAcc];       // one per block: ... and their sums are in tensor memory
-    unsigned long long acc_empty[kMaxAcc];    // used on the leader: the accumulator has been read, drain warps of both blocks
+    unsigned long long sum_full[2];           // one per block: [0] the h*h sums of a step, [1] the small sums of a group are complete
+    unsigned long long sum_empty[2];          // used on the leader: ... and have been read, drain warps of both blocks
     uint32_t tmem_base;
     int abort;
     int last_block;
@@ -72,8 +81,7 @@ struct Shape {
     static constexpr int STAGE_BYTES = 3 * PLANE;
     static constexpr int SLOT_BYTES = (BM + HALF) * BK * 4;  // panel rows, then weight rows
     static constexpr int RING = 6;
-    static constexpr int ACC = BN == 128 ? 2 : 4;        // accumulators
-    static constexpr int A_COL0 = ACC * BN;              // first tensor-memory column of the panel parts
+    static constexpr int A_COL0 = 2 * BN;                // tensor memory: h*h sums, small sums, then the panel parts
     static_assert(A_COL0 + kStages * A_COLS <= 512, "tensor memory has 512 columns");
     static constexpr int STORE_BYTES = kDrain * 1024;    // per drain warp: 8 rows x 32 columns on the way out
     static constexpr int SMEM_BYTES = kStages * STAGE_BYTES + RING * SLOT_BYTES + STORE_BYTES + 1024 + 2048;
@@ -110,18 +118,22 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t* r)
         : "memory");
 }
 
-// Four consecutive fp32 values -> their leading, middle and trailing eight bits as bf16.
+// Four consecutive fp32 values -> their leading, middle and trailing eight bits as bf16.  The leading part
+// of an infinity or NaN is one too (the conversion keeps every NaN a NaN); the other two are then NaN.
 __device__ __forceinline__ void split4(const float4& x, uint2* h, uint2* m, uint2* l) {
     const float v[4] = {x.x, x.y, x.z, x.w};
-    uint32_t top[4], mid[4], low[4];
+    uint32_t top[2], mid[4], low[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        top[k] = __float_as_uint(v[k]);
-        const float r = v[k] - __uint_as_float(top[k] & 0xffff0000u);  // exact
-        mid[k] = __float_as_uint(r);
-        low[k] = __float_as_uint(r - __uint_as_float(mid[k] & 0xffff0000u));
+    for (int k = 0; k < 4; k += 2) {
+        asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(top[k / 2]) : "f"(v[k + 1]), "f"(v[k]));
+        const float r[2] = {v[k] - __uint_as_float(top[k / 2] << 16), v[k + 1] - __uint_as_float(top[k / 2] & 0xffff0000u)};  // exact
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            mid[k + i] = __float_as_uint(r[i]);
+            low[k + i] = __float_as_uint(r[i] - __uint_as_float(mid[k + i] & 0xffff0000u));
+        }
     }
-    *h = make_uint2(__byte_perm(top[0], top[1], 0x7632), __byte_perm(top[2], top[3], 0x7632));
+    *h = make_uint2(top[0], top[1]);
     *m = make_uint2(__byte_perm(mid[0], mid[1], 0x7632), __byte_perm(mid[2], mid[3], 0x7632));
     *l = make_uint2(__byte_perm(low[0], low[1], 0x7632), __byte_perm(low[2], low[3], 0x7632));
 }
@@ -148,14 +160,6 @@ struct Turn {
         }
     }
 };
-
-// One output as the fp32 pipes compute it (K ascending, one chain).
-__device__ __forceinline__ float fma_dot(const float* a, const float* b, int n) {
-    float s = 0.f;
-#pragma unroll 1
-    for (int k = 0; k < n; ++k) s = fmaf(__ldg(a + k), __ldg(b + k), s);
-    return s;
-}
 
 }  // namespace gemm_f32
 
@@ -189,9 +193,9 @@ ffn_gemm_f32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
             mbar_init(&ctl->full[s], 2 * kSplit);
             mbar_init(&ctl->done[s], 1);
         }
-        for (int b = 0; b < Sh::ACC; ++b) {
-            mbar_init(&ctl->acc_full[b], 1);
-            mbar_init(&ctl->acc_empty[b], 2 * kDrain);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&ctl->sum_full[b], 1);
+            mbar_init(&ctl->sum_empty[b], 2 * kDrain);
         }
         ctl->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -216,7 +220,7 @@ ffn_gemm_f32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
     const int KB = g.Kd / BK;
     const int n_clusters = (int)gridDim.x >> 1, cluster_id = (int)blockIdx.x >> 1;
     const int my_tiles = total > cluster_id ? (total - cluster_id + n_clusters - 1) / n_clusters : 0;
-    const int slices = my_tiles * KB;
+    const int slices = my_tiles * KB, steps = KB / kStep;  // (a row is a multiple of 64 long)
 
     if (warp == kTmaWarp) {
         // ------------------------------------------------------------ TMA producer (both blocks)
@@ -251,41 +255,58 @@ ffn_gemm_f32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
     } else if (warp == kMmaWarp) {
         // ------------------------------------------------------------ MMA issuer (leader only)
         if (cta_rank == 0) {
-            // parts of the panel and of the weight rows, smallest products first
-            constexpr int kPartA[6] = {2, 0, 1, 1, 0, 0}, kPartB[6] = {0, 2, 1, 0, 1, 0};
+            // parts of the panel and of the weight rows whose products are summed apart from h*h, smallest first
+            constexpr int kPartA[7] = {2, 1, 2, 0, 1, 1, 0}, kPartB[7] = {1, 2, 0, 2, 1, 0, 1};
             const uint32_t elected = elect_one(), tmem = (uint32_t)uniform((int)tmem_base);
             const uint32_t bars = smem_u32(ctl), parts = smem_u32(stages);
-            const int n = uniform(slices);
-            int s = 0, d = 0;
-            uint32_t sp = 0, dp = 0;  // parities
-            for (int i = 0; i < n; ++i) {
-                if (!mbar_spin(&ctl->full[s], sp, g.wait_cycles, abort_flag) ||
-                    !mbar_spin(&ctl->acc_empty[d], dp ^ 1, g.wait_cycles, abort_flag)) {
-                    if (lane == 0) report_error(g.status, KLEOS_AT_GEMM_MMA, i, (int)g.epoch);
-                    *abort_flag = 1;
-                    break;
-                }
+            const int n = uniform(my_tiles * steps), n_steps = uniform(steps);
+            auto multiply = [&](int s, int pa, int pb, uint32_t d, bool more) {
+                const uint32_t ta = tmem + Sh::A_COL0 + s * A_COLS + pa * (BK / 2);
+                const uint64_t db = part_desc(parts + s * Sh::STAGE_BYTES + pb * Sh::PLANE);
+#pragma unroll
+                for (int k = 0; k < BK / UMMA_K; ++k)
+                    umma_bf16_pair_ta(elected, d, ta + k * (UMMA_K / 2), db + 2 * k, kInstrDesc, (more || k > 0) ? 1u : 0u);
+            };
+            auto wait = [&](unsigned long long* bar, uint32_t parity) {
+                const bool ok = mbar_spin(bar, parity, g.wait_cycles, abort_flag);
                 tc_fence_after();
-                const uint32_t ta = tmem + Sh::A_COL0 + s * A_COLS, sb = parts + s * Sh::STAGE_BYTES;
-                const uint32_t d_tmem = tmem + d * BN;
+                return ok;
+            };
+            int s = 0, kd = 0;                // stage; step of the tile
+            uint32_t sp = 0, hp = 0, lp = 0;  // parities: stages, h*h sums, small sums
+            bool ok = true;
+            for (int i = 0; i < n; ++i) {
+                ok = wait(&ctl->sum_empty[0], hp ^ 1);
+                hp ^= 1;
 #pragma unroll
-                for (int t = 0; t < 6; ++t) {
-                    const uint64_t db = part_desc(sb + kPartB[t] * Sh::PLANE);
-#pragma unroll
-                    for (int k = 0; k < BK / UMMA_K; ++k)
-                        umma_bf16_pair_ta(elected, d_tmem, ta + kPartA[t] * (BK / 2) + k * (UMMA_K / 2), db + 2 * k, kInstrDesc,
-                                          (t | k) != 0 ? 1u : 0u);
+                for (int j = 0; j < kStep; ++j) {
+                    ok = ok && wait(&ctl->full[s + j], sp);
+                    if (ok) multiply(s + j, 0, 0, tmem, j > 0);
                 }
-                umma_commit_both_if(elected, bars + (uint32_t)offsetof(Control, done) + 8 * s);
-                umma_commit_both_if(elected, bars + (uint32_t)offsetof(Control, acc_full) + 8 * d);
-                if (++s == kStages) {
+                if (!ok) break;
+                umma_commit_both_if(elected, bars + (uint32_t)offsetof(Control, sum_full));
+                const bool first = kd % kGroup == 0;
+                if (first) {
+                    if (!(ok = wait(&ctl->sum_empty[1], lp ^ 1))) break;
+                    lp ^= 1;
+                }
+#pragma unroll
+                for (int j = 0; j < kStep; ++j) {
+#pragma unroll
+                    for (int t = 0; t < 7; ++t) multiply(s + j, kPartA[t], kPartB[t], tmem + BN, !first || (j | t) != 0);
+                    umma_commit_both_if(elected, bars + (uint32_t)offsetof(Control, done) + 8 * (s + j));
+                }
+                if (++kd == n_steps) kd = 0;
+                if (kd % kGroup == 0) umma_commit_both_if(elected, bars + (uint32_t)offsetof(Control, sum_full) + 8);
+                s += kStep;
+                if (s == kStages) {
                     s = 0;
                     sp ^= 1;
                 }
-                if (++d == Sh::ACC) {
-                    d = 0;
-                    dp ^= 1;
-                }
+            }
+            if (!ok) {
+                if (lane == 0) report_error(g.status, KLEOS_AT_GEMM_MMA, kd, (int)g.epoch);
+                *abort_flag = 1;
             }
         }
         __syncwarp();
@@ -352,33 +373,46 @@ ffn_gemm_f32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
         float acc[CW];
 #pragma unroll
         for (int j = 0; j < CW; ++j) acc[j] = 0.f;
-        int tile = cluster_id, kd = 0;  // tile the accumulators belong to, its slices added up so far
-        Turn in(Sh::ACC);
-        for (int i = 0; i < slices; ++i) {
-            const int d = in.at;
-            if (!mbar_spin(&ctl->acc_full[d], in.parity, g.wait_cycles, abort_flag)) {
-                if (lane == 0) report_error(g.status, KLEOS_AT_GEMM_EPILOGUE, tile, (int)g.epoch);
-                *abort_flag = 1;
-                break;
-            }
-            in.next();
+        // Adds an accumulator to the registers and hands it back to the MMA issuer.  Small sums are NaN or
+        // infinite only beside h*h sums that are not finite either: limited, they leave those as they are.
+        auto add = [&](int which, uint32_t parity, auto small) -> bool {
+            if (!mbar_spin(&ctl->sum_full[which], parity, g.wait_cycles, abort_flag)) return false;
             tc_fence_after();
-            const uint32_t taddr = tmem_base + d * BN + half * CW + (static_cast<uint32_t>(q * 32) << 16);
+            const uint32_t taddr = tmem_base + which * BN + half * CW + (static_cast<uint32_t>(q * 32) << 16);
 #pragma unroll
             for (int c = 0; c < CW / 32; ++c) {
                 uint32_t v[32];
                 tmem_ld_32x32(taddr + c * 32, v);
                 tmem_ld_wait();
                 if (c + 1 == CW / 32) {
-                    // the whole accumulator is in registers: hand it back to the MMA issuer
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive_pair(map_to_cta(smem_u32(&ctl->acc_empty[d]), 0));
+                    if (lane == 0) mbar_arrive_pair(map_to_cta(smem_u32(&ctl->sum_empty[which]), 0));
                 }
 #pragma unroll
-                for (int j = 0; j < 32; ++j) acc[c * 32 + j] += __uint_as_float(v[j]);
+                for (int j = 0; j < 32; ++j) {
+                    float x = __uint_as_float(v[j]);
+                    if (decltype(small)::value) x = fmaxf(fminf(x, FLT_MAX), -FLT_MAX);
+                    acc[c * 32 + j] += x;
+                }
             }
-            if (++kd < KB) continue;
+            return true;
+        };
+        int tile = cluster_id, kd = 0;  // tile the sums belong to, its steps added up so far
+        uint32_t hp = 0, lp = 0;
+        for (int i = 0; i < my_tiles * steps; ++i) {
+            bool ok = add(0, hp, std::false_type());
+            hp ^= 1;
+            if (++kd == steps || kd % kGroup == 0) {
+                ok = ok && add(1, lp, std::true_type());
+                lp ^= 1;
+            }
+            if (!ok) {
+                if (lane == 0) report_error(g.status, KLEOS_AT_GEMM_EPILOGUE, tile, (int)g.epoch);
+                *abort_flag = 1;
+                break;
+            }
+            if (kd < steps) continue;
             kd = 0;
             // the tile is complete: transpose 32 columns at a time, so that each store instruction
             // writes whole 128-byte lines (the destination may be a peer's cell)
@@ -391,7 +425,6 @@ ffn_gemm_f32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
             const int n0 = pt.nt * BN + half * CW;
             float* obase = out_ptr<float>(g, p, q * 32, n0);
             const float* bq = bias + (size_t)pt.le * g.N + n0;
-            bool finite = true;
 #pragma unroll
             for (int c = 0; c < CW / 32; ++c) {
 #pragma unroll 1
@@ -414,7 +447,6 @@ ffn_gemm_f32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                         const float b4[4] = {bf.x, bf.y, bf.z, bf.w};
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
-                            finite = finite && isfinite(v[k]);
                             v[k] += b4[k];
                             if (g.mode == 0) v[k] = apply_act(v[k], g.hidden_act);
                         }
@@ -425,21 +457,6 @@ ffn_gemm_f32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
             }
 #pragma unroll
             for (int j = 0; j < CW; ++j) acc[j] = 0.f;
-            if (!__all_sync(0xffffffffu, finite)) {
-                // an infinity or NaN (of the operands, or from an overflow) among the warp's sums: all
-                // of them again as fp32 multiply-adds, one column per lane
-                const float* arow = static_cast<const float*>(g.A) + (size_t)(p.row_base + q * 32) * g.Kd;
-#pragma unroll 1
-                for (int c = lane; c < CW && n0 + c < g.N; c += 32) {
-                    const float* brow = static_cast<const float*>(g.B) + ((size_t)pt.le * g.N + n0 + c) * g.Kd;
-#pragma unroll 1
-                    for (int r = 0; r < rows_w; ++r) {
-                        float v = fma_dot(arow + (size_t)r * g.Kd, brow, g.Kd) + __ldg(bq + c);
-                        if (g.mode == 0) v = apply_act(v, g.hidden_act);
-                        obase[(size_t)r * g.N + c] = v;
-                    }
-                }
-            }
         }
     }
 

@@ -397,8 +397,8 @@ void launch_flow(int act, int K, cudaStream_t st, const flow::Args& fa, const CU
 
 // Float layers: tile width of the split-operand GEMM with N output columns: the one whose rounds of
 // tiles over the block pairs take least time, with the rows an expert gets when the tokens spread
-// evenly.  A 32-wide K slice took 1400 cycles at 128 columns and 950 at 64 (4096 tokens, 16 experts,
-// H = I = 2048: 368 and 490 us per launch; 256 tokens, 8 experts, 512 columns: 40 and 32 us).
+// evenly.  A 32-wide K slice takes about 1400 cycles at 128 columns and 950 at 64 (4096 tokens, 16
+// experts, H = I = 2048: 403 and 523 us per launch; 256 tokens, 8 experts, 512 columns: 51 and 43 us).
 int f32_tile_width(int N) {
     const LayerConfig& c = g.cfg;
     const long long rows = g.dense ? c.S : std::min<long long>((long long)g.world * c.EC, ((long long)c.S * c.K + g.nLx - 1) / g.nLx);

@@ -61,3 +61,60 @@ def test_values_that_are_not_finite(monkeypatch, act):
     plain[[3, 40, 70, 130, 200]] = False
     # two fp32 results, each within the layer's bound of the 64-bit one
     assert np.abs(got[plain] - want[plain]).max() <= 2 * hz.TOL[0] * np.abs(want[plain]).max()
+
+
+# tile widths of both GEMMs: 64 columns (one round of tiles either way) and 128 (half as many rounds)
+WIDTHS = pytest.mark.parametrize("S,N", [(256, 512), (2048, 2048)], ids=["narrow", "wide"])
+
+
+@WIDTHS
+def test_rows_of_a_single_term(S, N):
+    """One nonzero activation in a row: every sum is one product, as exact as a rounded fp32 product.
+    Of the product's nine part products the trailing times the trailing one is left out (under 2^-30 of
+    the product), the sum of the small ones is cut off below 2^-28, and the result is rounded once."""
+    rng = np.random.default_rng(S)
+    A = np.zeros((S, N), np.float32)
+    k = rng.integers(0, N, S)
+    A[np.arange(S), k] = (1 + rng.random(S)) * np.exp2(rng.integers(-20, 20, S))
+    W1 = (1 + rng.random((N, N))).astype(np.float32)
+    A[0, k[0]] = W1[0, k[0]] = np.float32(1 + 2.0 ** -7 - 2.0 ** -23)  # long middle and trailing parts
+    zeros = np.zeros(N, np.float32)
+    packed = np.concatenate([A.ravel(), W1.ravel(), np.eye(N, dtype=np.float32).ravel(), zeros, zeros])
+    cfg = _cfg(sequence_len=S, hidden_size=N, intermediate_size=N, num_experts=1, expert_top_k=1)
+    out = hz.run_layer_single_gpu(cfg, packed)[1]
+    want = A.sum(1, dtype=np.float64)[:, None] * W1.T.astype(np.float64)[k]
+    assert (np.abs(out - want) / want).max() <= 2.0 ** -24 * (1 + 2.0 ** -4)
+
+
+@WIDTHS
+def test_a_token_that_is_not_finite_leaves_the_others(S, N):
+    """The other tokens' results are the same bits with and without it."""
+    cfg = _cfg(sequence_len=S, hidden_size=N, intermediate_size=N, num_experts=1, expert_top_k=1, hidden_act=1)
+    packed, _ = hz.make_inputs(cfg, 1, bias_scale=0.5)
+    plain = hz.run_layer_single_gpu(cfg, packed[0])[1]
+    a = packed[0][:S * N].reshape(S, N)
+    a[5, 7], a[40, N - 1], a[S - 1, 0] = np.nan, np.inf, -np.inf
+    got = hz.run_layer_single_gpu(cfg, packed[0])[1]
+    hit = [5, 40, S - 1]
+    assert not np.isfinite(got[hit]).any()
+    assert np.array_equal(np.delete(got, hit, 0), np.delete(plain, hit, 0))
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(sequence_len=4096, hidden_size=1024, intermediate_size=2048, num_experts=4)],
+                         ids=["narrow", "wide"])
+def test_expert_weights_that_are_not_finite(monkeypatch, kw):
+    """Infinities and NaN in a routed layer's weights: the same values as from the FP32 FMA kernel, the
+    experts beside them bit for bit as without."""
+    cfg = _cfg(drop_tokens=0, **kw)
+    packed, views = hz.make_inputs(cfg, 1, bias_scale=0.5)
+    plain = hz.run_layer_single_gpu(cfg, packed[0])[1]
+    v = synth.split_packed(cfg, packed[0], 1)
+    v["W1"][1, 3, 5], v["W2"][2, 9, 70], v["W2"][2, 11, 71], v["W1"][2, 0, 0] = np.inf, -np.inf, np.nan, np.float32(3.4e38)
+    assert not np.isfinite(packed[0]).all()
+    _, got, routing = hz.run_layer_single_gpu(cfg, packed[0])
+    monkeypatch.setenv("KLEOS_DEBUG_SIMT_GEMM", "1")
+    want = hz.run_layer_single_gpu(cfg, packed[0])[1]
+    for same in (np.isnan, np.isposinf, np.isneginf):
+        assert np.array_equal(same(got), same(want)) and same(want).any()
+    untouched = ~np.isin(routing["topk"], [1, 2]).any(1)
+    assert untouched.any() and np.array_equal(got[untouched], plain[untouched])

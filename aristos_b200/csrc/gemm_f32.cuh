@@ -424,6 +424,8 @@ ffn_gemm_f32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
             const int rows_w = min(32, (have ? p.rows : 0) - q * 32);
             const int n0 = pt.nt * BN + half * CW;
             float* obase = out_ptr<float>(g, p, q * 32, n0);
+            // (the result of a dense layer lies where the caller put it)
+            const bool aligned = (reinterpret_cast<uintptr_t>(obase) & 15) == 0;
             const float* bq = bias + (size_t)pt.le * g.N + n0;
 #pragma unroll
             for (int c = 0; c < CW / 32; ++c) {
@@ -450,7 +452,13 @@ ffn_gemm_f32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                             v[k] += b4[k];
                             if (g.mode == 0) v[k] = apply_act(v[k], g.hidden_act);
                         }
-                        *reinterpret_cast<float4*>(obase + (size_t)(hr + r) * g.N + col) = make_float4(v[0], v[1], v[2], v[3]);
+                        float* o = obase + (size_t)(hr + r) * g.N + col;
+                        if (aligned) {
+                            *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) o[k] = v[k];
+                        }
                     }
                     __syncwarp();
                 }

@@ -118,3 +118,24 @@ def test_expert_weights_that_are_not_finite(monkeypatch, kw):
         assert np.array_equal(same(got), same(want)) and same(want).any()
     untouched = ~np.isin(routing["topk"], [1, 2]).any(1)
     assert untouched.any() and np.array_equal(got[untouched], plain[untouched])
+
+
+@WIDTHS
+def test_dense_result_at_any_float(S, N):
+    """The result of a dense float layer may lie at any address that a float may have."""
+    import torch
+    from aristos_b200 import kleos
+    cfg = _cfg(sequence_len=S, hidden_size=N, intermediate_size=N, num_experts=1, expert_top_k=1)
+    iP = torch.from_numpy(hz.make_inputs(cfg, 1, bias_scale=0.5)[0][0]).cuda()
+    kleos.initialize(cfg, 0, 1)
+    try:
+        results = []
+        for offset in (0, 1, 2, 3):
+            buf = torch.full((S * N + 8,), 7.0, device="cuda")
+            kleos.forward_host(iP, buf.data_ptr() + 4 * offset)
+            assert kleos.last_status().code == 0
+            assert (buf[:offset] == 7).all() and (buf[offset + S * N:] == 7).all()
+            results.append(buf[offset:offset + S * N].clone())
+    finally:
+        kleos.finalize()
+    assert all(torch.equal(r, results[0]) for r in results) and not (results[0] == 7).any()

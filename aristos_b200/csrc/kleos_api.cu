@@ -66,6 +66,10 @@ struct State {
     // as ONE persistent kernel (moe_flow.cuh) instead of separate launches.
     bool use_flow = false;
     bool fuse_route = false;                 // ... and the router runs inside it too (KLEOS_FUSE_ROUTE=0: separate launches)
+    // One rank, separate launches: it owns every expert, so the router writes the panel list and the rows
+    // only move inside this GPU's memory, with no flags to raise or to wait for (KLEOS_DISPATCH_KERNELS=1:
+    // the dispatch and plan kernels of several ranks instead)
+    bool local = false;
     bool route_by_flow = false;              // separate launches: the router is the persistent kernel's routing phase alone
     int flow_grid = 0;                       // blocks of the persistent kernel (co-resident pairs x 2)
     flow::Counters* flow_ctr = nullptr;      // [2] scheduler state, see moe_flow.cuh
@@ -487,9 +491,6 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     auto mark = [&]() -> cudaError_t { return timed ? cudaEventRecord(g.ev[evi++], st) : cudaSuccess; };
     KLEOS_CUDA(mark());
 
-    // One rank owns every expert: the router writes the panel list, and the rows only move inside this
-    // GPU's memory, with no flags to raise or to wait for.
-    const bool local = g.world == 1 && !g.use_flow;
     bool routed_in_kernel = g.use_flow && g.fuse_route;
     if (routed_in_kernel) {
         KLEOS_CUDA(mark());
@@ -506,7 +507,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
             fr.pEC = c.pEC; fr.nLx = g.nLx; fr.rank = g.rank; fr.world = g.world; fr.epoch = g.epoch;
             fr.sub = 1; fr.unit_rows = flow::kUnitRows; fr.fuse_route = 1; fr.route_only = 1;
             fr.Wg = s.Wg; fr.gate_bias = g.bias; fr.tile_hist = g.tile_hist; fr.tie_eps = 1e-4f;
-            if (local) { fr.panels = g.panels; fr.le_start = g.le_start; }
+            if (g.local) { fr.panels = g.panels; fr.le_start = g.le_start; }
             launch_flow<T>(c.hidden_act, c.K, st, fr, act_map);
         }
         KLEOS_CUDA(mark());
@@ -546,7 +547,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     for (int r = 0; r < kMaxWorld; ++r) sa.peer_arena[r] = g.peers.arena[r];
     sa.cflag_offset = g.lay.cflag; sa.rank = g.rank; sa.nLx = g.nLx; sa.epoch = g.epoch;
     sa.tile_hist = g.tile_hist;
-    if (local) { sa.panels = g.panels; sa.le_start = g.le_start; }
+    if (g.local) { sa.panels = g.panels; sa.le_start = g.le_start; }
     if (!routed_in_kernel) {
         launch(tile_hist_kernel, (c.S + kSlotTile - 1) / kSlotTile, 256, 0, st, sa);
         launch(slot_kernel, (c.S + kSlotTile - 1) / kSlotTile, 256, 0, st, sa);
@@ -594,7 +595,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     da.lay = g.lay; da.done_counter = g.done_dispatch; da.H = c.H; da.E = c.E; da.EC = c.EC;
     da.pEC = c.pEC; da.nLx = g.nLx; da.rank = g.rank; da.world = g.world; da.epoch = g.epoch;
     da.elem_bytes = c.elem_bytes; da.le_begin = 0; da.le_end = g.nLx;
-    if (local) launch(dispatch_local_kernel, (c.S + kDispatchTokens - 1) / kDispatchTokens, kDispatchTokens * 32, 0, st, LocalDispatchArgs{s.A, g.topk, g.slots, g.arena + g.lay.xcell, c.S, c.K, c.pEC, (unsigned)((size_t)c.H * c.elem_bytes / 16)});
+    if (g.local) launch(dispatch_local_kernel, (c.S + kDispatchTokens - 1) / kDispatchTokens, kDispatchTokens * 32, 0, st, LocalDispatchArgs{s.A, g.topk, g.slots, g.arena + g.lay.xcell, c.S, c.K, c.pEC, (unsigned)((size_t)c.H * c.elem_bytes / 16)});
     else launch(dispatch_kernel, g.sm_count * 4, 256, 0, st, da);
     KLEOS_CUDA(mark());
     // 4. plan: wait for every source's rows, list the panels
@@ -603,7 +604,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     pa.cell_counts = g.cell_counts; pa.status = g.status; pa.world = g.world; pa.nLx = g.nLx;
     pa.pEC = c.pEC; pa.epoch = g.epoch; pa.wait_cycles = g.wait_cycles; pa.rank = g.rank;
     pa.le_begin = 0; pa.le_end = g.nLx;
-    if (!local) launch(plan_kernel, 1, 1024, 0, st, pa);
+    if (!g.local) launch(plan_kernel, 1, 1024, 0, st, pa);
     KLEOS_CUDA(mark());
 
     // 5./6. expert FFN
@@ -976,6 +977,8 @@ static int initialize_impl(const char* config_json_path, int rank, int world, co
     g.use_flow = g.use_tc && !dense && flow_env && flow_env[0] == '1' && g.flow_grid >= 2 &&
                  (size_t)cfg.E * cfg.pEC / kTileM <= (size_t)flow::kMaxPanels && cfg.E <= flow::kMaxCells &&
                  g.nLx <= flow::kMaxLocal;
+    const char* dk = std::getenv("KLEOS_DISPATCH_KERNELS");
+    g.local = world == 1 && !g.use_flow && !(dk && dk[0] == '1');
     const char* fr = std::getenv("KLEOS_FUSE_ROUTE");
     g.fuse_route = g.use_flow && cfg.PX <= 128 && !cfg.is_training && !(fr && fr[0] == '0');
     // Separate launches of a 16-bit layer use the same kernel's routing phase as their router

@@ -188,7 +188,7 @@ __device__ __forceinline__ void warp_scan(F f, int* off, int n) {
 
 // The panel list when every expert is this rank's own, by a whole block that knows the routed rows
 // of every expert (cnt, off: shared memory, off has n + 1 entries).  The router does this in passing,
-// so that a one-rank forward has no dispatch and no plan launch.
+// so that a one-rank forward has no plan launch.
 __device__ __forceinline__ void write_local_plan(const int* cnt, int* off, int n, int pEC, int rank,
                                                  PanelEntry* panels, int* le_start) {
     __syncthreads();

@@ -374,6 +374,7 @@ int launch_route(const RouteArgs& ra, cudaStream_t st, bool prepare = false) {
     };
     if (ra.PX == 64) return one(route_kernel<T, 64>, route_fma::smem_bytes<T, 64>());
     if (ra.PX == 128) return one(route_kernel<T, 128>, route_fma::smem_bytes<T, 128>());
+    if (ra.PX == 192) return one(route_kernel<T, 192>, route_fma::smem_bytes<T, 192>());
     if (ra.PX == 256) return one(route_kernel<T, 256>, route_fma::smem_bytes<T, 256>());
     return fail(KLEOS_E_UNSUPPORTED, "more than 256 experts are not supported by the router");
 }
@@ -940,7 +941,7 @@ static int initialize_impl(const char* config_json_path, int rank, int world, co
     if (const char* gs = std::getenv("KLEOS_GEMM_STATS"))
         if (gs[0] == '1' && (rc = dev_alloc(&g.gemm_stats, (size_t)2 * g.sm_count * kStatSlots))) return rc;
 
-    if (!dense && !((g.use_tc || g.use_tf32_tc) && cfg.PX <= 128) && cfg.PX != 192) {
+    if (!dense && !((g.use_tc || g.use_tf32_tc) && cfg.PX <= 128)) {
         RouteArgs ra{};
         ra.PX = cfg.PX;
         rc = cfg.torch_dtype == 0   ? launch_route<float>(ra, 0, true)

@@ -64,3 +64,26 @@ def test_wide_layers(kw):
     ref = moe_oracle.moe_forward(cfg, 1, views)[0]
     probs, out, routing = hz.run_layer_single_gpu(cfg, packed[0], forwards=2)
     hz.check_against_oracle(cfg, ref, probs, out, routing)
+
+
+@pytest.mark.parametrize("E,kw", [(129, dict(torch_dtype=0, is_training=1)), (160, dict(torch_dtype=2)), (176, dict(torch_dtype=1, is_training=1)),
+                                  (192, dict(torch_dtype=3, expert_top_k=8))], ids=["129-float-training", "160-bf16", "176-tf32-training", "192-fp16"])
+def test_three_column_tiles(E, kw):
+    """129 to 192 experts."""
+    cfg = KleosConfig(sequence_len=384, hidden_size=256, intermediate_size=128, num_experts=E, **kw)
+    packed, views = hz.make_inputs(cfg, 1)
+    ref = moe_oracle.moe_forward(cfg, 1, views)[0]
+    probs, out, routing = hz.run_layer_single_gpu(cfg, packed[0], forwards=2)
+    hz.check_against_oracle(cfg, ref, probs, out, routing)
+    if not cfg.is_training:
+        return
+    import torch
+    info = kleos.initialize(cfg, 0, 1)
+    try:
+        iP, oP = torch.from_numpy(packed[0]).cuda(), torch.zeros(info.output_elems, device="cuda")
+        kleos.forward_host(iP, oP)
+        st = kleos.gate_stats(info)
+    finally:
+        kleos.finalize()
+    assert np.array_equal(st["mean_count"], ref["counts"].astype(np.float32) / np.float32(cfg.S))
+    assert np.abs(st["mean_prob"] - ref["mean_prob"]).max() <= 2e-6

@@ -472,6 +472,7 @@ ffn_gemm_f32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
     // barriers or tensor memory
     tc_fence_before();
     __syncthreads();
+    if (*abort_flag) settle_after_abort();
     cluster_sync_all();
     if (warp == kMmaWarp) {
         tc_fence_after();

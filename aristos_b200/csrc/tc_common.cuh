@@ -65,6 +65,13 @@ __device__ __forceinline__ bool mbar_wait_timed(unsigned long long* bar, uint32_
     return ok;
 }
 
+// For a block that gave up on a wait: copies and MMAs that it has issued go on writing its shared and
+// tensor memory, and end within microseconds.  It returns only after a pause of about half a millisecond.
+__device__ __forceinline__ void settle_after_abort() {
+    const long long t0 = clock64();
+    while (clock64() - t0 < 1000000) __nanosleep(1000);
+}
+
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int x, int y,
                                             unsigned long long* bar) {
     asm volatile(

@@ -24,7 +24,8 @@
 // Element types: bf16, fp16, and TF32 words (kind::tf32, torch_dtype 1; the reference's mma.sync
 // m16n8k8 block GEMM, os/processor/mmaConfig.cuh:73-81).  A K slice is 128 bytes of a row and four
 // instructions in either case: 64 16-bit or 32 4-byte elements.
-// ~TF32NOW~
+// TF32, 4096 tokens, 16 experts, H = I = 2048: 120 and 127 us per launch of 68.7 GFLOP (573 and 541
+// TFLOP/s); the 128 x 256 tiles of single blocks that it replaced took 148.
 #pragma once
 
 #include <cuda.h>

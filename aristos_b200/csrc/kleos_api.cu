@@ -56,7 +56,7 @@ struct State {
     bool use_tc = false;       // 16-bit layers: tcgen05 router and FFN GEMMs
     bool use_f32_tc = false;   // float layers: tcgen05 FFN GEMMs on split operands (the router stays on FP32 FMA)
     int f32_bn[2] = {};        // ... and their tile widths
-    bool use_tf32_tc = false;  // TF32 layers: tcgen05 kind::tf32 FFN GEMMs (the router stays on FP32 FMA)
+    bool use_tf32_tc = false;  // TF32 layers: tcgen05 kind::tf32 FFN GEMMs and, up to 128 experts, router
     // num_experts == 1: the layer is a plain FFN over this rank's tokens (the reference switches
     // to its fffn kernel, moe/moe.cuh:174-177,197-204): no gate, no exchange, and the packed
     // buffers carry no gate weight and no probabilities (moe/fffn.cuh:47-53)

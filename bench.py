@@ -479,9 +479,9 @@ def run_cuda(args):
         pairs_per_rank, active_experts = float(cfg.S), 1
     peaks = load_peaks()
     if cfg.torch_dtype == 0:
-        # float layers run on FP32 FMA (as in the reference): nominal 148 SMs x 128 FMA x 1.965 GHz
-        peaks = dict(peaks, tflops=74.4, tflops_sustained=74.4,
-                     source="nominal fp32 FMA rate (no measured figure)")
+        # float layers multiply split operands: eight bf16 products on the tensor cores per fp32 product
+        peaks = dict(peaks, tflops=peaks["tflops"] / 8, tflops_sustained=peaks["tflops_sustained"] / 8,
+                     source=f"one eighth of the bf16 rate ({peaks['source']}): eight bf16 products per fp32 product")
     elif cfg.torch_dtype == 1:
         peaks = dict(peaks, tflops=1125.0, tflops_sustained=1125.0,
                      source="nominal dense TF32 rate, half the bf16 figure (no measured figure)")

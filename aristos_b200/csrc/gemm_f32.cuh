@@ -3,10 +3,11 @@
 // Every fp32 operand is the exact sum of three bf16 values, its leading, middle and trailing eight
 // significand bits (x = h + m + l, each part a truncation of what the parts before it leave), so
 // a product of two operands is nine bf16 products.  All but l*l, which is below 2^-30 of the product,
-// are computed.  (Splitting fp32 operands over several low-precision products: Henry, Tang, Heinecke,
-// "Leveraging the bfloat16 Artificial Intelligence Datatype For Higher-Precision Computations", ARITH
-// 2019; summing short runs on the matrix unit and the runs in fp32 registers: Ootomo, Yokota,
-// "Recovering single precision accuracy from Tensor Cores", IJHPCA 2022.)  The matrix unit does not
+// are computed.  An operand below 2^-110 loses its bits under 2^-133, the smallest bf16 value.
+// (Splitting fp32 operands over several low-precision products: Henry, Tang, Heinecke, "Leveraging the
+// bfloat16 Artificial Intelligence Datatype For Higher-Precision Computations", ARITH 2019; summing
+// short runs on the matrix unit and the runs in fp32 registers: Ootomo, Yokota, "Recovering single
+// precision accuracy from Tensor Cores", IJHPCA 2022.)  The matrix unit does not
 // round its running sum to nearest, so h*h is summed apart from the seven small products, which
 // together are below 2^-6 of it, and no sum stays there for long: the h*h sums are read back every two
 // K slices of 32 (a step) and the small sums every two steps, and both are added up in registers with

@@ -32,6 +32,12 @@ struct GemmArgs {
     int nLx, pEC, rank, elem_bytes;
     int le_begin, le_end;  // local experts this launch works on
     uint32_t epoch;
+    // ffn_gemm_tc2 only
+    unsigned* next_tile;   // {tiles claimed, block pairs that are done}, both zero between launches
+    int contiguous;        // the rows of a local expert lie one after the other (one source rank)
+    const unsigned* counts;  // contiguous: unclamped rows of every expert, EC of them kept; null: pEC rows of one expert
+    int EC;
+    int plan_ready;        // the plan was complete before the kernel in front of this one began
 };
 
 struct TileCoord {
@@ -54,6 +60,38 @@ __device__ __forceinline__ bool decode_tile(int t, const int* le_start, int le_b
         t -= tiles;
     }
     return false;
+}
+
+// Pairs of panels: the float GEMM gives a tile to two blocks, one panel each.
+struct PairTile {
+    int panel0, n_panels_left, nt, le;
+};
+
+// Tiles ordered by local expert, then N tile, then panel pair.
+__device__ __forceinline__ bool decode_pair_tile(int t, const int* le_start, int le_begin,
+                                                 int le_end, int NT, PairTile* c) {
+    for (int le = le_begin; le < le_end; ++le) {
+        const int p0 = le_start[le], np = le_start[le + 1] - p0;
+        const int npair = (np + 1) >> 1;
+        const int tiles = npair * NT;
+        if (t < tiles) {
+            const int nt = t / npair, pi = t - nt * npair;
+            c->le = le;
+            c->nt = nt;
+            c->panel0 = p0 + 2 * pi;
+            c->n_panels_left = np - 2 * pi;  // 1 when the pair's second panel does not exist
+            return true;
+        }
+        t -= tiles;
+    }
+    return false;
+}
+
+__device__ __forceinline__ int total_pair_tiles(const int* le_start, int le_begin, int le_end,
+                                                int NT) {
+    int total = 0;
+    for (int le = le_begin; le < le_end; ++le) total += ((le_start[le + 1] - le_start[le] + 1) >> 1) * NT;
+    return total;
 }
 
 // Address of output element (row r of the panel, column n) for either mode.

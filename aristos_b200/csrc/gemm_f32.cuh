@@ -19,7 +19,8 @@
 // part of such a value is one too.  The small sums beside it are NaN; they are limited to finite values
 // on the way to the registers and so leave an infinity or NaN there as it is.
 //
-// A cluster of two blocks computes a 256 x BN tile (cta_group::2), as in gemm_tc2.cuh.  The parts of the
+// A cluster of two blocks computes a 256 x BN tile (cta_group::2), as in
+// moe_flow.cuh.  The parts of the
 // panel go to tensor memory (the MMA's A operand may come from there), those of the weight rows to
 // shared memory: with both in shared memory the eight products' operand reads would make its bandwidth
 // the limit (per K slice and block at BN = 128: 96 KiB of them, 36 KiB of part stores and 24 KiB each way
@@ -45,7 +46,8 @@
 #include <cfloat>
 #include <type_traits>
 
-#include "gemm_tc2.cuh"
+#include "gemm_common.cuh"
+#include "tc_common.cuh"
 
 namespace kleos {
 namespace gemm_f32 {
@@ -169,8 +171,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_f32::kThreads, 
 ffn_gemm_f32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, GemmArgs g) {
     using namespace tc;
     using namespace gemm_f32;
-    using gemm_tc2::decode_pair_tile;
-    using gemm_tc2::PairTile;
     using Sh = Shape<BN>;
     constexpr uint32_t kInstrDesc = make_instr_desc_bf16(2 * BM, BN);
     constexpr int CW = BN / 2;  // accumulator columns a drain warp keeps
@@ -217,7 +217,7 @@ ffn_gemm_f32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
     const uint32_t tmem_base = ctl->tmem_base;
 
     const int NT = (g.N + BN - 1) / BN;
-    const int total = gemm_tc2::total_pair_tiles(ctl->le_start, g.le_begin, g.le_end, NT);
+    const int total = total_pair_tiles(ctl->le_start, g.le_begin, g.le_end, NT);
     const int KB = g.Kd / BK;
     const int n_clusters = (int)gridDim.x >> 1, cluster_id = (int)blockIdx.x >> 1;
     const int my_tiles = total > cluster_id ? (total - cluster_id + n_clusters - 1) / n_clusters : 0;

@@ -1,31 +1,38 @@
-// Expert-FFN GEMM with paired blocks (tcgen05 cta_group::2): a cluster of two blocks on
-// neighbouring SMs computes a 256 x 256 output tile -- two 128-row panels of the same local
-// expert against the same 256 weight rows.  Each block TMA-loads its own panel (A) and only
-// HALF of the weight tile (B), so the bytes pulled into an SM per FLOP drop by a third compared
-// with one block per 128 x 256 tile.  Shared memory holds six 64-wide K slices per block, used
-// as six shallow or three deep pipeline stages (template parameter kSub).  The epilogue stages
-// its rows through a swizzled shared-memory tile so that every store instruction writes whole
-// 128-byte lines, also when the destination is a peer's cell.  No load is multicast: every block
-// fetches exactly the bytes it keeps.
+// Expert-FFN GEMM with paired blocks (tcgen05 cta_group::2), weight rows on the MMA's M side and token
+// rows on its N side: a cluster of two blocks on neighbouring SMs computes 256 output columns of up to
+// 288 rows of one local expert.  M is fixed at 256 by the instruction and an FFN has hundreds or
+// thousands of columns; the rows an expert gets are any number, and N takes any multiple of 32.  So
+// the work done for padding is below 32 rows of an expert, and an expert's weights are read once for
+// every 288 of its rows.  (With the rows on M, 128 a block, a layer of 256 rows an expert on average
+// multiplied 1.5 times what it had to: every second expert has some rows above 256, and they took a
+// tile of their own.)
+//
+// Tile = (local expert, 256 columns, up to 288 rows).  Each block TMA-loads 128 weight rows (A) and half
+// of the token rows (B), 64 wide K slices through a ring of six.  Accumulators are a ring in
+// tensor memory, 16 slots of 32 columns: a tile takes as many as its rows need, and the next tile's
+// follow, so that the read-back of one tile runs beside the main loop of the next whatever their sizes.
+// A tile of more than 256 rows, or one whose slots wrap around, is two instructions per K step.
+// No load is multicast: every block fetches exactly the bytes it keeps.
+//
+// Tiles are claimed from a global counter, one ahead, and handed to all roles of both blocks through a
+// ring in shared memory: their sizes differ by up to nine times, so no fixed split is even.
 //
 // Per block, 384 threads:
-//   warp 0      TMA producer (one lane): waits on its own `empty`, loads into its own shared
-//               memory, credits the bytes to the LEADER's `full` barrier
+//   warp 0      TMA producer of the token rows (one lane); in the leader it also claims the tiles
 //   warp 1      leader only: issues tcgen05.mma.cta_group::2, commits to `empty` and
 //               `acc_full` of BOTH blocks
 //   warp 2      tensor-memory allocation / release (both blocks, cta_group::2 forms)
-//   warps 4..11 epilogue of the block's own 128 accumulator rows, half of the columns each; arrives
-//               on the LEADER's `acc_empty`
+//   warp 3      TMA producer of the weight rows (one lane)
+//   warps 4..11 read-back of the block's 128 columns of all the tile's rows: two groups of four warps,
+//               16 rows at a time in turn; arrive on the LEADER's `slot_empty`
 // Work and epilogue semantics follow the reference's tile worker (os/processor/processor.cuh:
 // 350-489,706-741).  Every wait is bounded.  This kernel runs one GEMM over a finished panel
 // list (the dense single-expert layer, and the routed layer when its phases are launched one
-// by one); the persistent kernel in moe_flow.cuh reuses its tile shapes and pipeline.
+// by one).
 //
 // Element types: bf16, fp16, and TF32 words (kind::tf32, torch_dtype 1; the reference's mma.sync
 // m16n8k8 block GEMM, os/processor/mmaConfig.cuh:73-81).  A K slice is 128 bytes of a row and four
 // instructions in either case: 64 16-bit or 32 4-byte elements.
-// TF32, 4096 tokens, 16 experts, H = I = 2048: 120 and 127 us per launch of 68.7 GFLOP (573 and 541
-// TFLOP/s); the 128 x 256 tiles of single blocks that it replaced took 148.
 #pragma once
 
 #include <cuda.h>
@@ -36,107 +43,206 @@
 namespace kleos {
 namespace gemm_tc2 {
 
-constexpr int BM = 128, BN = 256, BK = 64, UMMA_K = 16;  // BK: of 16-bit elements
-constexpr int kSteps = BK / UMMA_K;                 // instructions per K slice, 32 bytes of a row each
-constexpr int kSlices = 6;                        // 64-wide K slices of shared memory in total
-constexpr int A_STAGE_BYTES = BM * BK * 2;        // 16 KiB: one K slice of this block's panel
-constexpr int B_STAGE_BYTES = (BN / 2) * BK * 2;  // 16 KiB: one K slice of this block's half weight tile
-constexpr int SLICE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
+constexpr int BM = 128;                             // output columns (weight rows) per block
+constexpr int kMaxHalf = 144;                       // token rows per block, a multiple of 16
+constexpr int kMaxRows = 2 * kMaxHalf;              // ... per tile
+constexpr int kSlices = 6;                          // K slices of shared memory
+constexpr int W_BYTES = BM * 128;                   // one K slice of the weight rows
+constexpr int SLICE_BYTES = W_BYTES + kMaxHalf * 128;
+constexpr int kSteps = 4;                           // instructions per K slice, 32 bytes of a row each
 constexpr int kBackWarps = 8, kThreads = (4 + kBackWarps) * 32;
-constexpr int TMEM_COLS = 512;  // two accumulators of 256 fp32 columns
-constexpr int SMEM_BYTES = kSlices * SLICE_BYTES + 1024 + 28672;
+constexpr int TMEM_COLS = 512, kSlotCols = 32, kSlots = TMEM_COLS / kSlotCols;
+// tiles on their way: at most six in the K ring, two ahead of it, sixteen in tensor memory
+constexpr int kTasks = 32;
+constexpr int STG_ROW = BM * 2 + 16;                // bytes of a staged row: padded, so that eight rows meet no bank conflict
+constexpr int kCtlBytes = 22528;
+constexpr int SMEM_BYTES = kSlices * SLICE_BYTES + 1024 + kCtlBytes;
+static_assert(SMEM_BYTES <= 232448, "227 KiB of shared memory per block");
+static_assert(SLICE_BYTES % 1024 == 0, "the swizzle repeats every 1024 bytes");
+
+// Token rows as boxes, 128 bytes wide, of the heights below: a K slice of a tile is one copy, of the lowest box
+// that holds the block's rows.  (Made up of boxes of 32 and 16 rows, 96 rows took three copies a slice, and
+// a layer of 384 rows and K = 8192 ran 0.72 times as fast as with one of 128.)
+constexpr int kBoxes = 6;
+struct RowMaps {
+    CUtensorMap box[kBoxes];
+};
+__host__ __device__ constexpr int box_rows(int i) { return i == 0 ? 16 : i == 1 ? 32 : i == 2 ? 64 : i == 3 ? 96 : i == 4 ? 128 : kMaxHalf; }
+__device__ __forceinline__ int box_of(int rows) {
+    int i = 0;
+    while (box_rows(i) < rows) ++i;
+    return i;
+}
+
+// A tile, as the scheduler hands it to the other roles.  Block r of the pair loads rows[r] token rows from
+// row_base[r] on; `half` of them, a multiple of 16, go into the MMA from each block.
+struct __align__(16) Task {
+    int half;          // 0: no more tiles
+    int le, mt;        // local expert, 256-column tile
+    int src;           // source ranks, eight bits each
+    int row_base[2], rows[2];
+};
 
 struct Control {
-    unsigned long long full[kSlices];   // used on the leader (one per pipeline stage)
-    unsigned long long empty[kSlices];  // one per block
-    unsigned long long acc_full[2];    // one per block
-    unsigned long long acc_empty[2];   // used on the leader, 16 arrivals (8 warps x 2 blocks)
+    unsigned long long full[kSlices];    // used on the leader
+    unsigned long long empty[kSlices];   // one per block
+    unsigned long long acc_full[kSlots];     // one per block, tile i uses [i % kSlots]
+    unsigned long long slot_empty[kSlots];   // used on the leader, 16 arrivals (8 warps x 2 blocks)
+    unsigned long long task_full[kTasks];    // one per block
+    unsigned long long begun[2];             // leader: the loads of tile i have begun, [i % 2]
     uint32_t tmem_base;
     int abort;
-    int le_start[257];
-    __align__(16) float bias_s[kBackWarps][BN / 2];   // bias of the columns being read back, per epilogue warp
-    __align__(16) uint4 stage_s[kBackWarps][16 * 8];  // per epilogue warp: 16 rows x 128 bytes, swizzled
+    bool last_block;
+    Task task[kTasks];
+    int rows[256];        // contiguous: rows of every local expert
+    int splits[256];      // tiles along the rows of every local expert
+    int first[257];       // tiles before every local expert
+    __align__(16) unsigned char stage[2][2][16 * STG_ROW];  // per read-back group, two turns: 16 rows x 256 bytes
 };
+static_assert(sizeof(Control) <= kCtlBytes, "control block must fit the shared memory set aside for it");
+constexpr int kBarriers = offsetof(Control, tmem_base) / 8;
+static_assert(kBarriers <= kThreads, "a thread per barrier");
 
-static_assert(sizeof(Control) <= 28672, "control block must fit the shared memory set aside for it");
+// Tiles along the rows of an expert.  A K slice of a tile of n rows takes the larger of 2 n cycles of the
+// tensor pipe and n + 256 of shared memory (32 KiB + 128 n bytes of operand reads and TMA writes);
+// one of more than 256 rows is two instructions a step, which read the weights twice: 672 cycles at 288
+// rows.  So 257 to 288 rows are best taken as one tile, and more of them 256 at a time.
+__device__ __forceinline__ int row_splits(int rows) {
+    return rows <= kMaxRows ? (rows + kMaxRows - 1) / kMaxRows : (rows + 255) / 256;
+}
 
-struct PairTile {
-    int panel0, n_panels_left, nt, le;
-};
-
-// Tiles ordered by local expert, then N tile, then panel pair.
-__device__ __forceinline__ bool decode_pair_tile(int t, const int* le_start, int le_begin,
-                                                 int le_end, int NT, PairTile* c) {
-    for (int le = le_begin; le < le_end; ++le) {
-        const int p0 = le_start[le], np = le_start[le + 1] - p0;
-        const int npair = (np + 1) >> 1;
-        const int tiles = npair * NT;
-        if (t < tiles) {
-            const int nt = t / npair, pi = t - nt * npair;
-            c->le = le;
-            c->nt = nt;
-            c->panel0 = p0 + 2 * pi;
-            c->n_panels_left = np - 2 * pi;  // 1 when the pair's second panel does not exist
-            return true;
-        }
-        t -= tiles;
+// Tiles in order of local expert, column tile, rows: tiles that run together read the same weights.
+// `le` is the caller's place in the list (its tiles only grow).
+__device__ __forceinline__ Task decode_task(int t, const Control* ctl, const GemmArgs& g, int* le) {
+    int e = *le;
+    while (ctl->first[e + 1] <= t) ++e;
+    *le = e;
+    const int splits = ctl->splits[e], r = t - ctl->first[e];
+    Task x;
+    x.le = e;
+    x.mt = r / splits;
+    const int j = r - x.mt * splits;
+    if (g.contiguous) {
+        const int rows = ctl->rows[e];
+        const int per = ((rows + splits - 1) / splits + 31) >> 5 << 5;
+        const int left = min(per, rows - j * per);
+        x.half = ((left + 31) >> 5) << 4;
+        x.row_base[0] = e * g.pEC + j * per;
+        x.rows[0] = min(x.half, left);
+        x.row_base[1] = x.row_base[0] + x.half;
+        x.rows[1] = left - x.rows[0];
+        x.src = g.rank | (g.rank << 8);
+    } else {
+        const int p0 = g.le_start[e] + 2 * j;
+        const bool second = p0 + 1 < g.le_start[e + 1];
+        const PanelEntry a = g.panels[p0], b = g.panels[second ? p0 + 1 : p0];
+        x.row_base[0] = a.row_base;
+        x.row_base[1] = b.row_base;  // (without a second panel its block re-reads the first one and discards)
+        x.rows[0] = a.rows;
+        x.rows[1] = second ? b.rows : 0;
+        x.src = a.src | (b.src << 8);
+        x.half = (max(x.rows[0], x.rows[1]) + 15) >> 4 << 4;
     }
-    return false;
+    return x;
 }
 
-__device__ __forceinline__ int total_pair_tiles(const int* le_start, int le_begin, int le_end,
-                                                int NT) {
-    int total = 0;
-    for (int le = le_begin; le < le_end; ++le) total += ((le_start[le + 1] - le_start[le] + 1) >> 1) * NT;
-    return total;
-}
+// The slots of a tile that starts at ring position `at`: as one run, or as two when they wrap around or
+// are more than the 256 columns of an instruction.
+struct Runs {
+    int n0, n1;       // slots
+    int slot0, slot1;
+    __device__ __forceinline__ Runs(uint32_t at, int half) {
+        const int n = half >> 4, room = kSlots - (int)(at % kSlots);
+        slot0 = (int)(at % kSlots);
+        n0 = n > room ? room : n > 8 ? (n + 1) >> 1 : n;
+        n1 = n - n0;
+        slot1 = (slot0 + n0) % kSlots;
+    }
+};
 
 template <typename TE>
-__host__ __device__ constexpr uint32_t instr_desc() {
-    if constexpr (sizeof(TE) == 4) return tc::make_instr_desc_tf32(2 * BM, BN);
-    else return tc::make_instr_desc_16b(2 * BM, BN, Pack2<TE>::kMmaFormat);
+__host__ __device__ constexpr uint32_t instr_desc() {  // N = 0
+    if constexpr (sizeof(TE) == 4) return tc::make_instr_desc_tf32(2 * BM, 0);
+    else return tc::make_instr_desc_16b(2 * BM, 0, Pack2<TE>::kMmaFormat);
+}
+
+// 16 lanes x 16 columns as two 16 x 8 fragments: register 4 x + 2 h + i of thread t is lane t / 4 + 8 h,
+// column 8 x + 2 (t % 4) + i
+__device__ __forceinline__ void tmem_ld_16x256_x2(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+// Four 8 x 8 blocks of 16-bit elements, transposed: thread 8 i + j gives the address of column j of block i.
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, const uint32_t* r) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};"
+                 ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])
+                 : "memory");
+}
+__device__ __forceinline__ bool try_wait_cluster(unsigned long long* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(tc::smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// Whether all 128 threads that meet at the barrier say yes.
+__device__ __forceinline__ bool all_of_group(bool yes, int barrier) {
+    uint32_t all;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %1, 0;\n\t"
+        "bar.red.and.pred q, %2, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(all)
+        : "r"((uint32_t)yes), "r"(barrier)
+        : "memory");
+    return all != 0;
+}
+__device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, uint4 v) {
+    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+                 : "memory");
+}
+// An arrival that announces nothing in memory: the tensor-memory reads before it have completed (tcgen05.wait::ld).
+// With release semantics it would wait for the thread's result rows on their way to global memory.
+__device__ __forceinline__ void arrive_relaxed(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 
 }  // namespace gemm_tc2
 
 // kEpi selects the fused epilogue at compile time (0: bias + ReLU, 1: bias + GELU, 2: bias only)
 // so the read-back loop stays a short straight-line sequence.
-// kSub = 64-wide K slices per pipeline stage: 1 gives six shallow stages (best when the weights
-// stream from HBM), 2 gives three deep stages and half the barrier round trips (best when the
-// operands come from L2 and the tensor pipe is the limit).
-template <typename TE, int kEpi, int kSub>
+// (Six stages of one K slice: three of two slices, with half the barrier round trips, took 1516 us instead of 1505
+// on the layer of 4096 tokens, H = 4096, I = 14336, 8 experts, and 65.3 instead of 64.3 on the dense layer of
+// 4096 tokens, H = I = 2048.)
+template <typename TE, int kEpi>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_tc2::kThreads, 1)
-ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-             GemmArgs g) {
+ffn_gemm_tc2(const __grid_constant__ gemm_tc2::RowMaps map_x, const __grid_constant__ CUtensorMap map_w, GemmArgs g) {
     using namespace tc;
     using namespace gemm_tc2;
-    constexpr int SUB = kSub, STAGES = kSlices / kSub, STAGE_BYTES = kSub * SLICE_BYTES;
-    constexpr int NST = STAGES;
     constexpr bool kWide = sizeof(TE) == 4;           // TF32
     constexpr int BKE = 128 / (int)sizeof(TE);        // elements of a K slice
-    constexpr uint32_t kInstrDesc = instr_desc<TE>();
     const long long t_kernel = clock64();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     Control* ctl = reinterpret_cast<Control*>(tiles + kSlices * SLICE_BYTES);
-    __shared__ bool last_block;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t cta_rank = cluster_ctarank();
     const bool leader = cta_rank == 0;
     volatile int* abort_flag = &ctl->abort;
 
-    if (tid == 0) {
-        for (int s = 0; s < NST; ++s) {
-            mbar_init(&ctl->full[s], 1);
-            mbar_init(&ctl->empty[s], 1);
-        }
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(&ctl->acc_full[b], 1);
-            mbar_init(&ctl->acc_empty[b], 2 * kBackWarps);
-        }
-        ctl->abort = 0;
+    if (tid < kBarriers) {  // one each: they lie one after the other at the start of Control
+        const int first_slot = (int)(offsetof(Control, slot_empty) / 8);
+        mbar_init(reinterpret_cast<unsigned long long*>(ctl) + tid, tid >= first_slot && tid < first_slot + kSlots ? 2 * kBackWarps : 1);
+        if (tid == 0) ctl->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 2) {
@@ -145,54 +251,100 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
-    pdl_wait();
-    pdl_trigger();
-    for (int i = tid; i <= g.nLx; i += blockDim.x) ctl->le_start[i] = g.le_start[i];
-    tc_fence_before();
+    // What the second GEMM of a forward needs to know of the plan was written before the first one began
+    // (whose blocks let this launch start only once they had waited for it), and no kernel writes the
+    // weights: its first weight slices are on their way before the first GEMM has ended.
+    if (!g.plan_ready) pdl_wait();
+    const int MT = (g.N + 2 * BM - 1) / (2 * BM);
+    for (int e = tid; e < g.nLx; e += kThreads) {
+        const bool in = e >= g.le_begin && e < g.le_end;
+        if (g.contiguous) {
+            ctl->rows[e] = !in ? 0 : g.counts ? (int)min(g.counts[e], (unsigned)g.EC) : g.pEC;
+            ctl->splits[e] = row_splits(ctl->rows[e]);
+        } else {
+            ctl->splits[e] = in ? (g.le_start[e + 1] - g.le_start[e] + 1) >> 1 : 0;
+        }
+    }
     __syncthreads();
-    cluster_sync_all();  // both blocks' barriers exist before anything remote touches them
+    const int n_clusters = (int)gridDim.x >> 1, cluster_id = blockIdx.x >> 1;
+    if (warp == 0) {
+        warp_scan([&](int e) { return ctl->splits[e] * MT; }, ctl->first, g.nLx);
+        __syncwarp();
+        // the pair's first tile needs no claim: each block decodes it for itself
+        if (lane == 0) {
+            int le = 0;
+            Task x{};
+            if (cluster_id < ctl->first[g.nLx]) x = decode_task(cluster_id, ctl, g, &le);
+            ctl->task[0] = x;
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    cluster_sync_all();  // (a barrier of both blocks; their mbarriers exist before anything remote touches them)
     tc_fence_after();
     const uint32_t tmem_base = ctl->tmem_base;
     if (g.stats && tid == 0) g.stats[blockIdx.x * kStatSlots + 8] = clock64() - t_kernel;
-    auto panel_at = [&](int i) -> PanelEntry { return g.panels[i]; };
+    if (warp != 3 || !g.plan_ready) pdl_wait();
+    if (warp == 0) pdl_trigger();
 
-    const int NT = (g.N + BN - 1) / BN;
-    const int total = total_pair_tiles(ctl->le_start, g.le_begin, g.le_end, NT);
     const int KS = g.Kd / BKE;                // K slices
-    const int KB = (KS + SUB - 1) / SUB;      // pipeline stages per tile
-    const int n_clusters = (int)gridDim.x >> 1, cluster_id = blockIdx.x >> 1;
+
+    // Tile i of this pair.  The ring needs no "empty" signal, see kTasks.  After a failed wait: no more tiles.
+    auto take = [&](uint32_t i, int where) -> Task {
+        if (i == 0) return ctl->task[0];
+        unsigned long long* bar = &ctl->task_full[(i - 1) % kTasks];
+        const uint32_t parity = ((i - 1) / kTasks) & 1u;
+        bool ok = try_wait_cluster(bar, parity);
+        if (!ok) {
+            const long long t0 = clock64();
+            uint32_t polls = 0;
+            while (!(ok = try_wait_cluster(bar, parity))) {
+                __nanosleep(40);
+                if ((++polls & 31u) == 0) {
+                    if (*abort_flag) break;
+                    if (clock64() - t0 > g.wait_cycles) {
+                        report_error(g.status, where, -2 - (int)i, (int)g.epoch);
+                        *abort_flag = 1;
+                        break;
+                    }
+                }
+            }
+        }
+        Task x = ctl->task[i % kTasks];
+        if (!ok) x.half = 0;
+        return x;
+    };
 
     if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer (both blocks)
+        // ------------------------------------------------------------ token rows (both blocks)
         if (lane == 0) {
             asm volatile("fence.proxy.async;" ::: "memory");
             uint32_t it = 0;
             long long w_empty = 0;
             const long long t_begin = clock64();
-            for (int t = cluster_id; t < total && !*abort_flag; t += n_clusters) {
-                PairTile pt;
-                if (!decode_pair_tile(t, ctl->le_start, g.le_begin, g.le_end, NT, &pt)) break;
-                // the block without a panel of its own re-reads the first one and discards
-                const int my_panel = pt.panel0 + ((int)cta_rank < pt.n_panels_left ? (int)cta_rank : 0);
-                const PanelEntry p = panel_at(my_panel);
-                for (int kb = 0; kb < KB; ++kb, ++it) {
-                    const int s = it % NST;
-                    const uint32_t ph = (it / NST) & 1;
+            for (uint32_t i = 0;; ++i) {
+                const Task x = take(i, KLEOS_AT_GEMM_PRODUCER);
+                if (x.half == 0) break;
+                if (leader) mbar_arrive(&ctl->begun[i & 1]);
+                const int row = leader ? x.row_base[0] : x.row_base[1];
+                const int box = box_of(x.half);
+                const CUtensorMap* map = &map_x.box[box];
+                const uint32_t bytes = 2u * (uint32_t)(W_BYTES + box_rows(box) * 128);
+                bool ok = true;
+                for (int kb = 0; kb < KS; ++kb, ++it) {
+                    const int s = it % kSlices;
+                    const uint32_t ph = (it / kSlices) & 1;
                     if (!mbar_wait_timed(&ctl->empty[s], ph ^ 1, g.wait_cycles, abort_flag, &w_empty)) {
-                        report_error(g.status, KLEOS_AT_GEMM_PRODUCER, t, (int)g.epoch);
+                        report_error(g.status, KLEOS_AT_GEMM_PRODUCER, (int)i, (int)g.epoch);
                         *abort_flag = 1;
+                        ok = false;
                         break;
                     }
                     // the leader announces the bytes of both blocks on its own barrier
-                    const int nsub = min(SUB, KS - kb * SUB);
-                    if (leader) mbar_expect_tx(&ctl->full[s], 2 * nsub * SLICE_BYTES);
-                    const uint32_t full_leader = map_to_cta(smem_u32(&ctl->full[s]), 0);
-                    uint8_t* sa = tiles + s * STAGE_BYTES;
-                    for (int sub = 0; sub < nsub; ++sub) {
-                        const int kx = (kb * SUB + sub) * BKE;
-                        tma_load_2d_pair(sa + sub * SLICE_BYTES, &map_a, kx, p.row_base, full_leader);
-                    }
+                    if (leader) mbar_expect_tx(&ctl->full[s], bytes);
+                    tma_load_2d_pair(tiles + s * SLICE_BYTES + W_BYTES, map, kb * BKE, row, map_to_cta(smem_u32(&ctl->full[s]), 0));
                 }
+                if (!ok) break;
             }
             if (g.stats) {
                 g.stats[blockIdx.x * kStatSlots + 0] = w_empty;
@@ -201,36 +353,59 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
         }
         __syncwarp();
     } else if (warp == 3) {
-        // ------------------------------------------------------------ second TMA producer (both blocks)
-        // The weight slices are issued by a thread of their own, next to the panel slices of
-        // warp 0 (measured: 1.6 % off the launch).  It waits for the same free-stage barrier and
-        // its bytes complete on the same full barrier; the byte count announced by warp 0 covers
-        // both, and a slice landing before that announcement only makes the barrier's byte
-        // count negative for a moment (the phase cannot complete before warp 0 has arrived).
+        // ------------------------------------------------------------ weight rows (both blocks)
+        // They wait for the same free-stage barrier as the token rows and complete on the same full
+        // barrier; the byte count announced by warp 0 covers both, and a slice landing before
+        // that announcement only makes the barrier's byte count negative for a moment (the phase
+        // cannot complete before warp 0 has arrived).
         if (lane == 0) {
             asm volatile("fence.proxy.async;" ::: "memory");
             uint32_t it = 0;
             long long w_unused = 0;
-            for (int t = cluster_id; t < total && !*abort_flag; t += n_clusters) {
-                PairTile pt;
-                if (!decode_pair_tile(t, ctl->le_start, g.le_begin, g.le_end, NT, &pt)) break;
-                const int brow = pt.le * g.N + pt.nt * BN + (int)cta_rank * (BN / 2);
+            for (uint32_t i = 0;; ++i) {
+                const Task x = take(i, KLEOS_AT_GEMM_PRODUCER);
+                if (x.half == 0) break;
+                // past the last column the block loads its partner's rows again and discards the results
+                const int col = x.mt * 2 * BM + (int)cta_rank * BM;
+                const int brow = x.le * g.N + (col < g.N ? col : x.mt * 2 * BM);
                 bool ok = true;
-                for (int kb = 0; kb < KB; ++kb, ++it) {
-                    const int s = it % NST;
-                    const uint32_t ph = (it / NST) & 1;
+                for (int kb = 0; kb < KS; ++kb, ++it) {
+                    const int s = it % kSlices;
+                    const uint32_t ph = (it / kSlices) & 1;
                     if (!mbar_wait_timed(&ctl->empty[s], ph ^ 1, g.wait_cycles, abort_flag, &w_unused)) {
                         ok = false;  // the first producer reports the failure
                         break;
                     }
-                    const int nsub = min(SUB, KS - kb * SUB);
                     const uint32_t full_leader = map_to_cta(smem_u32(&ctl->full[s]), 0);
-                    uint8_t* sa = tiles + s * STAGE_BYTES;
-                    for (int sub = 0; sub < nsub; ++sub)
-                        tma_load_2d_pair(sa + sub * SLICE_BYTES + A_STAGE_BYTES, &map_b, (kb * SUB + sub) * BKE, brow,
-                                         full_leader);
+                    tma_load_2d_pair(tiles + s * SLICE_BYTES, &map_w, kb * BKE, brow, full_leader);
                 }
                 if (!ok) break;
+            }
+        }
+        __syncwarp();
+    } else if (warp == 2) {
+        // ------------------------------------------------------------ scheduler (leader only)
+        // Claims a tile when the loads of the tile before it have begun, and hands it, decoded, to
+        // all roles of both blocks.
+        if (leader && lane == 0 && ctl->task[0].half != 0) {
+            const int total = ctl->first[g.nLx];
+            int le = 0;
+            bool ok = true;
+            long long w_unused = 0;
+            for (uint32_t i = 1; ok; ++i) {
+                ok = mbar_wait_timed(&ctl->begun[(i - 1) & 1], ((i - 1) >> 1) & 1, g.wait_cycles, abort_flag, &w_unused);
+                if (!ok) break;  // (the roles report what they wait for)
+                const unsigned t = (unsigned)n_clusters + atomicAdd(g.next_tile, 1u);
+                Task x{};
+                if (t < (unsigned)total) x = decode_task((int)t, ctl, g, &le);
+                ctl->task[i % kTasks] = x;
+                const uint32_t peer = map_to_cta(smem_u32(&ctl->task[i % kTasks]), 1);
+                st_cluster_v4(peer, *reinterpret_cast<const uint4*>(&x));
+                st_cluster_v4(peer + 16, *(reinterpret_cast<const uint4*>(&x) + 1));
+                const uint32_t bar = smem_u32(&ctl->task_full[(i - 1) % kTasks]);
+                mbar_arrive_cluster(map_to_cta(bar, 0));
+                mbar_arrive_cluster(map_to_cta(bar, 1));
+                ok = x.half != 0;
             }
         }
         __syncwarp();
@@ -240,50 +415,61 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
         if (leader) {
             const uint32_t elected = elect_one();
             const uint32_t slices = smem_u32(tiles), bars = smem_u32(ctl), tmem = (uint32_t)uniform((int)tmem_base);
-            const int n_tiles = uniform(total);
-            uint32_t s = 0, ph = 0, tile_n = 0;
+            uint32_t s = 0, ph = 0, at = 0;
             long long w_acc = 0, w_full = 0;
             const long long t_begin = clock64();
-            for (int t = cluster_id; t < n_tiles; t += n_clusters, ++tile_n) {
-                const uint32_t buf = tile_n & 1, use = tile_n >> 1;
-                if (!mbar_wait_timed(&ctl->acc_empty[buf], (use & 1) ^ 1, g.wait_cycles, abort_flag, &w_acc)) {
-                    if (lane == 0) report_error(g.status, KLEOS_AT_GEMM_MMA, t, (int)g.epoch);
+            for (uint32_t i = 0;; ++i) {
+                const int half = uniform(take(i, KLEOS_AT_GEMM_MMA).half);
+                if (half == 0) break;
+                const Runs runs(at, half);
+                bool ok = true;
+                {
+                    // a lane per slot
+                    const uint32_t slot = at + (uint32_t)lane;
+                    if (lane < runs.n0 + runs.n1)
+                        ok = mbar_wait_timed(&ctl->slot_empty[slot % kSlots], ((slot / kSlots) & 1) ^ 1, g.wait_cycles, abort_flag, &w_acc);
+                    ok = __all_sync(0xffffffffu, ok);
+                }
+                if (!ok) {
+                    if (lane == 0) report_error(g.status, KLEOS_AT_GEMM_MMA, (int)i, (int)g.epoch);
                     *abort_flag = 1;
                     break;
                 }
+                at += runs.n0 + runs.n1;
                 tc_fence_after();
-                const uint32_t d_tmem = tmem + buf * BN;
-                bool ok = true;
-                for (int kb = 0; kb < KB; ++kb) {
+                // N of a run: 32 columns a slot, 16 rows of each block
+                const uint32_t idesc0 = instr_desc<TE>() | ((uint32_t)runs.n0 << 19), idesc1 = instr_desc<TE>() | ((uint32_t)runs.n1 << 19);
+                const uint32_t d0 = tmem + runs.slot0 * kSlotCols, d1 = tmem + runs.slot1 * kSlotCols;
+                const uint32_t off1 = (uint32_t)runs.n0 * 2048;  // token rows of the second run
+                for (int kb = 0; kb < KS; ++kb) {
                     if (!mbar_wait_timed(&ctl->full[s], ph, g.wait_cycles, abort_flag, &w_full)) {
-                        if (lane == 0) report_error(g.status, KLEOS_AT_GEMM_MMA, t, (int)g.epoch);
+                        if (lane == 0) report_error(g.status, KLEOS_AT_GEMM_MMA, (int)i, (int)g.epoch);
                         *abort_flag = 1;
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t sa = slices + s * STAGE_BYTES;
-#pragma unroll
-                    for (int sub = 0; sub < SUB; ++sub) {
-                        if (sub > 0 && kb * SUB + sub >= KS) break;  // the last deep stage may be half full
-                        const uint64_t da = make_smem_desc(sa + sub * SLICE_BYTES);
-                        const uint64_t db = make_smem_desc(sa + sub * SLICE_BYTES + A_STAGE_BYTES);
+                    const uint32_t sa = slices + s * SLICE_BYTES;
+                    const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + W_BYTES);
+                    auto multiply = [&](uint32_t d, uint64_t db_run, uint32_t idesc) {
 #pragma unroll
                         for (int k = 0; k < kSteps; ++k) {
-                            const uint32_t more = (sub | k) != 0 ? 1u : (uint32_t)(kb != 0);
-                            if constexpr (kWide) umma_tf32_pair_if(elected, d_tmem, da + 2 * k, db + 2 * k, kInstrDesc, more);
-                            else umma_bf16_pair_if(elected, d_tmem, da + 2 * k, db + 2 * k, kInstrDesc, more);
+                            const uint32_t more = k != 0 ? 1u : (uint32_t)(kb != 0);
+                            if constexpr (kWide) umma_tf32_pair_if(elected, d, da + 2 * k, db_run + 2 * k, idesc, more);
+                            else umma_bf16_pair_if(elected, d, da + 2 * k, db_run + 2 * k, idesc, more);
                         }
-                    }
+                    };
+                    multiply(d0, db, idesc0);
+                    if (runs.n1 > 0) multiply(d1, make_smem_desc(sa + W_BYTES + off1), idesc1);
                     // the stage is free in both blocks once these MMAs have read it
                     umma_commit_both_if(elected, bars + (uint32_t)offsetof(Control, empty) + 8 * s);
-                    if (++s == NST) {
+                    if (++s == kSlices) {
                         s = 0;
                         ph ^= 1;
                     }
                 }
                 if (!ok) break;
-                umma_commit_both_if(elected, bars + (uint32_t)offsetof(Control, acc_full) + 8 * buf);
+                umma_commit_both_if(elected, bars + (uint32_t)offsetof(Control, acc_full) + 8 * (i % kSlots));
             }
             if (g.stats && lane == 0) {
                 g.stats[blockIdx.x * kStatSlots + 2] = w_acc;
@@ -293,130 +479,121 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
         }
         __syncwarp();
     } else if (warp >= 4) {
-        // ------------------------------------------------------------ epilogue (both blocks)
-        // Eight warps, two per quadrant of the accumulator rows, and a rolled loop over 64-column groups.
-        // With four warps and the tile's 256 erff per thread unrolled, layers with GELU waited for their
-        // read-back and for instructions: 6016 tokens, H = 1472, I = 3008, dense: 166 -> 91 us.
-        const int q = warp & 3, half = (warp - 4) >> 2, w8 = warp - 4;
+        // ------------------------------------------------------------ read-back (both blocks)
+        // Tensor-memory lane = output column, column = token row.  Group 0 takes the first 16 columns of
+        // every slot, group 1 the others; a warp reads the 32 lanes of its quadrant.
+        const int q = warp & 3, grp = (warp - 4) >> 2;
+        const int tg = tid - 128 - grp * 128;  // thread of the group
         const TE* bias = static_cast<const TE*>(g.bias);
-        uint32_t tile_n = 0;
-        long long w_accfull = 0, w_tmem = 0;
+        uint32_t at = 0, turn = 0;
+        long long w_accfull = 0;
         const long long t_begin = clock64();
-        for (int t = cluster_id; t < total; t += n_clusters, ++tile_n) {
-            PairTile pt;
-            if (!decode_pair_tile(t, ctl->le_start, g.le_begin, g.le_end, NT, &pt)) break;
-            const bool have_panel = (int)cta_rank < pt.n_panels_left;
-            const PanelEntry p = panel_at(pt.panel0 + (have_panel ? (int)cta_rank : 0));
-            const int rows = have_panel ? p.rows : 0;
-            const uint32_t buf = tile_n & 1, use = tile_n >> 1;
-            if (*abort_flag) break;
-            {
-                // stage the bias of this warp's 128 columns in shared memory (one load per lane)
-                // while the main loop of the tile is still running: global loads issued later would
-                // queue behind the operand traffic streaming into this SM
-                const int nb = pt.nt * BN + half * (BN / 2) + 4 * lane;
-                float* bs = &ctl->bias_s[w8][4 * lane];
-                if (nb < g.N) {
-                    const TE* src = bias + (size_t)pt.le * g.N + nb;
-                    if constexpr (kWide) {
-                        *reinterpret_cast<float4*>(bs) = __ldg(reinterpret_cast<const float4*>(src));
-                    } else {
-                        using TE2 = typename Pack2<TE>::type;
-                        const uint2 raw = __ldg(reinterpret_cast<const uint2*>(src));
-                        const TE2* h2 = reinterpret_cast<const TE2*>(&raw);
+        for (uint32_t i = 0;; ++i) {
+            // The warps of a group meet at barriers below, so all of them go on or none: whatever one of
+            // them gave up on, they find out here.
+            const Task x = take(i, KLEOS_AT_GEMM_EPILOGUE);
+            if (!all_of_group(x.half != 0, 1 + grp)) break;
+            const Runs runs(at, x.half);
+            const int n0 = x.mt * 2 * BM + (int)cta_rank * BM;  // this block's first output column
+            // bias of the columns this thread reads back, loaded while the main loop is still running
+            float bv[4];
 #pragma unroll
-                        for (int j = 0; j < 2; ++j) {
-                            const float2 f = Pack2<TE>::to_f2(h2[j]);
-                            bs[2 * j] = f.x;
-                            bs[2 * j + 1] = f.y;
-                        }
-                    }
-                }
-                __syncwarp();
+            for (int k = 0; k < 4; ++k) {
+                const int n = n0 + q * 32 + (kWide ? lane : 8 * k + (lane >> 2));
+                bv[k] = n < g.N && (k == 0 || !kWide) ? Elem<TE>::to_f(bias[(size_t)x.le * g.N + n]) : 0.f;
             }
-            if (!mbar_wait_timed(&ctl->acc_full[buf], use & 1, g.wait_cycles, abort_flag, &w_accfull)) {
-                if (lane == 0) report_error(g.status, KLEOS_AT_GEMM_EPILOGUE, t, (int)g.epoch);
+            TE* obase[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                obase[h] = out_ptr<TE>(g, PanelEntry{x.row_base[h], x.rows[h], x.le, (x.src >> (8 * h)) & 0xff}, 0, n0);
+            const bool ok = mbar_wait_timed(&ctl->acc_full[i % kSlots], (i / kSlots) & 1, g.wait_cycles, abort_flag, &w_accfull);
+            if (!ok) {
+                if (lane == 0) report_error(g.status, KLEOS_AT_GEMM_EPILOGUE, (int)i, (int)g.epoch);
                 *abort_flag = 1;
-                break;
             }
+            if (!all_of_group(ok, 1 + grp)) break;
             tc_fence_after();
-            const int n0 = pt.nt * BN + half * (BN / 2);
-            const uint32_t taddr = tmem_base + buf * BN + half * (BN / 2) + (static_cast<uint32_t>(q * 32) << 16);
-            // this warp's 32 accumulator rows; rows_w of them carry tokens
-            const int rows_w = min(32, rows - q * 32);
-            if (rows_w <= 0) {
+            const int n_slots = runs.n0 + runs.n1;
+            // A turn is 16 columns: 16 rows of one block's share.  Two turns' loads are in flight together.
+            auto fetch = [&](uint32_t slot, uint32_t* r) {
+                const uint32_t taddr = tmem_base + (slot % kSlots) * kSlotCols + grp * 16 + (static_cast<uint32_t>(q * 32) << 16);
+                if constexpr (kWide) {
+                    tmem_ld_32x16(taddr, r);
+                } else {
+                    tmem_ld_16x256_x2(taddr, r);
+                    tmem_ld_16x256_x2(taddr + (16u << 16), r + 8);
+                }
+            };
+            auto store = [&](int k, const uint32_t* r) {
+                const bool run1 = k >= runs.n0;
+                const int len = (run1 ? runs.n1 : runs.n0) * 16, off = run1 ? runs.n0 * 16 : 0;
+                const int c = (k - (run1 ? runs.n0 : 0)) * kSlotCols + grp * 16;
+                const int h = c >= len, r0 = off + c - (h ? len : 0);
+                const int valid = min(16, (h ? x.rows[1] : x.rows[0]) - r0);
+                if (valid <= 0) return;  // (the same for all warps of the group)
+                TE* o = (h ? obase[1] : obase[0]) + (size_t)r0 * g.N;
+                auto finish = [&](uint32_t bits, float b) {
+                    float v = __uint_as_float(bits) + b;
+                    if constexpr (kEpi == 0) v = fmaxf(v, 0.f);
+                    else if constexpr (kEpi == 1) v = apply_act(v, 1);
+                    return v;
+                };
+                if constexpr (kWide) {
+                    // 32 consecutive columns of a row: one 128-byte line per store instruction
+                    if (n0 + q * 32 < g.N) {
+                        float* of = reinterpret_cast<float*>(o) + q * 32 + lane;
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            if (j < valid) of[(size_t)j * g.N] = round_tf32(finish(r[j], bv[0]));
+                    }
+                } else {
+                    // transposed through shared memory: the group's four warps put the block's 128 columns of
+                    // 16 rows there, and every store instruction writes 256 bytes of two rows
+                    const uint32_t stg = smem_u32(ctl->stage[grp][turn & 1]);
+                    ++turn;
+#pragma unroll
+                    for (int x8 = 0; x8 < 2; ++x8) {
+                        uint32_t m[4];
+#pragma unroll
+                        for (int b = 0; b < 4; ++b) {  // columns 8 b .. 8 b + 7 of the warp's 32
+                            const uint32_t* f = r + (b >> 1) * 8 + x8 * 4 + (b & 1) * 2;
+                            const auto p = Pack2<TE>::from_f2(finish(f[0], bv[b]), finish(f[1], bv[b]));
+                            m[b] = *reinterpret_cast<const uint32_t*>(&p);
+                        }
+                        stmatrix_x4_trans(stg + (uint32_t)((8 * x8 + (lane & 7)) * STG_ROW + q * 64 + (lane >> 3) * 16), m);
+                    }
+                    asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
+                    const int col = (tg & 15) * 8;
+#pragma unroll
+                    for (int j = tg >> 4; j < 16; j += 8)
+                        if (j < valid && n0 + col < g.N) {
+                            uint4 v;
+                            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                                         : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                                         : "r"(stg + (uint32_t)(j * STG_ROW + col * 2)));
+                            *reinterpret_cast<uint4*>(o + (size_t)j * g.N + col) = v;
+                        }
+                }
+            };
+#pragma unroll 1
+            for (int k = 0; k < n_slots; k += 2, at += 2) {
+                uint32_t r0[16], r1[16];
+                const bool two = k + 1 < n_slots;
+                fetch(at, r0);
+                if (two) fetch(at + 1, r1);
+                tmem_ld_wait();
+                // this warp's part of the slots is in registers: hand it back to the MMA issuer
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_pair(map_to_cta(smem_u32(&ctl->acc_empty[buf]), 0));
-                continue;
+                if (lane < (two ? 2 : 1)) arrive_relaxed(map_to_cta(smem_u32(&ctl->slot_empty[(at + lane) % kSlots]), 0));
+                store(k, r0);
+                if (two) store(k + 1, r1);
             }
-            TE* obase = out_ptr<TE>(g, p, q * 32, n0);
-            uint4* stg = ctl->stage_s[w8];
-            // Every 128 bytes of the rows (64 or 32 columns) the warp transposes through a swizzled
-            // shared-memory tile, sixteen rows at a time, so that each store instruction writes four
-            // complete 128-byte lines (one row segment per 8 lanes) instead of 32 scattered 16-byte
-            // pieces: this is what the NVLink path to a peer's cell needs.
-#pragma unroll 1
-            for (int cc = 0; cc < BN / 2; cc += BKE) {
-                uint32_t r[BKE];
-                tmem_ld_32x32(taddr + cc, r);
-                if constexpr (!kWide) tmem_ld_32x32(taddr + cc + 32, r + 32);
-                const long long tq = clock64();
-                tmem_ld_wait();
-                w_tmem += clock64() - tq;
-                if (cc + BKE == BN / 2) {
-                    // this warp's part of the accumulator is in registers: hand it back to the MMA issuer
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_pair(map_to_cta(smem_u32(&ctl->acc_empty[buf]), 0));
-                }
-                if (n0 + cc >= g.N) continue;
-                const float4* bq = reinterpret_cast<const float4*>(&ctl->bias_s[w8][cc]);
-#pragma unroll
-                for (int j = 0; j < BKE / 2; ++j) {
-                    const float4 bf = bq[j >> 1];
-                    float v0 = __uint_as_float(r[2 * j]) + ((j & 1) ? bf.z : bf.x);
-                    float v1 = __uint_as_float(r[2 * j + 1]) + ((j & 1) ? bf.w : bf.y);
-                    if constexpr (kEpi == 0) {
-                        v0 = fmaxf(v0, 0.f);
-                        v1 = fmaxf(v1, 0.f);
-                    } else if constexpr (kEpi == 1) {
-                        v0 = apply_act(v0, 1);
-                        v1 = apply_act(v1, 1);
-                    }
-                    if constexpr (kWide) {
-                        r[2 * j] = __float_as_uint(round_tf32(v0));
-                        r[2 * j + 1] = __float_as_uint(round_tf32(v1));
-                    } else {
-                        const auto h = Pack2<TE>::from_f2(v0, v1);
-                        r[j] = *reinterpret_cast<const uint32_t*>(&h);
-                    }
-                }
-#pragma unroll
-                for (int p0 = 0; p0 < 32; p0 += 16) {
-                    if (p0 >= rows_w) break;
-                    if ((lane & 16) == p0) {
-#pragma unroll
-                        for (int ch = 0; ch < 8; ++ch)
-                            stg[(lane & 15) * 8 + (ch ^ (lane & 7))] =
-                                make_uint4(r[4 * ch], r[4 * ch + 1], r[4 * ch + 2], r[4 * ch + 3]);
-                    }
-                    __syncwarp();
-#pragma unroll
-                    for (int it = 0; it < 4; ++it) {
-                        const int rr = it * 4 + (lane >> 3), ch = lane & 7;
-                        const uint4 v = stg[rr * 8 + (ch ^ (rr & 7))];
-                        if (p0 + rr < rows_w)
-                            *reinterpret_cast<uint4*>(obase + (size_t)(p0 + rr) * g.N + cc + ch * (16 / (int)sizeof(TE))) = v;
-                    }
-                    __syncwarp();
-                }
-            }
+            at -= n_slots & 1;
         }
         if (g.stats && warp == 4 && lane == 0) {
             g.stats[blockIdx.x * kStatSlots + 5] = w_accfull;
             g.stats[blockIdx.x * kStatSlots + 6] = clock64() - t_begin;
-            g.stats[blockIdx.x * kStatSlots + 7] = w_tmem;
         }
     }
 
@@ -432,7 +609,9 @@ ffn_gemm_tc2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                      "r"(TMEM_COLS)
                      : "memory");
     }
-    if (g.mode == 1) publish_return_flags(g.ret, &last_block);
+    // the last pair to finish leaves the counters as it found them
+    if (leader && tid == 0 && atomicInc(g.next_tile + 1, (unsigned)n_clusters - 1) == (unsigned)n_clusters - 1) g.next_tile[0] = 0;
+    if (g.mode == 1) publish_return_flags(g.ret, &ctl->last_block);
 }
 
 }  // namespace kleos

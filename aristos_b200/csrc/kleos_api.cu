@@ -100,14 +100,16 @@ struct State {
     unsigned *counts = nullptr, *done_dispatch = nullptr, *done_gemm2 = nullptr,
              *cell_counts = nullptr;
     PanelEntry* panels = nullptr;
+    unsigned* tile_claims = nullptr;  // [2][2] claim counters of the two expert GEMMs, zero between launches
     DeviceStatus* status = nullptr;
     long long* gemm_stats = nullptr;  // [2][grid][8] when KLEOS_GEMM_STATS=1
 
     // tensor maps (rebuilt when the caller's weight pointer changes)
     const void* maps_for_iP = nullptr;
-    // map_w1 / map_w2: weight tiles of the float GEMM; map_w1h / map_w2h: the half tile each block of a
-    // pair loads (16-bit and TF32 GEMMs)
+    // map_w1 / map_w2: weight tiles of the float GEMM; map_w1h / map_w2h: the 128 weight rows each block of
+    // a pair loads (16-bit and TF32 GEMMs), rows_x / rows_y1: the token rows beside them
     CUtensorMap map_x{}, map_w1{}, map_y1{}, map_w2{}, map_act{}, map_wg{}, map_w1h{}, map_w2h{}, map_wgh{};
+    gemm_tc2::RowMaps rows_x{}, rows_y1{};
 
     // pipelined host-buffer path (kleos_forward_host_async): double-buffered staging of the
     // activations and of the layer output, one stream per direction
@@ -117,6 +119,7 @@ struct State {
         char* act[2] = {};
         char* res[2] = {};
         CUtensorMap map_act[2] = {};
+        gemm_tc2::RowMaps rows[2] = {};  // the dense layer's GEMM1 reads the staged activations
         cudaEvent_t in_done[2] = {}, comp_done[2] = {}, out_done[2] = {};
         unsigned long long step = 0;
     } hp;
@@ -277,6 +280,14 @@ int make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, u
     return KLEOS_OK;
 }
 
+// The boxes of token rows that ffn_gemm_tc2 loads
+int make_row_maps(gemm_tc2::RowMaps* m, const void* base, uint64_t rows, uint64_t cols) {
+    const uint32_t bk = 128 / (uint32_t)g.cfg.elem_bytes;
+    for (int i = 0; i < gemm_tc2::kBoxes; ++i)
+        if (const int rc = make_map(&m->box[i], base, rows, cols, (uint32_t)gemm_tc2::box_rows(i), bk)) return rc;
+    return KLEOS_OK;
+}
+
 struct Sections {
     const char *A, *Wg, *W1, *W2, *b1, *b2;
     char *probs, *out;
@@ -312,12 +323,12 @@ int ensure_maps(const Sections& s) {
         g.maps_for_iP = s.A;
         return KLEOS_OK;
     }
+    if ((rc = make_row_maps(&g.rows_x, g.dense ? s.A : g.arena + g.lay.xcell, cell_rows, c.H))) return rc;
+    if ((rc = make_row_maps(&g.rows_y1, g.y1, cell_rows, c.I))) return rc;
     if (g.use_tf32_tc) {
         const uint32_t bk = 32;  // 128 bytes
-        if ((rc = make_map(&g.map_x, g.dense ? s.A : g.arena + g.lay.xcell, cell_rows, c.H, gemm_tc2::BM, bk))) return rc;
-        if ((rc = make_map(&g.map_w1h, s.W1, (uint64_t)g.nLx * c.I, c.H, gemm_tc2::BN / 2, bk))) return rc;
-        if ((rc = make_map(&g.map_y1, g.y1, cell_rows, c.I, gemm_tc2::BM, bk))) return rc;
-        if ((rc = make_map(&g.map_w2h, s.W2, (uint64_t)g.nLx * c.H, c.I, gemm_tc2::BN / 2, bk))) return rc;
+        if ((rc = make_map(&g.map_w1h, s.W1, (uint64_t)g.nLx * c.I, c.H, gemm_tc2::BM, bk))) return rc;
+        if ((rc = make_map(&g.map_w2h, s.W2, (uint64_t)g.nLx * c.H, c.I, gemm_tc2::BM, bk))) return rc;
         if (c.PX <= 128 && !g.dense) {
             if ((rc = make_map(&g.map_act, s.A, c.S, c.H, route_tc::BM, bk))) return rc;
             if ((rc = make_map(&g.map_wg, s.Wg, c.PX, c.H, c.PX, bk))) return rc;
@@ -325,11 +336,11 @@ int ensure_maps(const Sections& s) {
         g.maps_for_iP = s.A;
         return KLEOS_OK;
     }
-    if ((rc = make_map(&g.map_x, g.dense ? s.A : g.arena + g.lay.xcell, cell_rows, c.H, gemm_tc2::BM))) return rc;
-    if ((rc = make_map(&g.map_y1, g.y1, cell_rows, c.I, gemm_tc2::BM))) return rc;
+    g.map_x = g.rows_x.box[4];  // 128 rows
+    g.map_y1 = g.rows_y1.box[4];
     const int promo = 3;  // 256-byte L2 promotion; 0/64/128 bytes measured the same on the C3 layer
-    if ((rc = make_map(&g.map_w1h, s.W1, (uint64_t)g.nLx * c.I, c.H, gemm_tc2::BN / 2, 64, true, promo))) return rc;
-    if ((rc = make_map(&g.map_w2h, s.W2, (uint64_t)g.nLx * c.H, c.I, gemm_tc2::BN / 2, 64, true, promo))) return rc;
+    if ((rc = make_map(&g.map_w1h, s.W1, (uint64_t)g.nLx * c.I, c.H, gemm_tc2::BM, 64, true, promo))) return rc;
+    if ((rc = make_map(&g.map_w2h, s.W2, (uint64_t)g.nLx * c.H, c.I, gemm_tc2::BM, 64, true, promo))) return rc;
     if (c.PX <= 128 && !g.dense) {
         if ((rc = make_map(&g.map_act, s.A, c.S, c.H, route_tc::BM))) return rc;
         if ((rc = make_map(&g.map_wg, s.Wg, c.PX, c.H, c.PX))) return rc;
@@ -379,15 +390,9 @@ int launch_route(const RouteArgs& ra, cudaStream_t st, bool prepare = false) {
     return fail(KLEOS_E_UNSUPPORTED, "more than 256 experts are not supported by the router");
 }
 
-// The paired GEMM comes in two pipeline shapes (see gemm_tc2.cuh): deep = three 128-wide stages,
-// otherwise six 64-wide stages.
 template <typename TE, int kEpi>
-void launch_tc2(bool deep, int grid, cudaStream_t st, const CUtensorMap& map_a, const CUtensorMap& map_b,
-                const GemmArgs& ga) {
-    if (deep)
-        launch(ffn_gemm_tc2<TE, kEpi, 2>, grid, gemm_tc2::kThreads, gemm_tc2::SMEM_BYTES, st, map_a, map_b, ga);
-    else
-        launch(ffn_gemm_tc2<TE, kEpi, 1>, grid, gemm_tc2::kThreads, gemm_tc2::SMEM_BYTES, st, map_a, map_b, ga);
+void launch_tc2(cudaStream_t st, const gemm_tc2::RowMaps& map_x, const CUtensorMap& map_w, const GemmArgs& ga) {
+    launch(ffn_gemm_tc2<TE, kEpi>, g.sm_count & ~1, gemm_tc2::kThreads, gemm_tc2::SMEM_BYTES, st, map_x, map_w, ga);
 }
 
 // The persistent kernel, instantiated per activation and per compile-time top-k of the combine.
@@ -424,6 +429,7 @@ struct Staging {
     const char* A;
     char* out;
     const CUtensorMap* map_act;
+    const gemm_tc2::RowMaps* rows;  // dense 16-bit and TF32 layers
 };
 
 // num_experts == 1: out = (act(A W1^T + b1)) W2^T + b2 over this rank's S tokens, both GEMMs by
@@ -432,7 +438,7 @@ struct Staging {
 // (moe/fffn.cuh:31-167): intermediate rounded to the element type, identity epilogue on the
 // second GEMM, no gate, no scaling.
 template <typename T>
-int forward_dense(const Sections& s, const CUtensorMap* map_a, cudaStream_t st, bool timed) {
+int forward_dense(const Sections& s, const Staging* stg, cudaStream_t st, bool timed) {
     const LayerConfig& c = g.cfg;
     int evi = 0;
     auto mark = [&]() -> cudaError_t { return timed ? cudaEventRecord(g.ev[evi++], st) : cudaSuccess; };
@@ -442,25 +448,26 @@ int forward_dense(const Sections& s, const CUtensorMap* map_a, cudaStream_t st, 
     ga.status = g.status; ga.wait_cycles = g.wait_cycles; ga.stats = nullptr;
     ga.nLx = 1; ga.pEC = c.S; ga.rank = g.rank; ga.elem_bytes = c.elem_bytes; ga.epoch = g.epoch;
     ga.le_begin = 0; ga.le_end = 1; ga.mode = 0;
+    ga.contiguous = 1; ga.next_tile = g.tile_claims;
     GemmArgs g1 = ga;
     g1.A = s.A; g1.B = s.W1; g1.bias = s.b1; g1.y1 = g.y1; g1.N = c.I; g1.Kd = c.H;
     g1.hidden_act = c.hidden_act;
     GemmArgs g2 = ga;
+    g2.next_tile = g.tile_claims + 2; g2.plan_ready = 1;
     g2.A = g.y1; g2.B = s.W2; g2.bias = s.b2; g2.y1 = s.out; g2.N = c.H; g2.Kd = c.I;
     g2.hidden_act = 2;  // identity
     if (g.use_tc || g.use_tf32_tc) {
         if constexpr (!std::is_same<T, float>::value) {
-            const int grid = g.sm_count & ~1;
-            const bool deep = c.S >= 512;
+            const gemm_tc2::RowMaps& rows = stg ? *stg->rows : g.rows_x;
             if (c.hidden_act == 0)
-                launch_tc2<T, 0>(deep, grid, st, *map_a, g.map_w1h, g1);
+                launch_tc2<T, 0>(st, rows, g.map_w1h, g1);
             else
-                launch_tc2<T, 1>(deep, grid, st, *map_a, g.map_w1h, g1);
+                launch_tc2<T, 1>(st, rows, g.map_w1h, g1);
             KLEOS_CUDA(mark());
-            launch_tc2<T, 2>(deep, grid, st, g.map_y1, g.map_w2h, g2);
+            launch_tc2<T, 2>(st, g.rows_y1, g.map_w2h, g2);
         }
     } else if (g.use_f32_tc) {
-        launch_f32(g.f32_bn[0], st, *map_a, g.map_w1, g1);
+        launch_f32(g.f32_bn[0], st, stg ? *stg->map_act : g.map_x, g.map_w1, g1);
         KLEOS_CUDA(mark());
         launch_f32(g.f32_bn[1], st, g.map_y1, g.map_w2, g2);
     } else {
@@ -487,7 +494,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
         act_map = stg->map_act;
     }
     g.epoch += 1;
-    if (g.dense) return forward_dense<T>(s, stg ? stg->map_act : &g.map_x, st, timed);
+    if (g.dense) return forward_dense<T>(s, stg, st, timed);
     int evi = 0;
     auto mark = [&]() -> cudaError_t { return timed ? cudaEventRecord(g.ev[evi++], st) : cudaSuccess; };
     KLEOS_CUDA(mark());
@@ -617,9 +624,11 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     ga.ret.peers = g.peers; ga.ret.lay = g.lay; ga.ret.done_counter = g.done_gemm2;
     ga.ret.rank = g.rank; ga.ret.world = g.world; ga.ret.epoch = g.epoch;
     ga.ret.suppress = g.suppress_return_flag ? 1 : 0;
+    ga.contiguous = g.world == 1; ga.next_tile = g.tile_claims; ga.counts = g.counts; ga.EC = c.EC;
     GemmArgs g1 = ga;
     g1.A = g.arena + g.lay.xcell; g1.B = s.W1; g1.bias = s.b1; g1.N = c.I; g1.Kd = c.H; g1.mode = 0;
     GemmArgs g2 = ga;
+    g2.next_tile = g.tile_claims + 2; g2.plan_ready = 1;
     g2.A = g.y1; g2.B = s.W2; g2.bias = s.b2; g2.N = c.H; g2.Kd = c.I; g2.mode = 1;
     if (g.gemm_stats) {
         g1.stats = g.gemm_stats;
@@ -627,14 +636,12 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     }
     if (g.use_tc || g.use_tf32_tc) {
         if constexpr (!std::is_same<T, float>::value) {
-            const int grid = g.sm_count & ~1;
-            const bool deep = (long long)g.world * c.EC >= 512;
             if (c.hidden_act == 0)
-                launch_tc2<T, 0>(deep, grid, st, g.map_x, g.map_w1h, g1);
+                launch_tc2<T, 0>(st, g.rows_x, g.map_w1h, g1);
             else
-                launch_tc2<T, 1>(deep, grid, st, g.map_x, g.map_w1h, g1);
+                launch_tc2<T, 1>(st, g.rows_x, g.map_w1h, g1);
             KLEOS_CUDA(mark());
-            launch_tc2<T, 2>(deep, grid, st, g.map_y1, g.map_w2h, g2);
+            launch_tc2<T, 2>(st, g.rows_y1, g.map_w2h, g2);
             KLEOS_CUDA(mark());
         }
     } else if (g.use_f32_tc) {
@@ -691,12 +698,9 @@ int sync_last_forward() {
 template <typename TE>
 int set_gemm_attributes() {
     const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 0, 1>, dyn, gemm_tc2::SMEM_BYTES));
-    KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 0, 2>, dyn, gemm_tc2::SMEM_BYTES));
-    KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 1, 1>, dyn, gemm_tc2::SMEM_BYTES));
-    KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 1, 2>, dyn, gemm_tc2::SMEM_BYTES));
-    KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 2, 1>, dyn, gemm_tc2::SMEM_BYTES));
-    KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 2, 2>, dyn, gemm_tc2::SMEM_BYTES));
+    KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 0>, dyn, gemm_tc2::SMEM_BYTES));
+    KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 1>, dyn, gemm_tc2::SMEM_BYTES));
+    KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 2>, dyn, gemm_tc2::SMEM_BYTES));
     return KLEOS_OK;
 }
 
@@ -747,7 +751,11 @@ int ensure_host_pipe() {
             if (rc) return rc;
         } else if ((g.use_tf32_tc && (g.dense || c.PX <= 128)) || (g.use_f32_tc && g.dense)) {
             // same box (128 rows x 32 words) serves the tf32 router and the dense layers' GEMM1
-            int rc = make_map(&hp.map_act[b], hp.act[b], c.S, c.H, gemm_tc2::BM, 32);
+            int rc = make_map(&hp.map_act[b], hp.act[b], c.S, c.H, gemm_f32::BM, 32);
+            if (rc) return rc;
+        }
+        if (g.dense && (g.use_tc || g.use_tf32_tc)) {
+            int rc = make_row_maps(&hp.rows[b], hp.act[b], c.S, c.H);
             if (rc) return rc;
         }
     }
@@ -762,7 +770,7 @@ void release_all() {
     cudaFree(g.y1); cudaFree(g.topk); cudaFree(g.slots); cudaFree(g.cell_tokens);
     cudaFree(g.refine_list); cudaFree(g.refine_count); cudaFree(g.tile_hist); cudaFree(g.refine_done); cudaFree(g.refine_logits); cudaFree(g.le_start); cudaFree(g.mcw);
     cudaFree(g.bias); cudaFree(g.counts); cudaFree(g.done_dispatch); cudaFree(g.done_gemm2);
-    cudaFree(g.cell_counts); cudaFree(g.flow_ctr); cudaFree(g.flow_stamps); cudaFree(g.flow_stalls); cudaFree(g.panels); cudaFree(g.status); cudaFree(g.gemm_stats);
+    cudaFree(g.cell_counts); cudaFree(g.flow_ctr); cudaFree(g.flow_stamps); cudaFree(g.flow_stalls); cudaFree(g.panels); cudaFree(g.tile_claims); cudaFree(g.status); cudaFree(g.gemm_stats);
     cudaFree(g.col_partial); cudaFree(g.gate_stats);
     for (auto& e : g.ev)
         if (e) cudaEventDestroy(e);
@@ -931,6 +939,7 @@ static int initialize_impl(const char* config_json_path, int rank, int world, co
     if ((rc = dev_alloc(&g.done_gemm2, 1))) return rc;
     if ((rc = dev_alloc(&g.cell_counts, (size_t)cfg.E))) return rc;
     if ((rc = dev_alloc(&g.panels, (size_t)cfg.E * cfg.pEC / kTileM))) return rc;
+    if ((rc = dev_alloc(&g.tile_claims, 4))) return rc;
     if ((rc = dev_alloc(&g.status, 1))) return rc;
     if (cfg.is_training && !dense) {
         if ((rc = dev_alloc(&g.col_partial, (size_t)((cfg.S + route_fma::TM - 1) / route_fma::TM) * cfg.PX))) return rc;
@@ -1176,7 +1185,7 @@ int kleos_forward_host_async(const void* host_activations, void* iP, void* oP, v
     KLEOS_CUDA(cudaEventRecord(hp.in_done[b], hp.in));
     KLEOS_CUDA(cudaStreamWaitEvent(st, hp.in_done[b], 0));
     if (reuse) KLEOS_CUDA(cudaStreamWaitEvent(st, hp.out_done[b], 0));
-    const Staging stg{hp.act[b], hp.res[b], &hp.map_act[b]};
+    const Staging stg{hp.act[b], hp.res[b], &hp.map_act[b], &hp.rows[b]};
     if ((rc = forward_any(iP, oP, st, false, &stg))) return rc;
     KLEOS_CUDA(cudaEventRecord(hp.comp_done[b], st));
     KLEOS_CUDA(cudaStreamWaitEvent(hp.out, hp.comp_done[b], 0));

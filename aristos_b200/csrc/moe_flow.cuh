@@ -41,20 +41,18 @@
 
 #include <cuda.h>
 
-#include "gemm_tc2.cuh"
+#include "gemm_common.cuh"
+#include "tc_common.cuh"
 
 namespace kleos {
 namespace flow {
 
-using gemm_tc2::A_STAGE_BYTES;
-using gemm_tc2::BK;
-using gemm_tc2::BM;
-using gemm_tc2::BN;
-using gemm_tc2::kSlices;
-using gemm_tc2::SLICE_BYTES;
-using gemm_tc2::TMEM_COLS;
-using gemm_tc2::UMMA_K;
-
+constexpr int BM = 128, BN = 256, BK = 64, UMMA_K = 16;  // rows per block, columns per pair, K slice
+constexpr int kSlices = 6;                        // 64-wide K slices of shared memory in total
+constexpr int A_STAGE_BYTES = BM * BK * 2;        // 16 KiB: one K slice of this block's panel
+constexpr int B_STAGE_BYTES = (BN / 2) * BK * 2;  // 16 KiB: one K slice of this block's half weight tile
+constexpr int SLICE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
+constexpr int TMEM_COLS = 512;                    // two accumulators of 256 fp32 columns
 constexpr int kThreads = 384;      // 12 warps
 constexpr int kRing = 8;           // claimed-tile ring per block (see hand_out())
 constexpr int kMaxPanels = 384;    // 128-row panels one rank can plan
@@ -440,7 +438,7 @@ __device__ __forceinline__ double warp_dot64(const T* x, const T* w, int H, int 
 
 // kAct: the expert's activation (0 ReLU, 1 GELU); KT: compile-time top-k of the combine (0 = read
 // it from the arguments).  Args::sub = 64-wide K slices per pipeline stage (1: six shallow stages,
-// 2: three deep ones, see gemm_tc2.cuh).
+// 2: three deep ones).
 template <typename TE, int kAct, int KT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(flow::kThreads, 1)
 moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w1,

@@ -28,7 +28,7 @@
 #include "moe_flow.cuh"
 #include "placement.hpp"
 #include "route.cuh"
-#include "route_tc.cuh"
+#include "route_split.cuh"
 #include "transport.cuh"
 
 namespace kleos {
@@ -70,7 +70,10 @@ struct State {
     // only move inside this GPU's memory, with no flags to raise or to wait for (KLEOS_DISPATCH_KERNELS=1:
     // the dispatch and plan kernels of several ranks instead)
     bool local = false;
-    bool route_by_flow = false;              // separate launches: the router is the persistent kernel's routing phase alone
+    bool split_route = false;                // the router is route_split_kernel (KLEOS_ROUTE_KERNELS=1: the kernels of route.cuh)
+    int route_parts = 1;                     // ... blocks per 128 tokens: parts of K whose logits are summed apart
+    int route_grid = 0;                      // ... its blocks, no more than the device holds at once
+    unsigned long long* place_hist = nullptr;  // see PlaceArgs
     int flow_grid = 0;                       // blocks of the persistent kernel (co-resident pairs x 2)
     flow::Counters* flow_ctr = nullptr;      // [2] scheduler state, see moe_flow.cuh
     long long* flow_stamps = nullptr;        // [flow_grid][kStampSlots] timeline of a timed forward
@@ -249,35 +252,35 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn g_encode = nullptr;
 
-// Matrix [rows][cols] of the layer's element type with cols contiguous; box = box_cols columns x
-// box_rows rows, 128-byte swizzle (64 16-bit or 32 4-byte elements = 128 bytes, the swizzle span).
-int make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,
-             uint32_t box_cols = 64, bool swizzle = true, int promo = 3) {
+// Matrix [rows][cols] with cols contiguous; box = box_cols columns x box_rows rows, 128-byte swizzle
+// (64 16-bit or 32 4-byte elements = 128 bytes, the swizzle span).
+const char* encode_map(CUtensorMap* map, CUtensorMapDataType type, int elem_bytes, const void* base, uint64_t rows, uint64_t cols,
+                       uint32_t box_rows, uint32_t box_cols) {
     if (!g_encode) {
         void* fn = nullptr;
         cudaDriverEntryPointQueryResult q;
-        KLEOS_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q));
-        if (!fn || q != cudaDriverEntryPointSuccess)
-            return fail(KLEOS_E_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess || !fn ||
+            q != cudaDriverEntryPointSuccess)
+            return "cuTensorMapEncodeTiled is not available from the driver";
         g_encode = reinterpret_cast<EncodeTiledFn>(fn);
     }
     const cuuint64_t dims[2] = {cols, rows};
-    const cuuint64_t strides[1] = {cols * (cuuint64_t)g.cfg.elem_bytes};
+    const cuuint64_t strides[1] = {cols * (cuuint64_t)elem_bytes};
     const cuuint32_t box[2] = {box_cols, box_rows};
     const cuuint32_t estr[2] = {1, 1};
+    // (256-byte L2 promotion; 0/64/128 bytes measured the same)
+    const CUresult r = g_encode(map, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? nullptr : "cuTensorMapEncodeTiled failed";
+}
+
+// ... of the layer's element type
+int make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_cols = 64) {
     const CUtensorMapDataType dt = g.cfg.torch_dtype == 3   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                    : g.cfg.torch_dtype == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                                                             : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-    const CUresult r = g_encode(map, dt, 2, const_cast<void*>(base),
-                                dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                                promo == 0 ? CU_TENSOR_MAP_L2_PROMOTION_NONE
-                                : promo == 1 ? CU_TENSOR_MAP_L2_PROMOTION_L2_64B
-                                : promo == 2 ? CU_TENSOR_MAP_L2_PROMOTION_L2_128B
-                                             : CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(KLEOS_E_CUDA, "cuTensorMapEncodeTiled failed: %d", (int)r);
-    return KLEOS_OK;
+    const char* err = encode_map(map, dt, g.cfg.elem_bytes, base, rows, cols, box_rows, box_cols);
+    return err ? fail(KLEOS_E_CUDA, "%s", err) : KLEOS_OK;
 }
 
 // The boxes of token rows that ffn_gemm_tc2 loads
@@ -330,7 +333,7 @@ int ensure_maps(const Sections& s) {
         if ((rc = make_map(&g.map_w1h, s.W1, (uint64_t)g.nLx * c.I, c.H, gemm_tc2::BM, bk))) return rc;
         if ((rc = make_map(&g.map_w2h, s.W2, (uint64_t)g.nLx * c.H, c.I, gemm_tc2::BM, bk))) return rc;
         if (c.PX <= 128 && !g.dense) {
-            if ((rc = make_map(&g.map_act, s.A, c.S, c.H, route_tc::BM, bk))) return rc;
+            if ((rc = make_map(&g.map_act, s.A, c.S, c.H, route_split::BM, bk))) return rc;
             if ((rc = make_map(&g.map_wg, s.Wg, c.PX, c.H, c.PX, bk))) return rc;
         }
         g.maps_for_iP = s.A;
@@ -338,11 +341,10 @@ int ensure_maps(const Sections& s) {
     }
     g.map_x = g.rows_x.box[4];  // 128 rows
     g.map_y1 = g.rows_y1.box[4];
-    const int promo = 3;  // 256-byte L2 promotion; 0/64/128 bytes measured the same on the C3 layer
-    if ((rc = make_map(&g.map_w1h, s.W1, (uint64_t)g.nLx * c.I, c.H, gemm_tc2::BM, 64, true, promo))) return rc;
-    if ((rc = make_map(&g.map_w2h, s.W2, (uint64_t)g.nLx * c.H, c.I, gemm_tc2::BM, 64, true, promo))) return rc;
+    if ((rc = make_map(&g.map_w1h, s.W1, (uint64_t)g.nLx * c.I, c.H, gemm_tc2::BM))) return rc;
+    if ((rc = make_map(&g.map_w2h, s.W2, (uint64_t)g.nLx * c.H, c.I, gemm_tc2::BM))) return rc;
     if (c.PX <= 128 && !g.dense) {
-        if ((rc = make_map(&g.map_act, s.A, c.S, c.H, route_tc::BM))) return rc;
+        if ((rc = make_map(&g.map_act, s.A, c.S, c.H, route_split::BM))) return rc;
         if ((rc = make_map(&g.map_wg, s.Wg, c.PX, c.H, c.PX))) return rc;
         // the half of the gate weight each block of a pair loads when the router runs inside the
         // persistent kernel
@@ -355,19 +357,71 @@ int ensure_maps(const Sections& s) {
 // One kernel of a forward, launched so that its blocks may arrive while the kernel before it drains
 // (see pdl_wait()).
 template <typename... P, typename... A>
-void launch(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
+void launch_clusters(int cluster, void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
     cudaLaunchConfig_t lc{};
     lc.gridDim = dim3((unsigned)grid);
     lc.blockDim = dim3((unsigned)threads);
     lc.dynamicSmemBytes = smem;
     lc.stream = st;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    lc.attrs = &at;
-    lc.numAttrs = 1;
+    cudaLaunchAttribute at[2] = {};
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = (unsigned)cluster;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    lc.attrs = at;
+    lc.numAttrs = cluster > 0 ? 2 : 1;
     ++g.launches;
     cudaLaunchKernelEx(&lc, kernel, args...);  // failures: cudaGetLastError() at the end of the forward
+}
+template <typename... P, typename... A>
+void launch(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
+    launch_clusters(0, kernel, grid, threads, smem, st, args...);  // clusters only where the kernel declares them
+}
+
+// Calls f with the instance of route_split_kernel for this layer and its shared memory.
+template <typename T, typename F>
+int with_route_split(F f) {
+    const bool top2 = g.cfg.K == 2;
+    if (g.cfg.PX == 64) return top2 ? f(route_split_kernel<T, 64, 2>, route_split::Shape<64>::SMEM_BYTES) : f(route_split_kernel<T, 64, 0>, route_split::Shape<64>::SMEM_BYTES);
+    return top2 ? f(route_split_kernel<T, 128, 2>, route_split::Shape<128>::SMEM_BYTES) : f(route_split_kernel<T, 128, 0>, route_split::Shape<128>::SMEM_BYTES);
+}
+
+// Expert weights that the router brings into L2 (126 MB, which also holds the layer's rows).
+constexpr size_t kAheadBytes = (size_t)64 << 20;
+
+// How the router's work is spread: as many blocks per 128 tokens (1, 2 or 4 in a cluster) as find room
+// on the chip beside those of the other tokens, none without a slice of K, and no more than the
+// persistent kernel's routing phase has accumulator columns for.
+template <typename T>
+int prepare_route_split() {
+    const LayerConfig& c = g.cfg;
+    const int tiles = c.S / route_split::BM, slices = c.H * c.elem_bytes / 128;
+    for (int parts = route_split::kMaxParts;; parts >>= 1) {
+        if (parts > 1 && (parts * c.PX > 256 || parts > slices || tiles * parts > g.sm_count)) continue;
+        int clusters = 0;
+        const int rc = with_route_split<T>([&](auto kernel, int smem) -> int {
+            KLEOS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            cudaLaunchConfig_t lc{};
+            lc.gridDim = dim3((unsigned)(tiles * parts));
+            lc.blockDim = dim3(route_split::kThreads);
+            lc.dynamicSmemBytes = (size_t)smem;
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = (unsigned)parts;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            lc.attrs = &at;
+            lc.numAttrs = 1;
+            KLEOS_CUDA(cudaOccupancyMaxActiveClusters(&clusters, kernel, &lc));
+            return KLEOS_OK;
+        });
+        if (rc) return rc;
+        if (parts > 1 && clusters < tiles) continue;
+        if (clusters < 1) return fail(KLEOS_E_CUDA, "the router does not fit the device");
+        g.route_parts = parts;
+        g.route_grid = clusters * parts;  // (those beyond the tokens only bring weights into L2)
+        return KLEOS_OK;
+    }
 }
 
 // Router on the FP32 pipes, for the layer's padded expert count.  `prepare` only sets the kernel up.
@@ -503,27 +557,10 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     if (routed_in_kernel) {
         KLEOS_CUDA(mark());
         KLEOS_CUDA(mark());
-    } else if (g.route_by_flow) {
-        if constexpr (sizeof(T) == 2) {
-            // router of the separate launches: the routing phase of moe_flow_kernel on its own (gate
-            // GEMM, top-k, in-place near-tie re-evaluation, grid barrier, slots, counts)
-            flow::Args fr{};
-            fr.tokens = s.A; fr.probs = s.probs; fr.topk = g.topk; fr.slots = g.slots; fr.mcw = g.mcw;
-            fr.cell_tokens = g.cell_tokens; fr.counts = g.counts; fr.peers = g.peers; fr.lay = g.lay;
-            fr.ctr = g.flow_ctr; fr.status = g.status; fr.wait_cycles = g.wait_cycles;
-            fr.S = c.S; fr.H = c.H; fr.I = c.I; fr.E = c.E; fr.K = c.K; fr.PX = c.PX; fr.EC = c.EC;
-            fr.pEC = c.pEC; fr.nLx = g.nLx; fr.rank = g.rank; fr.world = g.world; fr.epoch = g.epoch;
-            fr.sub = 1; fr.unit_rows = flow::kUnitRows; fr.fuse_route = 1; fr.route_only = 1;
-            fr.Wg = s.Wg; fr.gate_bias = g.bias; fr.tile_hist = g.tile_hist; fr.tie_eps = 1e-4f;
-            if (g.local) { fr.panels = g.panels; fr.le_start = g.le_start; }
-            launch_flow<T>(c.hidden_act, c.K, st, fr, act_map);
-        }
-        KLEOS_CUDA(mark());
-        KLEOS_CUDA(mark());
-        routed_in_kernel = true;  // nothing left to launch for routing and slots
     }
+    const bool split = g.split_route && !routed_in_kernel;
     // 1. router
-    if (!routed_in_kernel) KLEOS_CUDA(cudaMemsetAsync(g.refine_count, 0, sizeof(int), st));
+    if (!routed_in_kernel && !split) KLEOS_CUDA(cudaMemsetAsync(g.refine_count, 0, sizeof(int), st));
     RouteArgs ra{};
     ra.A = s.A; ra.Wg = s.Wg; ra.bias = g.bias; ra.probs = s.probs; ra.topk = g.topk;
     ra.mcw = g.mcw; ra.refine_list = g.refine_list; ra.refine_count = g.refine_count;
@@ -531,39 +568,48 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     ra.S = c.S; ra.H = c.H; ra.E = c.E; ra.K = c.K; ra.PX = c.PX; ra.tie_eps = 1e-4f;
     ra.col_partial = g.col_partial;  // null unless is_training
     int route_blocks = (c.S + route_fma::TM - 1) / route_fma::TM;
-    if (routed_in_kernel) {
-        // nothing to launch here
-    } else if ((g.use_tc || g.use_tf32_tc) && c.PX <= 128) {
-        route_blocks = (c.S + route_tc::BM - 1) / route_tc::BM;
+    PlaceArgs pl{};
+    pl.topk = g.topk; pl.A = s.A; pl.slots = g.slots; pl.cell_tokens = g.cell_tokens; pl.counts = g.counts;
+    pl.hist = g.place_hist; pl.peers = g.peers; pl.cflag = g.lay.cflag; pl.row_chunks = (unsigned)((size_t)c.H * c.elem_bytes / 16);
+    pl.status = g.status; pl.wait_cycles = g.wait_cycles; pl.S = c.S; pl.K = c.K; pl.E = c.E; pl.PX = c.PX; pl.EC = c.EC;
+    pl.pEC = c.pEC; pl.nLx = g.nLx; pl.rank = g.rank; pl.world = g.world; pl.epoch = g.epoch;
+    if (g.local) {
+        pl.xcell = g.arena + g.lay.xcell;
+        if (!g.use_tc && !g.use_tf32_tc) { pl.panels = g.panels; pl.le_start = g.le_start; }
+    }
+    if (split) {
+        // gate GEMM, top-k, near-ties, slots, counts and the panel list in one launch
         if constexpr (!std::is_same<T, float>::value) {
-            const int grid = (c.S + route_tc::BM - 1) / route_tc::BM;
-            if (c.PX == 64)
-                launch(route_tc_kernel<T, 64>, grid, 256, route_tc::Shape<64>::SMEM_BYTES, st, *act_map, g.map_wg, ra, g.status, g.wait_cycles, (int)g.epoch);
-            else
-                launch(route_tc_kernel<T, 128>, grid, 256, route_tc::Shape<128>::SMEM_BYTES, st, *act_map, g.map_wg, ra, g.status, g.wait_cycles, (int)g.epoch);
-            launch(refine_kernel<T>, 148, 256, 0, st, ra);
+            route_split::Args sp{};
+            sp.r = ra; sp.place = pl; sp.status = g.status; sp.parts = g.route_parts;
+            // (an expert is likely to get a token at all)
+            if ((long long)c.S * c.K * g.world >= 2LL * c.E) {
+                sp.ahead = s.W1;
+                sp.ahead_bytes = std::min<size_t>(kAheadBytes, (size_t)(s.b1 - s.W1)) & ~(size_t)15;
+            }
+            with_route_split<T>([&](auto kernel, int smem) -> int {
+                launch_clusters(g.route_parts, kernel, g.route_grid, route_split::kThreads, smem, st, *act_map, g.map_wg, sp);
+                return KLEOS_OK;
+            });
+            route_blocks = c.S / route_split::BM * g.route_parts;
         }
+    } else if (routed_in_kernel) {
+        // nothing to launch here
     } else if ((rc = launch_route<T>(ra, st))) {
         return rc;
     }
     if (!routed_in_kernel) KLEOS_CUDA(mark());
 
-    // 2. slots
-    SlotArgs sa{};
-    sa.topk = g.topk; sa.slots = g.slots; sa.cell_tokens = g.cell_tokens; sa.counts = g.counts;
-    sa.S = c.S; sa.K = c.K; sa.E = c.E; sa.EC = c.EC; sa.pEC = c.pEC;
-    for (int r = 0; r < kMaxWorld; ++r) sa.peer_arena[r] = g.peers.arena[r];
-    sa.cflag_offset = g.lay.cflag; sa.rank = g.rank; sa.nLx = g.nLx; sa.epoch = g.epoch;
-    sa.tile_hist = g.tile_hist;
-    if (g.local) { sa.panels = g.panels; sa.le_start = g.le_start; }
+    // 2. slots, counts, and on one rank the rows
     if (!routed_in_kernel) {
-        launch(tile_hist_kernel, (c.S + kSlotTile - 1) / kSlotTile, 256, 0, st, sa);
-        launch(slot_kernel, (c.S + kSlotTile - 1) / kSlotTile, 256, 0, st, sa);
-        if (g.col_partial)
-            launch(gate_stats_kernel, 1, 256, 0, st, g.col_partial, route_blocks, c.PX, g.counts, c.S, c.E, g.gate_stats);
+        if (!split) launch(place_kernel, (c.S + kPlaceOwn - 1) / kPlaceOwn, kPlaceThreads, 0, st, pl);
         KLEOS_CUDA(mark());
     }
 
+    if (!routed_in_kernel) {
+        if (g.col_partial)
+            launch(gate_stats_kernel, 1, 256, 0, st, g.col_partial, route_blocks, c.PX, g.counts, c.S, c.E, g.gate_stats);
+    }
     if (g.use_flow) {
         if constexpr (sizeof(T) == 2) {
             // 3.-7. one persistent kernel: dispatch, plan, GEMM1, GEMM2, combine
@@ -583,6 +629,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
             fa.unit_rows = g.flow_unit_rows;
             fa.fuse_route = routed_in_kernel ? 1 : 0;
             fa.Wg = s.Wg; fa.gate_bias = g.bias; fa.tile_hist = g.tile_hist; fa.tie_eps = 1e-4f;
+            fa.parts = g.route_parts;
             if (timed) {
                 KLEOS_CUDA(cudaMemsetAsync(g.flow_stamps, 0,
                                            sizeof(long long) * g.flow_grid * flow::kStampSlots, st));
@@ -603,8 +650,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     da.lay = g.lay; da.done_counter = g.done_dispatch; da.H = c.H; da.E = c.E; da.EC = c.EC;
     da.pEC = c.pEC; da.nLx = g.nLx; da.rank = g.rank; da.world = g.world; da.epoch = g.epoch;
     da.elem_bytes = c.elem_bytes; da.le_begin = 0; da.le_end = g.nLx;
-    if (g.local) launch(dispatch_local_kernel, (c.S + kDispatchTokens - 1) / kDispatchTokens, kDispatchTokens * 32, 0, st, LocalDispatchArgs{s.A, g.topk, g.slots, g.arena + g.lay.xcell, c.S, c.K, c.pEC, (unsigned)((size_t)c.H * c.elem_bytes / 16)});
-    else launch(dispatch_kernel, g.sm_count * 4, 256, 0, st, da);
+    if (!g.local) launch(dispatch_kernel, g.sm_count * 4, 256, 0, st, da);
     KLEOS_CUDA(mark());
     // 4. plan: wait for every source's rows, list the panels
     PlanArgs pa{};
@@ -707,8 +753,6 @@ int set_gemm_attributes() {
 template <typename TE>
 int set_tc_attributes() {
     const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    KLEOS_CUDA(cudaFuncSetAttribute(route_tc_kernel<TE, 64>, dyn, route_tc::Shape<64>::SMEM_BYTES));
-    KLEOS_CUDA(cudaFuncSetAttribute(route_tc_kernel<TE, 128>, dyn, route_tc::Shape<128>::SMEM_BYTES));
     if (const int rc = set_gemm_attributes<TE>()) return rc;
     KLEOS_CUDA(cudaFuncSetAttribute(moe_flow_kernel<TE, 0, 2>, dyn, flow::SMEM_BYTES));
     KLEOS_CUDA(cudaFuncSetAttribute(moe_flow_kernel<TE, 0, 0>, dyn, flow::SMEM_BYTES));
@@ -747,7 +791,7 @@ int ensure_host_pipe() {
         KLEOS_CUDA(cudaEventCreateWithFlags(&hp.comp_done[b], cudaEventDisableTiming));
         KLEOS_CUDA(cudaEventCreateWithFlags(&hp.out_done[b], cudaEventDisableTiming));
         if (g.use_tc && c.PX <= 128) {
-            int rc = make_map(&hp.map_act[b], hp.act[b], c.S, c.H, route_tc::BM);
+            int rc = make_map(&hp.map_act[b], hp.act[b], c.S, c.H, route_split::BM);
             if (rc) return rc;
         } else if ((g.use_tf32_tc && (g.dense || c.PX <= 128)) || (g.use_f32_tc && g.dense)) {
             // same box (128 rows x 32 words) serves the tf32 router and the dense layers' GEMM1
@@ -770,7 +814,7 @@ void release_all() {
     cudaFree(g.y1); cudaFree(g.topk); cudaFree(g.slots); cudaFree(g.cell_tokens);
     cudaFree(g.refine_list); cudaFree(g.refine_count); cudaFree(g.tile_hist); cudaFree(g.refine_done); cudaFree(g.refine_logits); cudaFree(g.le_start); cudaFree(g.mcw);
     cudaFree(g.bias); cudaFree(g.counts); cudaFree(g.done_dispatch); cudaFree(g.done_gemm2);
-    cudaFree(g.cell_counts); cudaFree(g.flow_ctr); cudaFree(g.flow_stamps); cudaFree(g.flow_stalls); cudaFree(g.panels); cudaFree(g.tile_claims); cudaFree(g.status); cudaFree(g.gemm_stats);
+    cudaFree(g.cell_counts); cudaFree(g.place_hist); cudaFree(g.flow_ctr); cudaFree(g.flow_stamps); cudaFree(g.flow_stalls); cudaFree(g.panels); cudaFree(g.tile_claims); cudaFree(g.status); cudaFree(g.gemm_stats);
     cudaFree(g.col_partial); cudaFree(g.gate_stats);
     for (auto& e : g.ev)
         if (e) cudaEventDestroy(e);
@@ -928,7 +972,7 @@ static int initialize_impl(const char* config_json_path, int rank, int world, co
     if ((rc = dev_alloc(&g.cell_tokens, (size_t)cfg.E * cfg.pEC))) return rc;
     if ((rc = dev_alloc(&g.refine_list, (size_t)cfg.S))) return rc;
     if ((rc = dev_alloc(&g.refine_count, 1))) return rc;
-    if ((rc = dev_alloc(&g.tile_hist, (size_t)((cfg.S + kSlotTile - 1) / kSlotTile) * cfg.E))) return rc;
+    if ((rc = dev_alloc(&g.tile_hist, (size_t)((cfg.S + flow::BM - 1) / flow::BM) * cfg.E))) return rc;
     if ((rc = dev_alloc(&g.refine_done, (size_t)cfg.S))) return rc;
     if ((rc = dev_alloc(&g.refine_logits, (size_t)cfg.S * cfg.E))) return rc;
     if ((rc = dev_alloc(&g.le_start, (size_t)g.nLx + 1))) return rc;
@@ -950,7 +994,14 @@ static int initialize_impl(const char* config_json_path, int rank, int world, co
     if (const char* gs = std::getenv("KLEOS_GEMM_STATS"))
         if (gs[0] == '1' && (rc = dev_alloc(&g.gemm_stats, (size_t)2 * g.sm_count * kStatSlots))) return rc;
 
-    if (!dense && !((g.use_tc || g.use_tf32_tc) && cfg.PX <= 128)) {
+    const char* rk = std::getenv("KLEOS_ROUTE_KERNELS");
+    g.split_route = !dense && (g.use_tc || g.use_tf32_tc) && cfg.PX <= 128 && !(rk && rk[0] == '1');
+    if (g.split_route) {
+        rc = cfg.torch_dtype == 1   ? prepare_route_split<tf32_t>()
+             : cfg.torch_dtype == 2 ? prepare_route_split<__nv_bfloat16>()
+                                    : prepare_route_split<__half>();
+        if (rc) return rc;
+    } else if (!dense) {
         RouteArgs ra{};
         ra.PX = cfg.PX;
         rc = cfg.torch_dtype == 0   ? launch_route<float>(ra, 0, true)
@@ -959,6 +1010,7 @@ static int initialize_impl(const char* config_json_path, int rank, int world, co
                                     : launch_route<__half>(ra, 0, true);
         if (rc) return rc;
     }
+    if (!dense && (rc = dev_alloc(&g.place_hist, (size_t)((cfg.S + kPlaceOwn - 1) / kPlaceOwn) * place_words(cfg.PX)))) return rc;
     if (g.use_tc) {
         if (cfg.torch_dtype == 2) rc = set_tc_attributes<__nv_bfloat16>();
         else rc = set_tc_attributes<__half>();
@@ -972,10 +1024,7 @@ static int initialize_impl(const char* config_json_path, int rank, int world, co
         g.f32_bn[1] = f32_tile_width(cfg.H);
     }
     if (g.use_tf32_tc) {
-        const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
         if ((rc = set_gemm_attributes<tf32_t>())) return rc;
-        KLEOS_CUDA(cudaFuncSetAttribute(route_tc_kernel<tf32_t, 64>, dyn, route_tc::Shape<64>::SMEM_BYTES));
-        KLEOS_CUDA(cudaFuncSetAttribute(route_tc_kernel<tf32_t, 128>, dyn, route_tc::Shape<128>::SMEM_BYTES));
     }
     // KLEOS_FLOW=1 runs 16-bit routed layers as ONE persistent kernel (moe_flow.cuh).  It is the
     // reference's arrangement and passes the same parity tests, but on this machine it has so far
@@ -991,12 +1040,7 @@ static int initialize_impl(const char* config_json_path, int rank, int world, co
     g.local = world == 1 && !g.use_flow && !(dk && dk[0] == '1');
     const char* fr = std::getenv("KLEOS_FUSE_ROUTE");
     g.fuse_route = g.use_flow && cfg.PX <= 128 && !cfg.is_training && !(fr && fr[0] == '0');
-    // Separate launches of a 16-bit layer use the same kernel's routing phase as their router
-    // (KLEOS_ROUTE_KERNELS=1: the gate, near-tie, histogram and slot kernels instead)
-    const char* rk = std::getenv("KLEOS_ROUTE_KERNELS");
-    g.route_by_flow = g.use_tc && !dense && !g.use_flow && cfg.PX <= 128 && !cfg.is_training &&
-                      g.flow_grid >= 2 && cfg.E <= flow::kMaxCells && !(rk && rk[0] == '1');
-    if (g.use_flow || g.route_by_flow) {
+    if (g.use_flow) {
         flow::Counters* ctr = nullptr;
         if ((rc = dev_alloc(&ctr, 2))) return rc;
         g.flow_ctr = ctr;

@@ -169,13 +169,11 @@ struct Args {
     // routing inside the kernel (fuse_route != 0): the kernel then WRITES probs, topk, slots, mcw,
     // cell_tokens and counts before it reads them
     int fuse_route;
-    int route_only;          // with fuse_route: leave after the routing phase (router of the separate launches)
     const void* Wg;          // [PX,H] gate weight, row e = expert e
     const float* gate_bias;  // [E]
     int* tile_hist;          // [S/128][E] per-tile histogram of the chosen experts
     float tie_eps;
-    PanelEntry* panels;      // route_only on one rank: the panel list is written here (else null)
-    int* le_start;
+    int parts;               // parts of K whose gate logits are summed apart, as route_split.cuh does it
 };
 
 struct Tile {
@@ -569,9 +567,14 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t d_tmem = tmem_r + buf * BN;
                     bool ok = true;
+                    int part = 0, part_kb = 0;  // part of K the slice belongs to, and its first slice
                     for (int kb = 0; kb < KSr; ++kb, ++it) {
+                        if (kb == (part + 1) * KSr / a.parts) {
+                            ++part;
+                            part_kb = kb;
+                        }
+                        const uint32_t d_tmem = tmem_r + buf * BN + (uint32_t)(part * a.PX);
                         const int s = it % kSlices;
                         const uint32_t ph = (it / kSlices) & 1;
                         if (!mbar_wait(&ctl->full[s], ph, budget, abort_flag)) {
@@ -586,7 +589,7 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                         const uint64_t db = make_smem_desc(sa + A_STAGE_BYTES);
 #pragma unroll
                         for (int k = 0; k < BK / UMMA_K; ++k)
-                            umma_bf16_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                            umma_bf16_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb != part_kb || k != 0) ? 1u : 0u);
                         const uint32_t e_local = smem_u32(&ctl->empty[s]);
                         umma_commit_pair(map_to_cta(e_local, 0));
                         umma_commit_pair(map_to_cta(e_local, 1));
@@ -632,6 +635,19 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 const int row = row_w + lane;
                 const bool valid = row < a.S;
                 const uint32_t taddr = tmem_r + buf * BN + (static_cast<uint32_t>(q * 32) << 16);
+                // 32 logits, without their bias: the parts of K in order
+                auto load_logits = [&](int c, uint32_t* v) {
+                    tmem_ld_32x32(taddr + c * 32, v);
+                    tmem_ld_wait();
+#pragma unroll 1
+                    for (int p = 1; p < a.parts; ++p) {
+                        uint32_t w[32];
+                        tmem_ld_32x32(taddr + p * a.PX + c * 32, w);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
+                    }
+                };
                 float val[KC + 1];
                 int idx[KC + 1];
 #pragma unroll
@@ -642,8 +658,7 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
 #pragma unroll 1
                 for (int c = 0; c < chunks; ++c) {
                     uint32_t v[32];
-                    tmem_ld_32x32(taddr + c * 32, v);
-                    tmem_ld_wait();
+                    load_logits(c, v);
 #pragma unroll
                     for (int jj = 0; jj < 32; ++jj) {
                         const int e = c * 32 + jj;
@@ -666,18 +681,32 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 }
                 if (stamp && q == 0 && lane == 0) stamp[kTopkPass1] = global_ns();
                 const float m = val[0];
-                float d = 0.f;
+                // sum of the exponentials by quarters of the PX experts, then (q0 + q1) + (q2 + q3): the order
+                // in which the four threads per token of route_split.cuh add them
+                float quarter[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
                 for (int c = 0; c < chunks; ++c) {
                     uint32_t v[32];
-                    tmem_ld_32x32(taddr + c * 32, v);
-                    tmem_ld_wait();
+                    load_logits(c, v);
+                    float lo = 0.f, hi = 0.f;  // a chunk of 32 is a quarter (PX = 128) or two (PX = 64)
 #pragma unroll
-                    for (int jj = 0; jj < 32; ++jj) {
+                    for (int jj = 0; jj < 16; ++jj) {
                         const int e = c * 32 + jj;
-                        if (e < a.E) d += __expf(__uint_as_float(v[jj]) + bias_r[e] - m);
+                        if (e < a.E) lo += __expf(__uint_as_float(v[jj]) + bias_r[e] - m);
+                    }
+                    if (chunks > 2) hi = lo;
+#pragma unroll
+                    for (int jj = 16; jj < 32; ++jj) {
+                        const int e = c * 32 + jj;
+                        if (e < a.E) hi += __expf(__uint_as_float(v[jj]) + bias_r[e] - m);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        if (chunks > 2 ? k == c : k == 2 * c + 1) quarter[k] = hi;
+                        else if (chunks <= 2 && k == 2 * c) quarter[k] = lo;
                     }
                 }
+                const float d = (quarter[0] + quarter[1]) + (quarter[2] + quarter[3]);
                 const float inv = 1.f / d;
                 if (stamp && q == 0 && lane == 0) stamp[kTopkDone] = global_ns();
                 float kth = 0.f, next = -INFINITY;
@@ -702,8 +731,7 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
 #pragma unroll 1
                     for (int c = 0; c < chunks; ++c) {
                         uint32_t v[32];
-                        tmem_ld_32x32(taddr + c * 32, v);
-                        tmem_ld_wait();
+                        load_logits(c, v);
                         if (lane == src) {
 #pragma unroll
                             for (int jj = 0; jj < 32; ++jj) {
@@ -756,13 +784,12 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 float wsum = 0.f;
 #pragma unroll
                 for (int j = 0; j < KC; ++j)
-                    if (j < K) wsum += __expf(val[j] - m) * inv;
+                    if (j < K) wsum = fmaf(__expf(val[j] - m), inv, wsum);
                 // probabilities, padding columns zero, one 16-byte store per eight experts
 #pragma unroll 1
                 for (int c = 0; c < chunks; ++c) {
                     uint32_t v[32];
-                    tmem_ld_32x32(taddr + c * 32, v);
-                    tmem_ld_wait();
+                    load_logits(c, v);
                     if (c + 1 == chunks) {
                         // last read of this accumulator: hand it back to the MMA issuer
                         tc_fence_before();
@@ -886,13 +913,6 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                                    make_flag(a.epoch, (unsigned)min(total, a.EC)));
                 }
             };
-            auto write_plan = [&](int last_tile_too) {
-                if (a.panels == nullptr) return;
-                int* cnt = ctl->cnt_s;
-                for (int e = tid; e < a.E; e += kThreads)
-                    cnt[e] = min(base[e] + (last_tile_too ? __ldcg(a.tile_hist + (size_t)(n_tiles - 1) * a.E + e) : 0), a.EC);
-                write_local_plan(cnt, reinterpret_cast<int*>(ctl->prefix_s), a.E, a.pEC, a.rank, a.panels, a.le_start);
-            };
             // When the last block pair routed no tile it has nothing to do here: its second block
             // adds up ALL tiles and publishes the counts, off the path of the blocks that write
             // slots.  Otherwise the block of the last tile does it on top of its own work.
@@ -900,7 +920,6 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             if (spare && blockIdx.x == gridDim.x - 1) {
                 sum_tiles_before(n_tiles);
                 publish_counts(0);
-                write_plan(0);
             }
             for (int rt = cluster_id; rt < n_rt; rt += n_clusters) {
                 const int tile = rt * 2 + (int)cta_rank;
@@ -911,7 +930,6 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 if (stamp && tid == 0) stamp[kSlotBase] = global_ns();
                 if (!spare && tile == n_tiles - 1) {
                     publish_counts(1);
-                    write_plan(1);
                 }
                 const int n_own = min(BM, a.S - tok0) * a.K;
                 for (int i0 = 0; i0 < n_own; i0 += 256) {
@@ -950,22 +968,6 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         grid_barrier(1);
         if (stamp && tid == 0) stamp[kSlotted] = global_ns();
     }
-    if (a.route_only) {
-        // The router alone (the separate-launch arrangement uses this kernel as its router: one
-        // launch instead of gate, near-tie, histogram and slot kernels).  Same teardown as below.
-        tc_fence_before();
-        __syncthreads();
-        cluster_sync_all();
-        if (warp == 2) {
-            tc_fence_after();
-            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(ctl->tmem_base),
-                         "r"(TMEM_COLS)
-                         : "memory");
-        }
-        if (stamp && tid == 0) stamp[kEnd] = global_ns();
-        return;
-    }
-
     // ------------------------------------------------------------------ plan (every block, same result)
     // Routed count of every (source, local expert) cell, published by the sources' routers
     // (reference: the first-stage signal carries the count, types.cuh:300-317); then the panel

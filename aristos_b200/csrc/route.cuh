@@ -425,122 +425,189 @@ __global__ void __launch_bounds__(256) refine_kernel(RouteArgs a) {
     }
 }
 
-struct SlotArgs {
-    const int* topk;        // [S,K]
+// Slots in ascending token order (the reference hands them out in atomicAdd arrival order,
+// moe/gate.cuh:689-718; ascending order is one of its possible outcomes and is reproducible).
+struct PlaceArgs {
+    const int* topk;        // [S,K], place_kernel only
+    const void* A;          // [S,H]
     int* slots;             // [S,K] slot or kDropped
     int* cell_tokens;       // [E,pEC] token id held by each slot
     unsigned* counts;       // [E] unclamped
-    int* tile_hist;         // [tiles, E] per-tile histogram of the chosen experts
-    int S, K, E, EC, pEC;
-    // count flags: cflag[owner][rank*nLx + le] = (epoch<<32)|routed, one 8-byte peer store per
-    // expert (the reference's first-stage signal carries the same count, types.cuh:300-317)
-    char* peer_arena[kMaxWorld];
-    size_t cflag_offset;
-    int rank, nLx;
-    uint32_t epoch;
-    // one rank: the last block also writes the panel list (else null)
+    // [rows][place_words(PX)]: every block's histogram of chosen experts, four counts of 12 bits and 16 bits
+    // of the epoch in a word, so that a reader knows from the word itself that it is this forward's.  (A count
+    // reaches 128 * k = 1024: a token of NaN logits chooses expert 0 k times.)
+    unsigned long long* hist;
+    // several ranks: count flags, cflag[owner][rank*nLx + le] = (epoch<<32)|routed, one 8-byte peer store
+    // per expert (the reference's first-stage signal carries the same count, types.cuh:300-317)
+    PeerTable peers;
+    size_t cflag;
+    // one rank: the token rows go to this rank's own cells [E][pEC][H] (else null)
+    char* xcell;
+    unsigned row_chunks;    // 16-byte chunks of a token row
+    // one rank, GEMMs that work through a panel list: the last block writes it (else null)
     PanelEntry* panels;
     int* le_start;
+    DeviceStatus* status;
+    long long wait_cycles;
+    int S, K, E, PX, EC, pEC, nLx, rank, world;
+    uint32_t epoch;
 };
 
-// Slots in ascending token order (the reference hands them out in atomicAdd arrival order,
-// moe/gate.cuh:689-718; ascending order is one of its possible outcomes and is reproducible).
-// Two small launches over tiles of 128 tokens:
-//   tile_hist_kernel  per-tile histogram of the chosen experts;
-//   slot_kernel       base slot of every expert for the tile = sum of the earlier tiles'
-//                     histograms, then each token's rank inside the tile; the last block also
-//                     has the totals and publishes them: counts[e] and one count flag per
-//                     expert to the expert's owner rank.
-constexpr int kSlotTile = 128;
+constexpr int kPlaceThreads = 512, kPlaceWarps = kPlaceThreads / 32;
+constexpr int kPlaceMaxE = 256;
+__host__ __device__ constexpr int place_words(int px) { return px / 4; }  // px is a multiple of 64
+struct PlaceScratch {
+    int wcount[kPlaceWarps][kPlaceMaxE];
+    int part[kPlaceThreads * 4];
+    int base[kPlaceMaxE], total[kPlaceMaxE], off[kPlaceMaxE + 1];
+};
 
-__global__ void __launch_bounds__(256) tile_hist_kernel(SlotArgs a) {
-    __shared__ int hist[256];  // E <= 256
-    pdl_trigger();
-    pdl_wait();
-    const int tid = threadIdx.x, tok0 = blockIdx.x * kSlotTile;
-    for (int e = tid; e < a.E; e += blockDim.x) hist[e] = 0;
-    __syncthreads();
-    const int n_own = min(kSlotTile, a.S - tok0) * a.K;
-    for (int i = tid; i < n_own; i += blockDim.x) atomicAdd(&hist[a.topk[(size_t)tok0 * a.K + i]], 1);
-    __syncthreads();
-    for (int e = tid; e < a.E; e += blockDim.x) a.tile_hist[(size_t)blockIdx.x * a.E + e] = hist[e];
+__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
 }
 
-__global__ void __launch_bounds__(256) slot_kernel(SlotArgs a) {
-    __shared__ int base[256];
-    const int tid = threadIdx.x, b = blockIdx.x;
-    pdl_trigger();
-    pdl_wait();
-    const int tok0 = b * kSlotTile;
-    const bool last = b == (int)gridDim.x - 1;
-    // base slot of every expert = sum of the earlier tiles' histograms; the tiles are split
-    // over the threads that share an expert so the loads are independent and coalesced
-    __shared__ int part[256];
-    {
-        int ep = 1;
-        while (ep < a.E) ep <<= 1;            // experts rounded up to a power of two (<= 256)
-        const int groups = blockDim.x / ep;   // threads per expert
-        const int e = tid % ep, grp = tid / ep;
-        int run = 0;
-        if (e < a.E && grp < groups)
-            for (int t = grp; t < b; t += groups) run += a.tile_hist[(size_t)t * a.E + e];
-        part[tid] = run;
-        __syncthreads();
-        if (tid < a.E) {
-            int sum = 0;
-            for (int gi = 0; gi < groups; ++gi) sum += part[gi * ep + tid];
-            base[tid] = sum;
-        }
-        __syncthreads();
+// Slots, counts and (one rank) the way of the rows into the cells for one block's `own` <= 128 tokens, from tok0
+// on, row `row` of n_rows: 512 threads, all of them.  top[own * K] and hist[PX] are the chosen experts and
+// their histogram, in shared memory.  The block publishes its histogram and adds up those of the rows
+// before it as they come, without a fence, a flag or a grid barrier: it only waits for blocks of lower
+// index.  A wait that runs out raises *abort_flag.
+__device__ __forceinline__ void place_tokens(const PlaceArgs& a, int row, int n_rows, int tok0, int own, int* top, const int* hist,
+                                             PlaceScratch* s, volatile int* abort_flag, DeviceStatus* status) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, K = a.K, E = a.E, words = place_words(a.PX);
+    if (tid < words && !*abort_flag) {
+        unsigned long long w = (unsigned long long)(a.epoch & 0xffffu) << 48;
+        for (int j = 0; j < 4; ++j) w |= (unsigned long long)hist[4 * tid + j] << (12 * j);
+        asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(a.hist + (size_t)row * words + tid), "l"(w) : "memory");
     }
-    __shared__ int routed[256], off[257];
-    for (int e = tid; e < a.E; e += blockDim.x) {
-        const int run = base[e];
-        if (last) {
-            const int total = run + a.tile_hist[(size_t)b * a.E + e];
-            a.counts[e] = (unsigned)total;
-            const int owner = e / a.nLx, le = e - owner * a.nLx;
-            st_release_sys(reinterpret_cast<unsigned long long*>(a.peer_arena[owner] + a.cflag_offset) +
-                               ((size_t)a.rank * a.nLx + le),
-                           make_flag(a.epoch, (unsigned)min(total, a.EC)));
-            routed[e] = min(total, a.EC);
-        }
-    }
-    if (last && a.panels != nullptr) write_local_plan(routed, off, a.E, a.pEC, a.rank, a.panels, a.le_start);
-    // Rank of every (token, choice) entry among the earlier entries of the tile that chose the
-    // same expert.  Entries are taken in order, 256 at a time: inside a warp the rank comes from
-    // a match mask, across the eight warps from a per-warp count table, and `base` carries the
-    // running total into the next group of 256.
-    __shared__ int wcount[8][256];
-    for (int i = tid; i < 8 * 256; i += blockDim.x) (&wcount[0][0])[i] = 0;
-    const int n_own = min(kSlotTile, a.S - tok0) * a.K;
-    const int warp = tid >> 5, lane = tid & 31;
-    __syncthreads();
-    for (int i0 = 0; i0 < n_own; i0 += 256) {
-        const int i = i0 + tid;
-        const int e = i < n_own ? a.topk[(size_t)tok0 * a.K + i] : -1;
-        const unsigned peers = __match_any_sync(0xffffffffu, e);
-        const int before = __popc(peers & ((1u << lane) - 1u));
-        const bool leader = e >= 0 && before == 0;
-        if (leader) wcount[warp][e] = __popc(peers);
-        __syncthreads();
-        if (e >= 0) {
-            int pos = base[e] + before;
-            for (int w = 0; w < warp; ++w) pos += wcount[w][e];
-            if (pos < a.EC) {
-                a.slots[(size_t)tok0 * a.K + i] = pos;
-                a.cell_tokens[(size_t)e * a.pEC + pos] = tok0 + i / a.K;
-            } else {
-                a.slots[(size_t)tok0 * a.K + i] = kDropped;
+    for (int i = tid; i < kPlaceWarps * kPlaceMaxE; i += kPlaceThreads) (&s->wcount[0][0])[i] = 0;
+    // `width` threads per row, a word each; four rows in flight
+    const int width = words <= 16 ? 16 : words <= 32 ? 32 : 64, groups = kPlaceThreads / width;
+    const int word = tid % width, grp = tid / width;
+    int run[4] = {0, 0, 0, 0};
+    if (word < words) {
+        const long long t0 = clock64();
+#pragma unroll 1
+        for (int r0 = grp; r0 < row && !*abort_flag; r0 += 4 * groups) {
+            unsigned long long v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                v[j] = r0 + j * groups < row ? ld_relaxed_u64(a.hist + (size_t)(r0 + j * groups) * words + word) : 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (r0 + j * groups >= row) break;
+                while ((uint32_t)(v[j] >> 48) != (a.epoch & 0xffffu)) {
+                    __nanosleep(100);
+                    v[j] = ld_relaxed_u64(a.hist + (size_t)(r0 + j * groups) * words + word);
+                    if (*abort_flag) break;
+                    if (clock64() - t0 > a.wait_cycles) {
+                        report_error(status, KLEOS_AT_GRID_BARRIER, row, (int)a.epoch);
+                        *abort_flag = 1;
+                        break;
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) run[q] += (int)((v[j] >> (12 * q)) & 0xfff);
             }
         }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s->part[(grp * width + word) * 4 + q] = run[q];
+    }
+    __syncthreads();
+    for (int e = tid; e < a.PX; e += kPlaceThreads) {
+        int sum = 0;
+#pragma unroll 4
+        for (int i = 0; i < groups; ++i) sum += s->part[i * width * 4 + e];
+        s->base[e] = sum;
+        s->total[e] = sum + hist[e];
+    }
+    __syncthreads();
+    if (*abort_flag) return;  // (the same for all threads: nothing raises it from here on)
+    // Rank of every (token, choice) entry among the earlier entries of the block that chose the same
+    // expert: inside a warp from a match mask, across the warps from a per-warp count table.
+    const int n_own = own * K;
+#pragma unroll 1
+    for (int i0 = 0; i0 < n_own; i0 += kPlaceThreads) {
+        const int i = i0 + tid;
+        const int e = i < n_own ? top[i] : -1;
+        const unsigned same = __match_any_sync(0xffffffffu, e);
+        const int before = __popc(same & ((1u << lane) - 1u));
+        const bool lead = e >= 0 && before == 0;
+        if (lead) s->wcount[warp][e] = __popc(same);
         __syncthreads();
-        if (leader) {
-            atomicAdd(&base[e], wcount[warp][e]);
-            wcount[warp][e] = 0;
+        if (e >= 0) {
+            int pos = s->base[e] + before;
+            for (int w = 0; w < warp; ++w) pos += s->wcount[w][e];
+            const bool kept = pos < a.EC;
+            a.slots[(size_t)tok0 * K + i] = kept ? pos : kDropped;
+            if (kept) a.cell_tokens[(size_t)e * a.pEC + pos] = tok0 + i / K;
+            top[i] = kept ? e * a.pEC + pos : -1;  // from here on: the entry's row in the cells
+        }
+        __syncthreads();
+        if (lead) {
+            atomicAdd(&s->base[e], s->wcount[warp][e]);
+            s->wcount[warp][e] = 0;
         }
         __syncthreads();
     }
+    if (row == n_rows - 1) {
+        // totals of every expert: unclamped count for this rank, clamped count to the owner
+        for (int e = tid; e < E; e += kPlaceThreads) {
+            const int total = s->total[e];
+            a.counts[e] = (unsigned)total;
+            s->total[e] = min(total, a.EC);
+            if (a.world > 1 || a.xcell == nullptr) {
+                const int owner = e / a.nLx, le = e - owner * a.nLx;
+                st_release_sys(reinterpret_cast<unsigned long long*>(a.peers.arena[owner] + a.cflag) + ((size_t)a.rank * a.nLx + le),
+                               make_flag(a.epoch, (unsigned)min(total, a.EC)));
+            }
+        }
+        if (a.panels != nullptr) write_local_plan(s->total, s->off, E, a.pEC, a.rank, a.panels, a.le_start);
+    }
+    if (a.xcell != nullptr) {
+        // a warp per token, which is read once and stored to each expert that kept it
+#pragma unroll 1
+        for (int tk = warp; tk < own; tk += kPlaceWarps) {
+            const uint4* src = static_cast<const uint4*>(a.A) + (size_t)(tok0 + tk) * a.row_chunks;
+#pragma unroll 1
+            for (unsigned c0 = lane; c0 - lane < a.row_chunks; c0 += 256) {
+                uint4 v[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    if (c0 + 32 * q < a.row_chunks) v[q] = __ldg(src + c0 + 32 * q);
+#pragma unroll 1
+                for (int j = 0; j < K; ++j) {
+                    const int to = top[tk * K + j];
+                    if (to < 0) continue;
+                    uint4* dst = reinterpret_cast<uint4*>(a.xcell) + (size_t)to * a.row_chunks;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (c0 + 32 * q < a.row_chunks) dst[c0 + 32 * q] = v[q];
+                }
+            }
+        }
+    }
+}
+
+// The same on its own, behind the routers whose blocks do not have 512 threads or whose choices the near-tie
+// kernel may change: one block per 32 tokens.  It stands for three kernels (histogram, slots, rows).
+constexpr int kPlaceOwn = 32;
+__global__ void __launch_bounds__(kPlaceThreads) place_kernel(PlaceArgs a) {
+    __shared__ PlaceScratch s;
+    __shared__ int hist[kPlaceMaxE], top[kPlaceOwn * kMaxTopK], abort;
+    pdl_wait();
+    pdl_trigger();
+    const int tid = threadIdx.x, tok0 = blockIdx.x * kPlaceOwn, own = min(kPlaceOwn, a.S - tok0);
+    for (int e = tid; e < kPlaceMaxE; e += kPlaceThreads) hist[e] = 0;
+    if (tid == 0) abort = 0;
+    __syncthreads();
+    if (tid < own * a.K) {
+        top[tid] = a.topk[(size_t)tok0 * a.K + tid];
+        atomicAdd(&hist[top[tid]], 1);
+    }
+    __syncthreads();
+    place_tokens(a, blockIdx.x, gridDim.x, tok0, own, top, hist, &s, &abort, a.status);
 }
 
 }  // namespace kleos

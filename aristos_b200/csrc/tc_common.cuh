@@ -258,7 +258,7 @@ __device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a,
 // One lane of a converged warp, the same one every time.  The MMA warps of ffn_gemm_tc2 and ffn_gemm_f32
 // run their loops as a whole and let the elected lane issue: operand descriptors and addresses then
 // live in uniform registers, where the instruction wants them.  (The loops of moe_flow.cuh and
-// route_tc.cuh are run by lane 0 alone, and move each instruction's descriptors there first.)
+// route_split.cuh are run by lane 0 alone, and move each instruction's descriptors there first.)
 __device__ __forceinline__ uint32_t elect_one() {
     uint32_t e;
     asm volatile(

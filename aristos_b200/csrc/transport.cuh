@@ -116,49 +116,6 @@ __global__ void __launch_bounds__(256) dispatch_kernel(DispatchArgs a) {
     }
 }
 
-struct LocalDispatchArgs {
-    const void* A;        // [S,H]
-    const int* topk;      // [S,K]
-    const int* slots;     // [S,K]
-    char* xcell;          // [E][pEC][H] this rank's own cells
-    int S, K, pEC;
-    unsigned row_chunks;  // 16-byte chunks of a row
-};
-constexpr int kDispatchTokens = 8;  // warps of a block, one token each
-
-// Dispatch on one rank: warp per token, which is read once and stored to each expert that kept it (the
-// kernel above goes by destination row, reads a token once per expert, and has to find its place in the
-// sending order first).  Bound by L2 and HBM: S rows in, S k rows out.
-// 8192 tokens, k = 2, 4 KiB rows (96 MiB in all): 12.7 us, the kernel above 19.6.
-__global__ void __launch_bounds__(kDispatchTokens * 32) dispatch_local_kernel(LocalDispatchArgs a) {
-    pdl_trigger();
-    pdl_wait();
-    const int t = blockIdx.x * kDispatchTokens + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (t >= a.S) return;
-    // destination row of choice `lane`, k <= 8
-    long long row = -1;
-    if (lane < a.K) {
-        const int e = a.topk[(size_t)t * a.K + lane], slot = a.slots[(size_t)t * a.K + lane];
-        if (slot != kDropped) row = (long long)e * a.pEC + slot;
-    }
-    const uint4* src = static_cast<const uint4*>(a.A) + (size_t)t * a.row_chunks;
-    uint4* cells = reinterpret_cast<uint4*>(a.xcell);
-    for (unsigned c0 = lane; c0 - lane < a.row_chunks; c0 += 256) {
-        uint4 v[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-            if (c0 + 32 * q < a.row_chunks) v[q] = __ldg(src + c0 + 32 * q);
-        for (int j = 0; j < a.K; ++j) {
-            const long long to = __shfl_sync(0xffffffffu, row, j);
-            if (to < 0) continue;
-            uint4* dst = cells + to * a.row_chunks;
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-                if (c0 + 32 * q < a.row_chunks) dst[c0 + 32 * q] = v[q];
-        }
-    }
-}
-
 // One 128-row panel of one cell: what a GEMM m-tile works on.
 struct PanelEntry {
     int row_base;  // first row in the xcell / y1cell row space

@@ -480,7 +480,7 @@ ffn_gemm_f32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(Sh::TMEM_COLS)
                      : "memory");
     }
-    if (g.mode == 1) publish_return_flags(g.ret, &ctl->last_block);
+    if (g.mode == 1 && g.ret.world > 0) publish_return_flags(g.ret, &ctl->last_block);
 }
 
 }  // namespace kleos

@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(256) ffn_gemm_simt(GemmArgs g) {
             }
         }
     }
-    if (g.mode == 1) publish_return_flags(g.ret, &last_block);
+    if (g.mode == 1 && g.ret.world > 0) publish_return_flags(g.ret, &last_block);
 }
 
 }  // namespace kleos

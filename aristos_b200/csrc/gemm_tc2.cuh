@@ -611,7 +611,7 @@ ffn_gemm_tc2(const __grid_constant__ gemm_tc2::RowMaps map_x, const __grid_const
     }
     // the last pair to finish leaves the counters as it found them
     if (leader && tid == 0 && atomicInc(g.next_tile + 1, (unsigned)n_clusters - 1) == (unsigned)n_clusters - 1) g.next_tile[0] = 0;
-    if (g.mode == 1) publish_return_flags(g.ret, &ctl->last_block);
+    if (g.mode == 1 && g.ret.world > 0) publish_return_flags(g.ret, &ctl->last_block);
 }
 
 }  // namespace kleos

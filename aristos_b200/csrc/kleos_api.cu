@@ -668,7 +668,8 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     ga.hidden_act = c.hidden_act; ga.nLx = g.nLx; ga.pEC = c.pEC; ga.rank = g.rank;
     ga.elem_bytes = c.elem_bytes; ga.epoch = g.epoch; ga.le_begin = 0; ga.le_end = g.nLx;
     ga.ret.peers = g.peers; ga.ret.lay = g.lay; ga.ret.done_counter = g.done_gemm2;
-    ga.ret.rank = g.rank; ga.ret.world = g.world; ga.ret.epoch = g.epoch;
+    const int flags = g.local && !g.suppress_return_flag ? 0 : g.world;  // (the test hook needs something to wait for)
+    ga.ret.rank = g.rank; ga.ret.world = flags; ga.ret.epoch = g.epoch;
     ga.ret.suppress = g.suppress_return_flag ? 1 : 0;
     ga.contiguous = g.world == 1; ga.next_tile = g.tile_claims; ga.counts = g.counts; ga.EC = c.EC;
     GemmArgs g1 = ga;
@@ -706,7 +707,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     CombineArgs ca{};
     ca.arena = g.arena; ca.lay = g.lay; ca.probs = s.probs; ca.topk = g.topk; ca.slots = g.slots;
     ca.mcw = g.mcw; ca.out = s.out; ca.status = g.status; ca.S = c.S; ca.H = c.H; ca.K = c.K;
-    ca.PX = c.PX; ca.pEC = c.pEC; ca.world = g.world; ca.epoch = g.epoch;
+    ca.PX = c.PX; ca.pEC = c.pEC; ca.world = flags; ca.epoch = g.epoch;
     ca.wait_cycles = g.wait_cycles;
     if (c.K == 2)
         launch(combine_kernel<T, 2>, g.sm_count * 4, 256, 0, st, ca);

@@ -606,11 +606,13 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
         KLEOS_CUDA(mark());
     }
 
-    if (!routed_in_kernel) {
-        if (g.col_partial)
-            launch(gate_stats_kernel, 1, 256, 0, st, g.col_partial, route_blocks, c.PX, g.counts, c.S, c.E, g.gate_stats);
+    GateStatsArgs gs{};
+    if (g.col_partial) {
+        gs.col_partial = g.col_partial; gs.counts = g.counts; gs.out = g.gate_stats; gs.blocks = route_blocks;
+        gs.PX = c.PX; gs.S = c.S; gs.E = c.E;
     }
     if (g.use_flow) {
+        if (g.col_partial) launch(gate_stats_kernel, 1, 256, 0, st, gs);
         if constexpr (sizeof(T) == 2) {
             // 3.-7. one persistent kernel: dispatch, plan, GEMM1, GEMM2, combine
             flow::Args fa{};
@@ -708,13 +710,14 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     ca.arena = g.arena; ca.lay = g.lay; ca.probs = s.probs; ca.topk = g.topk; ca.slots = g.slots;
     ca.mcw = g.mcw; ca.out = s.out; ca.status = g.status; ca.S = c.S; ca.H = c.H; ca.K = c.K;
     ca.PX = c.PX; ca.pEC = c.pEC; ca.world = flags; ca.epoch = g.epoch;
-    ca.wait_cycles = g.wait_cycles;
+    ca.wait_cycles = g.wait_cycles; ca.stats = gs;
+    const int combine_blocks = g.sm_count * 4 + (g.col_partial ? 1 : 0);
     if (c.K == 2)
-        launch(combine_kernel<T, 2>, g.sm_count * 4, 256, 0, st, ca);
+        launch(combine_kernel<T, 2>, combine_blocks, 256, 0, st, ca);
     else if (c.K == 1)
-        launch(combine_kernel<T, 1>, g.sm_count * 4, 256, 0, st, ca);
+        launch(combine_kernel<T, 1>, combine_blocks, 256, 0, st, ca);
     else
-        launch(combine_kernel<T, 0>, g.sm_count * 4, 256, 0, st, ca);
+        launch(combine_kernel<T, 0>, combine_blocks, 256, 0, st, ca);
     KLEOS_CUDA(mark());
     KLEOS_CUDA(cudaGetLastError());
     return KLEOS_OK;

@@ -290,36 +290,6 @@ __global__ void __launch_bounds__(256) route_kernel(RouteArgs a) {
     }
 }
 
-// Training-mode gate statistics of one rank's tokens, as the reference keeps them in its
-// bookkeeping (types.cuh:944-960): mean probability per expert (moe/gate.cuh:607-635), fraction
-// of the tokens that chose each expert (unclamped, :698-705) and the auxiliary loss
-// sum_e mean_prob[e] * mean_count[e] / E (:763-773).  One block; all sums in a fixed order.
-// out = [mean_prob E][mean_count E][loss 1].
-__global__ void __launch_bounds__(256) gate_stats_kernel(const float* col_partial, int blocks,
-                                                         int PX, const unsigned* counts, int S,
-                                                         int E, float* out) {
-    __shared__ float term[256];
-    pdl_trigger();
-    pdl_wait();
-    const int e = threadIdx.x;
-    float t = 0.f;
-    if (e < E) {
-        float sum = 0.f;
-        for (int b = 0; b < blocks; ++b) sum += col_partial[(size_t)b * PX + e];
-        const float mp = sum / (float)S, mc = (float)counts[e] / (float)S;
-        out[e] = mp;
-        out[E + e] = mc;
-        t = mp * mc / (float)E;
-    }
-    term[e] = t;
-    __syncthreads();
-    if (e == 0) {
-        float loss = 0.f;
-        for (int i = 0; i < E; ++i) loss += term[i];
-        out[2 * E] = loss;
-    }
-}
-
 // fp64 re-evaluation of the tokens on the refine list.  One warp per (listed token, expert)
 // dot product; the warp that completes a token's last logit redoes that token's selection.
 template <typename T>

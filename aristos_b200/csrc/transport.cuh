@@ -229,7 +229,52 @@ __global__ void __launch_bounds__(1024) plan_kernel(PlanArgs a) {
     }
 }
 
+// Training-mode gate statistics of one rank's tokens, as the reference keeps them in its
+// bookkeeping (types.cuh:944-960): mean probability per expert (moe/gate.cuh:607-635), fraction
+// of the tokens that chose each expert (unclamped, :698-705) and the auxiliary loss
+// sum_e mean_prob[e] * mean_count[e] / E (:763-773).  One block of 256 threads; all sums in a fixed order.
+// out = [mean_prob E][mean_count E][loss 1].
+struct GateStatsArgs {
+    const float* col_partial;  // [blocks][PX] column sums of the router's blocks, or null
+    const unsigned* counts;    // [E]
+    float* out;
+    int blocks, PX, S, E;
+};
+__device__ __forceinline__ void gate_stats(const GateStatsArgs& a) {
+    __shared__ float part[256], term[256];
+    // 256 / PX threads per expert (PX = 192: one), each with its own run of blocks
+    const int groups = 256 / a.PX, e = threadIdx.x % a.PX, grp = threadIdx.x / a.PX, per = (a.blocks + groups - 1) / groups;
+    float sum = 0.f;
+    if (grp < groups) {
+#pragma unroll 8
+        for (int b = grp * per; b < min((grp + 1) * per, a.blocks); ++b) sum += a.col_partial[(size_t)b * a.PX + e];
+    }
+    part[threadIdx.x] = sum;
+    __syncthreads();
+    float t = 0.f;
+    if ((int)threadIdx.x < a.E) {
+        for (int i = 1; i < groups; ++i) sum += part[i * a.PX + e];
+        const float mp = sum / (float)a.S, mc = (float)a.counts[e] / (float)a.S;
+        a.out[e] = mp;
+        a.out[a.E + e] = mc;
+        t = mp * mc / (float)a.E;
+    }
+    term[threadIdx.x] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float loss = 0.f;
+        for (int i = 0; i < a.E; ++i) loss += term[i];
+        a.out[2 * a.E] = loss;
+    }
+}
+__global__ void __launch_bounds__(256) gate_stats_kernel(GateStatsArgs a) {
+    pdl_trigger();
+    pdl_wait();
+    gate_stats(a);
+}
+
 struct CombineArgs {
+    GateStatsArgs stats;  // training mode: a last block beside those of the combine computes them
     const char* arena;   // this rank's arena (ycell, yflag)
     ArenaLayout lay;
     const void* probs;   // [S,PX] element-rounded gate probabilities
@@ -254,6 +299,11 @@ __global__ void __launch_bounds__(256) combine_kernel(CombineArgs a) {
     __shared__ int failed;
     pdl_trigger();
     pdl_wait();
+    const int blocks = (int)gridDim.x - (a.stats.col_partial != nullptr ? 1 : 0);
+    if ((int)blockIdx.x == blocks) {
+        gate_stats(a.stats);
+        return;
+    }
     if (threadIdx.x == 0) failed = 0;
     __syncthreads();
     if (threadIdx.x < a.world) {
@@ -273,7 +323,7 @@ __global__ void __launch_bounds__(256) combine_kernel(CombineArgs a) {
     constexpr int UNR = KT > 0 && KT <= 2 ? 4 : 1;
     const int K = KT > 0 ? KT : a.K;
     const int lane = threadIdx.x & 31;
-    const int warps = gridDim.x * (blockDim.x >> 5);
+    const int warps = blocks * (blockDim.x >> 5);
     const T* probs = static_cast<const T*>(a.probs);
     const T* ycell = reinterpret_cast<const T*>(a.arena + a.lay.ycell);
     const int chunks = a.H / VEC;

@@ -76,10 +76,11 @@ __device__ __forceinline__ int box_of(int rows) {
 
 // A tile, as the scheduler hands it to the other roles.  Block r of the pair loads rows[r] token rows from
 // row_base[r] on; `half` of them, a multiple of 16, go into the MMA from each block.
+constexpr int kReadOnce = 1 << 16;
 struct __align__(16) Task {
     int half;          // 0: no more tiles
     int le, mt;        // local expert, 256-column tile
-    int src;           // source ranks, eight bits each
+    int src;           // source ranks, eight bits each, and kReadOnce when no other tile reads these weights
     int row_base[2], rows[2];
 };
 
@@ -143,6 +144,7 @@ __device__ __forceinline__ Task decode_task(int t, const Control* ctl, const Gem
         x.src = a.src | (b.src << 8);
         x.half = (max(x.rows[0], x.rows[1]) + 15) >> 4 << 4;
     }
+    if (splits == 1) x.src |= kReadOnce;
     return x;
 }
 
@@ -362,6 +364,9 @@ ffn_gemm_tc2(const __grid_constant__ gemm_tc2::RowMaps map_x, const __grid_const
             asm volatile("fence.proxy.async;" ::: "memory");
             uint32_t it = 0;
             long long w_unused = 0;
+            // weights that one tile reads leave L2 first, so that the rows between the kernels stay there
+            uint64_t stream;
+            asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(stream));
             for (uint32_t i = 0;; ++i) {
                 const Task x = take(i, KLEOS_AT_GEMM_PRODUCER);
                 if (x.half == 0) break;
@@ -377,7 +382,9 @@ ffn_gemm_tc2(const __grid_constant__ gemm_tc2::RowMaps map_x, const __grid_const
                         break;
                     }
                     const uint32_t full_leader = map_to_cta(smem_u32(&ctl->full[s]), 0);
-                    tma_load_2d_pair(tiles + s * SLICE_BYTES, &map_w, kb * BKE, brow, full_leader);
+                    uint8_t* dst = tiles + s * SLICE_BYTES;
+                    if (x.src & kReadOnce) tma_load_2d_pair_hint(dst, &map_w, kb * BKE, brow, full_leader, stream);
+                    else tma_load_2d_pair(dst, &map_w, kb * BKE, brow, full_leader);
                 }
                 if (!ok) break;
             }

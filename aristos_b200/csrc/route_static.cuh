@@ -17,7 +17,7 @@
 
 #include <cstdio>
 
-#include "route.cuh"
+#include "route_split.cuh"
 
 namespace {
 
@@ -27,6 +27,7 @@ constexpr int kMaxDevices = 64;
 
 // Layout of the scratch array (byte offsets, all 256-byte aligned).
 constexpr size_t kOffCount = 0;                                                // int
+constexpr size_t kOffStatus = 64;                                              // DeviceStatus
 constexpr size_t kOffDone = 256;                                               // int[S]
 constexpr size_t kOffList = kOffDone + sizeof(int) * kStaticMaxTokens;         // int[S]
 constexpr size_t kOffZeroBias = kOffList + sizeof(int) * kStaticMaxTokens;     // float[E], stays 0
@@ -74,7 +75,8 @@ extern "C" int kleos_route_static(const void* A, const void* Wg, const float* ga
         cudaError_t e = cudaGetSymbolAddress(&p, g_route_scratch);
         const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
         if (e == cudaSuccess) e = cudaFuncSetAttribute(route_kernel<float, 64>, dyn, route_fma::smem_bytes<float, 64>());
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(route_kernel<__nv_bfloat16, 64>, dyn, route_fma::smem_bytes<__nv_bfloat16, 64>());
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(route_split_kernel<__nv_bfloat16, 64, 2>, dyn, route_split::Shape<64>::SMEM_BYTES);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(route_split_kernel<__nv_bfloat16, 64, 0>, dyn, route_split::Shape<64>::SMEM_BYTES);
         if (e != cudaSuccess || !p) {
             std::fprintf(stderr, "[kleos_b200] setting up kleos_route_static failed: %s\n",
                          cudaGetErrorString(e));
@@ -84,11 +86,6 @@ extern "C" int kleos_route_static(const void* A, const void* Wg, const float* ga
     }
     unsigned char* scratch = g_scratch_ptr[dev];
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : cudaStreamPerThread;
-
-    // the counter, the completion flags and the zero bias must start at zero; the previous
-    // call (or an aborted one) may have left anything there
-    if (cudaMemsetAsync(scratch, 0, kClearBytes, st) != cudaSuccess)
-        return complain(KLEOS_E_CUDA, "cudaMemsetAsync on the scratch array failed");
 
     RouteArgs ra{};
     ra.A = A;
@@ -107,13 +104,42 @@ extern "C" int kleos_route_static(const void* A, const void* Wg, const float* ga
     ra.K = K;
     ra.PX = 64;
     ra.tie_eps = 1e-4f;
-    const int grid = (S + route_fma::TM - 1) / route_fma::TM;
     if (torch_dtype == 0) {
+        // the counter, the completion flags and the zero bias must start at zero; the previous
+        // call (or an aborted one) may have left anything there
+        if (cudaMemsetAsync(scratch, 0, kClearBytes, st) != cudaSuccess)
+            return complain(KLEOS_E_CUDA, "cudaMemsetAsync on the scratch array failed");
+        const int grid = (S + route_fma::TM - 1) / route_fma::TM;
         route_kernel<float, 64><<<grid, 256, route_fma::smem_bytes<float, 64>(), st>>>(ra);
         refine_kernel<float><<<148, 256, 0, st>>>(ra);
     } else {
-        route_kernel<__nv_bfloat16, 64><<<grid, 256, route_fma::smem_bytes<__nv_bfloat16, 64>(), st>>>(ra);
-        refine_kernel<__nv_bfloat16><<<148, 256, 0, st>>>(ra);
+        // bf16 goes to the tensor cores (route_split.cuh): four blocks per 128 tokens, or as many as there
+        // are 64-wide slices of K.  mCw is a 32-bit result, so the running sums stay short: eight accumulators
+        // a block, added up in fp32 registers, each over an eighth of the block's slices.
+        CUtensorMap map_a, map_wg;
+        const char* err = encode_map(&map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, (uint64_t)S, (uint64_t)H, route_split::BM, 64);
+        if (!err) err = encode_map(&map_wg, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, Wg, 64, (uint64_t)H, 64, 64);
+        if (err) return complain(KLEOS_E_CUDA, err);
+        route_split::Args sp{};
+        sp.r = ra;
+        sp.status = reinterpret_cast<DeviceStatus*>(scratch + kOffStatus);
+        sp.place.wait_cycles = 20000000000LL;
+        const int slices = H / 64;
+        sp.parts = slices >= 4 ? 4 : slices >= 2 ? 2 : 1;
+        sp.acc_slices = ((slices + sp.parts - 1) / sp.parts + 7) / 8;
+        cudaLaunchConfig_t lc{};
+        lc.gridDim = dim3((unsigned)((S + route_split::BM - 1) / route_split::BM * sp.parts));
+        lc.blockDim = dim3(route_split::kThreads);
+        lc.dynamicSmemBytes = route_split::Shape<64>::SMEM_BYTES;
+        lc.stream = st;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)sp.parts;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        lc.attrs = &at;
+        lc.numAttrs = 1;
+        if (K == 2) cudaLaunchKernelEx(&lc, route_split_kernel<__nv_bfloat16, 64, 2>, map_a, map_wg, sp);
+        else cudaLaunchKernelEx(&lc, route_split_kernel<__nv_bfloat16, 64, 0>, map_a, map_wg, sp);
     }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {

@@ -37,6 +37,7 @@ struct GemmArgs {
     int contiguous;        // the rows of a local expert lie one after the other (one source rank)
     const unsigned* counts;  // contiguous: unclamped rows of every expert, EC of them kept; null: pEC rows of one expert
     int EC;
+    const int* row_token;    // gathering form: token whose activations are row r of the cells
     int plan_ready;        // the plan was complete before the kernel in front of this one began
 };
 

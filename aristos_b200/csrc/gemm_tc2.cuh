@@ -51,6 +51,8 @@ constexpr int W_BYTES = BM * 128;                   // one K slice of the weight
 constexpr int SLICE_BYTES = W_BYTES + kMaxHalf * 128;
 constexpr int kSteps = 4;                           // instructions per K slice, 32 bytes of a row each
 constexpr int kBackWarps = 8, kThreads = (4 + kBackWarps) * 32;
+constexpr int kGatherWarps = 4;
+template <bool kGather> constexpr int kBlock = kThreads + (kGather ? kGatherWarps * 32 : 0);
 constexpr int TMEM_COLS = 512, kSlotCols = 32, kSlots = TMEM_COLS / kSlotCols;
 // tiles on their way: at most six in the K ring, two ahead of it, sixteen in tensor memory
 constexpr int kTasks = 32;
@@ -223,8 +225,13 @@ __device__ __forceinline__ void arrive_relaxed(uint32_t cluster_addr) {
 // (Six stages of one K slice: three of two slices, with half the barrier round trips, took 1516 us instead of 1505
 // on the layer of 4096 tokens, H = 4096, I = 14336, 8 experts, and 65.3 instead of 64.3 on the dense layer of
 // 4096 tokens, H = I = 2048.)
-template <typename TE, int kEpi>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_tc2::kThreads, 1)
+// kGather: the token rows are fetched from the activations by token index, four rows a copy, instead of from
+// the cells, so that on one rank nobody copies them there (a layer of 8192 tokens, k = 2, 4 KiB rows: 13 us
+// of the router's 43, and 64 MB written and read back).  Four warps issue the copies: 128 rows take 0.33 us,
+// which a weight stream from HBM hides (0.4 us a slice) and the tensor pipe at 256 rows a tile does not
+// (0.26 us); one warp took 1.06.
+template <typename TE, int kEpi, bool kGather>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_tc2::kBlock<kGather>, 1)
 ffn_gemm_tc2(const __grid_constant__ gemm_tc2::RowMaps map_x, const __grid_constant__ CUtensorMap map_w, GemmArgs g) {
     using namespace tc;
     using namespace gemm_tc2;
@@ -258,7 +265,7 @@ ffn_gemm_tc2(const __grid_constant__ gemm_tc2::RowMaps map_x, const __grid_const
     // weights: its first weight slices are on their way before the first GEMM has ended.
     if (!g.plan_ready) pdl_wait();
     const int MT = (g.N + 2 * BM - 1) / (2 * BM);
-    for (int e = tid; e < g.nLx; e += kThreads) {
+    for (int e = tid; e < g.nLx; e += kBlock<kGather>) {
         const bool in = e >= g.le_begin && e < g.le_end;
         if (g.contiguous) {
             ctl->rows[e] = !in ? 0 : g.counts ? (int)min(g.counts[e], (unsigned)g.EC) : g.pEC;
@@ -329,9 +336,9 @@ ffn_gemm_tc2(const __grid_constant__ gemm_tc2::RowMaps map_x, const __grid_const
                 if (x.half == 0) break;
                 if (leader) mbar_arrive(&ctl->begun[i & 1]);
                 const int row = leader ? x.row_base[0] : x.row_base[1];
-                const int box = box_of(x.half);
+                const int box = kGather ? 0 : box_of(x.half);
                 const CUtensorMap* map = &map_x.box[box];
-                const uint32_t bytes = 2u * (uint32_t)(W_BYTES + box_rows(box) * 128);
+                const uint32_t bytes = 2u * (uint32_t)(W_BYTES + (kGather ? x.half : box_rows(box)) * 128);
                 bool ok = true;
                 for (int kb = 0; kb < KS; ++kb, ++it) {
                     const int s = it % kSlices;
@@ -344,7 +351,8 @@ ffn_gemm_tc2(const __grid_constant__ gemm_tc2::RowMaps map_x, const __grid_const
                     }
                     // the leader announces the bytes of both blocks on its own barrier
                     if (leader) mbar_expect_tx(&ctl->full[s], bytes);
-                    tma_load_2d_pair(tiles + s * SLICE_BYTES + W_BYTES, map, kb * BKE, row, map_to_cta(smem_u32(&ctl->full[s]), 0));
+                    if (!kGather)
+                        tma_load_2d_pair(tiles + s * SLICE_BYTES + W_BYTES, map, kb * BKE, row, map_to_cta(smem_u32(&ctl->full[s]), 0));
                 }
                 if (!ok) break;
             }
@@ -485,6 +493,32 @@ ffn_gemm_tc2(const __grid_constant__ gemm_tc2::RowMaps map_x, const __grid_const
             }
         }
         __syncwarp();
+    } else if (kGather && warp >= 4 + kBackWarps) {
+        // ------------------------------------------------------------ token rows by index (both blocks)
+        // A lane per four rows; warp 0 of the leader announces the bytes.
+        asm volatile("fence.proxy.async;" ::: "memory");
+        uint32_t it = 0;
+        long long w_unused = 0;
+        for (uint32_t i = 0;; ++i) {
+            const Task x = take(i, KLEOS_AT_GEMM_PRODUCER);
+            if (!__all_sync(0xffffffffu, x.half != 0)) break;
+            const int per = (x.half / 4 + kGatherWarps - 1) / kGatherWarps, at = 4 * ((warp - 4 - kBackWarps) * per + lane);
+            const bool mine = lane < per && at < x.half;
+            const int row = (leader ? x.row_base[0] : x.row_base[1]) + at;
+            int4 rows = make_int4(0, 0, 0, 0);
+            if (mine) rows = __ldg(reinterpret_cast<const int4*>(g.row_token + row));  // (past the last row: some earlier forward's tokens)
+            bool ok = true;
+            for (int kb = 0; kb < KS; ++kb, ++it) {
+                const int s = it % kSlices;
+                ok = mbar_wait_timed(&ctl->empty[s], ((it / kSlices) & 1) ^ 1, g.wait_cycles, abort_flag, &w_unused);
+                if (!__all_sync(0xffffffffu, ok)) break;  // the first producer reports the failure
+                if (mine)
+                    tma_gather4_pair(tiles + s * SLICE_BYTES + W_BYTES + at * 128, &map_x.box[0], kb * BKE, rows,
+                                     map_to_cta(smem_u32(&ctl->full[s]), 0));
+                __syncwarp();
+            }
+            if (!__all_sync(0xffffffffu, ok)) break;
+        }
     } else if (warp >= 4) {
         // ------------------------------------------------------------ read-back (both blocks)
         // Tensor-memory lane = output column, column = token row.  Group 0 takes the first 16 columns of

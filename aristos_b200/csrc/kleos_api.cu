@@ -70,6 +70,7 @@ struct State {
     // only move inside this GPU's memory, with no flags to raise or to wait for (KLEOS_DISPATCH_KERNELS=1:
     // the dispatch and plan kernels of several ranks instead)
     bool local = false;
+    bool gather = false;                     // GEMM1 fetches the token rows from the activations by index
     bool split_route = false;                // the router is route_split_kernel (KLEOS_ROUTE_KERNELS=1: the kernels of route.cuh)
     int route_parts = 1;                     // ... blocks per 128 tokens: parts of K whose logits are summed apart
     int route_grid = 0;                      // ... its blocks, no more than the device holds at once
@@ -112,7 +113,7 @@ struct State {
     // map_w1 / map_w2: weight tiles of the float GEMM; map_w1h / map_w2h: the 128 weight rows each block of
     // a pair loads (16-bit and TF32 GEMMs), rows_x / rows_y1: the token rows beside them
     CUtensorMap map_x{}, map_w1{}, map_y1{}, map_w2{}, map_act{}, map_wg{}, map_w1h{}, map_w2h{}, map_wgh{};
-    gemm_tc2::RowMaps rows_x{}, rows_y1{};
+    gemm_tc2::RowMaps rows_x{}, rows_y1{}, rows_act{};
 
     // pipelined host-buffer path (kleos_forward_host_async): double-buffered staging of the
     // activations and of the layer output, one stream per direction
@@ -122,7 +123,7 @@ struct State {
         char* act[2] = {};
         char* res[2] = {};
         CUtensorMap map_act[2] = {};
-        gemm_tc2::RowMaps rows[2] = {};  // the dense layer's GEMM1 reads the staged activations
+        gemm_tc2::RowMaps rows[2] = {};  // GEMM1 of the dense layer and of layers that gather reads the staged activations
         cudaEvent_t in_done[2] = {}, comp_done[2] = {}, out_done[2] = {};
         unsigned long long step = 0;
     } hp;
@@ -328,6 +329,7 @@ int ensure_maps(const Sections& s) {
     }
     if ((rc = make_row_maps(&g.rows_x, g.dense ? s.A : g.arena + g.lay.xcell, cell_rows, c.H))) return rc;
     if ((rc = make_row_maps(&g.rows_y1, g.y1, cell_rows, c.I))) return rc;
+    if (g.gather && (rc = make_map(&g.rows_act.box[0], s.A, c.S, c.H, 1, 128 / (uint32_t)c.elem_bytes))) return rc;
     if (g.use_tf32_tc) {
         const uint32_t bk = 32;  // 128 bytes
         if ((rc = make_map(&g.map_w1h, s.W1, (uint64_t)g.nLx * c.I, c.H, gemm_tc2::BM, bk))) return rc;
@@ -444,9 +446,9 @@ int launch_route(const RouteArgs& ra, cudaStream_t st, bool prepare = false) {
     return fail(KLEOS_E_UNSUPPORTED, "more than 256 experts are not supported by the router");
 }
 
-template <typename TE, int kEpi>
+template <typename TE, int kEpi, bool kGather = false>
 void launch_tc2(cudaStream_t st, const gemm_tc2::RowMaps& map_x, const CUtensorMap& map_w, const GemmArgs& ga) {
-    launch(ffn_gemm_tc2<TE, kEpi>, g.sm_count & ~1, gemm_tc2::kThreads, gemm_tc2::SMEM_BYTES, st, map_x, map_w, ga);
+    launch(ffn_gemm_tc2<TE, kEpi, kGather>, g.sm_count & ~1, gemm_tc2::kBlock<kGather>, gemm_tc2::SMEM_BYTES, st, map_x, map_w, ga);
 }
 
 // The persistent kernel, instantiated per activation and per compile-time top-k of the combine.
@@ -483,7 +485,7 @@ struct Staging {
     const char* A;
     char* out;
     const CUtensorMap* map_act;
-    const gemm_tc2::RowMaps* rows;  // dense 16-bit and TF32 layers
+    const gemm_tc2::RowMaps* rows;  // 16-bit and TF32 layers: dense ones, and those that gather
 };
 
 // num_experts == 1: out = (act(A W1^T + b1)) W2^T + b2 over this rank's S tokens, both GEMMs by
@@ -572,9 +574,9 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     pl.topk = g.topk; pl.A = s.A; pl.slots = g.slots; pl.cell_tokens = g.cell_tokens; pl.counts = g.counts;
     pl.hist = g.place_hist; pl.peers = g.peers; pl.cflag = g.lay.cflag; pl.row_chunks = (unsigned)((size_t)c.H * c.elem_bytes / 16);
     pl.status = g.status; pl.wait_cycles = g.wait_cycles; pl.S = c.S; pl.K = c.K; pl.E = c.E; pl.PX = c.PX; pl.EC = c.EC;
-    pl.pEC = c.pEC; pl.nLx = g.nLx; pl.rank = g.rank; pl.world = g.world; pl.epoch = g.epoch;
+    pl.pEC = c.pEC; pl.nLx = g.nLx; pl.rank = g.rank; pl.epoch = g.epoch; pl.publish = !g.local;
     if (g.local) {
-        pl.xcell = g.arena + g.lay.xcell;
+        if (!g.gather) pl.xcell = g.arena + g.lay.xcell;
         if (!g.use_tc && !g.use_tf32_tc) { pl.panels = g.panels; pl.le_start = g.le_start; }
     }
     if (split) {
@@ -675,6 +677,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     ga.ret.suppress = g.suppress_return_flag ? 1 : 0;
     ga.contiguous = g.world == 1; ga.next_tile = g.tile_claims; ga.counts = g.counts; ga.EC = c.EC;
     GemmArgs g1 = ga;
+    g1.row_token = g.cell_tokens;
     g1.A = g.arena + g.lay.xcell; g1.B = s.W1; g1.bias = s.b1; g1.N = c.I; g1.Kd = c.H; g1.mode = 0;
     GemmArgs g2 = ga;
     g2.next_tile = g.tile_claims + 2; g2.plan_ready = 1;
@@ -685,10 +688,11 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     }
     if (g.use_tc || g.use_tf32_tc) {
         if constexpr (!std::is_same<T, float>::value) {
-            if (c.hidden_act == 0)
-                launch_tc2<T, 0>(st, g.rows_x, g.map_w1h, g1);
-            else
-                launch_tc2<T, 1>(st, g.rows_x, g.map_w1h, g1);
+            const gemm_tc2::RowMaps& rows = !g.gather ? g.rows_x : stg ? *stg->rows : g.rows_act;
+            if (g.gather && c.hidden_act == 0) launch_tc2<T, 0, true>(st, rows, g.map_w1h, g1);
+            else if (g.gather) launch_tc2<T, 1, true>(st, rows, g.map_w1h, g1);
+            else if (c.hidden_act == 0) launch_tc2<T, 0>(st, rows, g.map_w1h, g1);
+            else launch_tc2<T, 1>(st, rows, g.map_w1h, g1);
             KLEOS_CUDA(mark());
             launch_tc2<T, 2>(st, g.rows_y1, g.map_w2h, g2);
             KLEOS_CUDA(mark());
@@ -748,9 +752,11 @@ int sync_last_forward() {
 template <typename TE>
 int set_gemm_attributes() {
     const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 0>, dyn, gemm_tc2::SMEM_BYTES));
-    KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 1>, dyn, gemm_tc2::SMEM_BYTES));
-    KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 2>, dyn, gemm_tc2::SMEM_BYTES));
+    KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 0, false>, dyn, gemm_tc2::SMEM_BYTES));
+    KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 1, false>, dyn, gemm_tc2::SMEM_BYTES));
+    KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 2, false>, dyn, gemm_tc2::SMEM_BYTES));
+    KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 0, true>, dyn, gemm_tc2::SMEM_BYTES));
+    KLEOS_CUDA(cudaFuncSetAttribute(ffn_gemm_tc2<TE, 1, true>, dyn, gemm_tc2::SMEM_BYTES));
     return KLEOS_OK;
 }
 
@@ -804,6 +810,10 @@ int ensure_host_pipe() {
         }
         if (g.dense && (g.use_tc || g.use_tf32_tc)) {
             int rc = make_row_maps(&hp.rows[b], hp.act[b], c.S, c.H);
+            if (rc) return rc;
+        }
+        if (g.gather) {
+            int rc = make_map(&hp.rows[b].box[0], hp.act[b], c.S, c.H, 1, 128 / (uint32_t)c.elem_bytes);
             if (rc) return rc;
         }
     }
@@ -1042,6 +1052,10 @@ static int initialize_impl(const char* config_json_path, int rank, int world, co
                  g.nLx <= flow::kMaxLocal;
     const char* dk = std::getenv("KLEOS_DISPATCH_KERNELS");
     g.local = world == 1 && !g.use_flow && !(dk && dk[0] == '1');
+    // The rows are fetched by index where the weights' way from HBM hides it (see ffn_gemm_tc2): up to 256 rows
+    // an expert on average.  KLEOS_GATHER=0 copies them to the cells there too.
+    const char* gt = std::getenv("KLEOS_GATHER");
+    g.gather = g.local && g.split_route && (long long)cfg.S * cfg.K <= 256LL * cfg.E && !(gt && gt[0] == '0');
     const char* fr = std::getenv("KLEOS_FUSE_ROUTE");
     g.fuse_route = g.use_flow && cfg.PX <= 128 && !cfg.is_training && !(fr && fr[0] == '0');
     if (g.use_flow) {

@@ -407,11 +407,12 @@ struct PlaceArgs {
     // of the epoch in a word, so that a reader knows from the word itself that it is this forward's.  (A count
     // reaches 128 * k = 1024: a token of NaN logits chooses expert 0 k times.)
     unsigned long long* hist;
-    // several ranks: count flags, cflag[owner][rank*nLx + le] = (epoch<<32)|routed, one 8-byte peer store
+    // publish: count flags, cflag[owner][rank*nLx + le] = (epoch<<32)|routed, one 8-byte peer store
     // per expert (the reference's first-stage signal carries the same count, types.cuh:300-317)
     PeerTable peers;
     size_t cflag;
-    // one rank: the token rows go to this rank's own cells [E][pEC][H] (else null)
+    int publish;
+    // one rank, GEMMs that read the cells: the token rows go to this rank's own cells [E][pEC][H] (else null)
     char* xcell;
     unsigned row_chunks;    // 16-byte chunks of a token row
     // one rank, GEMMs that work through a panel list: the last block writes it (else null)
@@ -419,7 +420,7 @@ struct PlaceArgs {
     int* le_start;
     DeviceStatus* status;
     long long wait_cycles;
-    int S, K, E, PX, EC, pEC, nLx, rank, world;
+    int S, K, E, PX, EC, pEC, nLx, rank;
     uint32_t epoch;
 };
 
@@ -527,7 +528,7 @@ __device__ __forceinline__ void place_tokens(const PlaceArgs& a, int row, int n_
             const int total = s->total[e];
             a.counts[e] = (unsigned)total;
             s->total[e] = min(total, a.EC);
-            if (a.world > 1 || a.xcell == nullptr) {
+            if (a.publish) {
                 const int owner = e / a.nLx, le = e - owner * a.nLx;
                 st_release_sys(reinterpret_cast<unsigned long long*>(a.peers.arena[owner] + a.cflag) + ((size_t)a.rank * a.nLx + le),
                                make_flag(a.epoch, (unsigned)min(total, a.EC)));

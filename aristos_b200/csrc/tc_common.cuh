@@ -256,6 +256,15 @@ __device__ __forceinline__ void tma_load_2d_pair_hint(void* smem_dst, const CUte
         "r"(bar_cluster), "l"(policy)
         : "memory");
 }
+// Four rows of a matrix, one after the other in shared memory (the map's box is one row high)
+__device__ __forceinline__ void tma_gather4_pair(void* smem_dst, const CUtensorMap* map, int x, int4 rows, uint32_t bar_cluster) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes.cta_group::2 "
+        "[%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+        ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(rows.x), "r"(rows.y), "r"(rows.z),
+        "r"(rows.w), "r"(bar_cluster)
+        : "memory");
+}
 __device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
                                                uint32_t idesc, uint32_t accumulate) {
     asm volatile(

@@ -113,6 +113,13 @@ static_assert(kBarriers <= kThreads, "a thread per barrier");
 __device__ __forceinline__ int row_splits(int rows) {
     return rows <= kMaxRows ? (rows + kMaxRows - 1) / kMaxRows : (rows + 255) / 256;
 }
+// A dense layer is one expert, so its tiles are all alike and take whole rounds over the block pairs: as many
+// (and as small) ones as fit the same number of rounds.  (Of several experts' tiles a pair that is done
+// early takes another.)
+__device__ __forceinline__ int dense_splits(int rows, int column_tiles, int pairs) {
+    const int least = row_splits(rows), rounds = (least * column_tiles + pairs - 1) / pairs;
+    return max(least, min(rounds * pairs / column_tiles, (rows + 31) >> 5));
+}
 
 // Tiles in order of local expert, column tile, rows: tiles that run together read the same weights.
 // `le` is the caller's place in the list (its tiles only grow).
@@ -126,11 +133,12 @@ __device__ __forceinline__ Task decode_task(int t, const Control* ctl, const Gem
     x.mt = r / splits;
     const int j = r - x.mt * splits;
     if (g.contiguous) {
-        const int rows = ctl->rows[e];
-        const int per = ((rows + splits - 1) / splits + 31) >> 5 << 5;
-        const int left = min(per, rows - j * per);
-        x.half = ((left + 31) >> 5) << 4;
-        x.row_base[0] = e * g.pEC + j * per;
+        // 32 rows are the unit, and the tiles of an expert differ by one at most
+        const int rows = ctl->rows[e], units = (rows + 31) >> 5, share = units / splits, more = units - share * splits;
+        const int at = j * share + min(j, more), n = share + (j < more ? 1 : 0);
+        const int left = min(32 * n, rows - 32 * at);
+        x.half = 16 * n;
+        x.row_base[0] = e * g.pEC + 32 * at;
         x.rows[0] = min(x.half, left);
         x.row_base[1] = x.row_base[0] + x.half;
         x.rows[1] = left - x.rows[0];
@@ -269,7 +277,7 @@ ffn_gemm_tc2(const __grid_constant__ gemm_tc2::RowMaps map_x, const __grid_const
         const bool in = e >= g.le_begin && e < g.le_end;
         if (g.contiguous) {
             ctl->rows[e] = !in ? 0 : g.counts ? (int)min(g.counts[e], (unsigned)g.EC) : g.pEC;
-            ctl->splits[e] = row_splits(ctl->rows[e]);
+            ctl->splits[e] = g.counts ? row_splits(ctl->rows[e]) : dense_splits(ctl->rows[e], MT, (int)gridDim.x >> 1);
         } else {
             ctl->splits[e] = in ? (g.le_start[e + 1] - g.le_start[e] + 1) >> 1 : 0;
         }

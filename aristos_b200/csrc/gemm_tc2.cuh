@@ -3,9 +3,12 @@
 // 288 rows of one local expert.  M is fixed at 256 by the instruction and an FFN has hundreds or
 // thousands of columns; the rows an expert gets are any number, and N takes any multiple of 32.  So
 // the work done for padding is below 32 rows of an expert, and an expert's weights are read once for
-// every 288 of its rows.  (With the rows on M, 128 a block, a layer of 256 rows an expert on average
-// multiplied 1.5 times what it had to: every second expert has some rows above 256, and they took a
-// tile of their own.)
+// every 256 or 288 of its rows.  With the rows on M, 128 a block, every tile cost as much as one of 256 rows.
+// What bounds it: the weight stream from HBM up to about 256 rows an expert (128 tokens, 64 experts,
+// H = I = 2048: 537 MB of weights in 85 us = 6.3 TB/s, where plain loads reach 6.2; before 106 and 115 us
+// a launch), above that the tensor pipe, in steady state at the clock the power limit leaves (4096 tokens,
+// H = 4096, I = 14336, 8 experts: 614 us = 1.57 PFLOP/s alone, both GEMMs and the rest 1538 us one after the
+// other, before 1565).  16384 tokens on 128 experts of Zipf popularity: 135 + 143 us -> 103 + 112.
 //
 // Tile = (local expert, 256 columns, up to 288 rows).  Each block TMA-loads 128 weight rows (A) and half
 // of the token rows (B), 64 wide K slices through a ring of six.  Accumulators are a ring in
@@ -18,13 +21,15 @@
 // ring in shared memory: their sizes differ by up to nine times, so no fixed split is even.
 //
 // Per block, 384 threads:
-//   warp 0      TMA producer of the token rows (one lane); in the leader it also claims the tiles
+//   warp 0      TMA producer of the token rows (one lane)
 //   warp 1      leader only: issues tcgen05.mma.cta_group::2, commits to `empty` and
 //               `acc_full` of BOTH blocks
-//   warp 2      tensor-memory allocation / release (both blocks, cta_group::2 forms)
+//   warp 2      tensor-memory allocation / release (both blocks, cta_group::2 forms); in the leader
+//               also the scheduler, which claims the tiles
 //   warp 3      TMA producer of the weight rows (one lane)
 //   warps 4..11 read-back of the block's 128 columns of all the tile's rows: two groups of four warps,
 //               16 rows at a time in turn; arrive on the LEADER's `slot_empty`
+//   warps 12..15  gathering form only: token rows by index
 // Work and epilogue semantics follow the reference's tile worker (os/processor/processor.cuh:
 // 350-489,706-741).  Every wait is bounded.  This kernel runs one GEMM over a finished panel
 // list (the dense single-expert layer, and the routed layer when its phases are launched one

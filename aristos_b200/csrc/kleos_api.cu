@@ -66,9 +66,9 @@ struct State {
     // as ONE persistent kernel (moe_flow.cuh) instead of separate launches.
     bool use_flow = false;
     bool fuse_route = false;                 // ... and the router runs inside it too (KLEOS_FUSE_ROUTE=0: separate launches)
-    // One rank, separate launches: it owns every expert, so the router writes the panel list and the rows
-    // only move inside this GPU's memory, with no flags to raise or to wait for (KLEOS_DISPATCH_KERNELS=1:
-    // the dispatch and plan kernels of several ranks instead)
+    // One rank, separate launches: it owns every expert, so the rows only move inside this GPU's memory, with
+    // no plan, and no flags to raise or to wait for (KLEOS_DISPATCH_KERNELS=1: the dispatch and plan
+    // kernels of several ranks instead)
     bool local = false;
     bool gather = false;                     // GEMM1 fetches the token rows from the activations by index
     bool split_route = false;                // the router is route_split_kernel (KLEOS_ROUTE_KERNELS=1: the kernels of route.cuh)
@@ -389,7 +389,9 @@ int with_route_split(F f) {
     return top2 ? f(route_split_kernel<T, 128, 2>, route_split::Shape<128>::SMEM_BYTES) : f(route_split_kernel<T, 128, 0>, route_split::Shape<128>::SMEM_BYTES);
 }
 
-// Expert weights that the router brings into L2 (126 MB, which also holds the layer's rows).
+// Expert weights that the router brings into L2 (126 MB, which also holds the layer's rows): 64 MB are ten
+// microseconds of HBM.  GEMM1 of a decode step of 128 tokens, 64 experts, took 102 us without and 88 with.
+// Every block of the chip issues its share: left to the four with tokens it took the router 98 us.
 constexpr size_t kAheadBytes = (size_t)64 << 20;
 
 // How the router's work is spread: as many blocks per 128 tokens (1, 2 or 4 in a cluster) as find room

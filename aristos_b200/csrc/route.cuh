@@ -562,7 +562,9 @@ __device__ __forceinline__ void place_tokens(const PlaceArgs& a, int row, int n_
 }
 
 // The same on its own, behind the routers whose blocks do not have 512 threads or whose choices the near-tie
-// kernel may change: one block per 32 tokens.  It stands for three kernels (histogram, slots, rows).
+// kernel may change: one block per 32 tokens.  Blocks wait for lower ones, which are placed on the chip first.
+// It stands for three kernels (histogram 2.8 us, slots 5.9, rows 3.9 at 256 tokens, 8 float experts, where the
+// forward went from 97.5 to 85 with the return flags gone too).
 constexpr int kPlaceOwn = 32;
 __global__ void __launch_bounds__(kPlaceThreads) place_kernel(PlaceArgs a) {
     __shared__ PlaceScratch s;

@@ -1,5 +1,5 @@
 // Router of 16-bit and TF32 layers of up to 128 experts in ONE launch: gate GEMM on the tensor cores,
-// softmax, top-k, near-tie re-evaluation, slots, counts and, on one rank, the panel list.
+// softmax, top-k, near-tie re-evaluation, slots, counts and, on one rank, the rows' way into the cells.
 //
 // What bounds it is latency: the bytes and multiply-adds take 5 us at most on the largest layers and
 // next to nothing on the others, while one block that walks all of K, then thread by thread
@@ -9,8 +9,11 @@
 //     distributed shared memory, one bulk copy per pair of blocks (16-byte stores from tensor memory to
 //     the other block took 4 us): block r gets all parts of the tokens [r, r + 1) * 128 / C and adds
 //     them in order of K;
-//   * four threads per token, each with a quarter of the experts in registers, do softmax and top-k;
+//   * four threads per token, each with a quarter of the experts, do softmax and top-k;
 //   * slots without a grid barrier: place_tokens(), route.cuh.
+// Measured, router and row copy, alone and cold: 256 tokens, 8 experts 28 us -> 15; 8192 tokens, 64 experts
+// 54 -> 43 (29 where GEMM1 gathers the rows); 16384 tokens, 128 experts 67 -> 61 (45); of the 128 tokens of a
+// decode step, 64 experts, 39 -> 25 with 64 MB of weights brought into L2 meanwhile.
 // A block only waits for blocks of lower index and for its own cluster; the host launches no more
 // clusters than the device holds at once.
 //

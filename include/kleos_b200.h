@@ -188,8 +188,7 @@ long long kleos_launch_count(void);
 /* Stall counters of the last GEMM1 and GEMM2 launches, only when the environment variable
  * KLEOS_GEMM_STATS=1 was set at initialise time: [2][blocks][12] clock cycles per block
  * {producer wait-empty, producer total, MMA wait-accumulator, MMA wait-operands, MMA total,
- *  epilogue wait-accumulator, epilogue total, epilogue TMEM wait, plan prologue, producer wait
- *  for cell data, dispatch finished at, unused}.  Returns the number of values written.
+ *  epilogue wait-accumulator, epilogue total, unused, prologue, unused, unused, unused}.  Returns the number of values written.
  * A tuning aid with no counterpart in the reference. */
 int kleos_debug_gemm_stats(long long* out, int max_values);
 

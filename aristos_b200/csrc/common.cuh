@@ -109,6 +109,17 @@ __device__ __forceinline__ float apply_act(float z, int hidden_act) {
     return 0.5f * z * (1.f + erff(z * 0.70710678118654752f));
 }
 
+// w[0] + .. + w[N - 1], halves onto halves: the order in which the routers add the winning probabilities
+template <int N>
+__device__ __forceinline__ float pair_sum(float (&w)[N]) {
+    static_assert((N & (N - 1)) == 0, "a power of two");
+#pragma unroll
+    for (int o = N / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int j = 0; j < o; ++j) w[j] += w[j + o];
+    return w[0];
+}
+
 // ---------------------------------------------------------------- system-scope flags
 // A flag word is (epoch << 32) | payload.  Writers store it with release semantics after
 // their data stores; readers poll with acquire semantics.  Epochs only grow, so flags never

@@ -684,22 +684,25 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 // sum of the exponentials by quarters of the PX experts, then (q0 + q1) + (q2 + q3): the order
                 // in which the four threads per token of route_split.cuh add them
                 float quarter[4] = {0.f, 0.f, 0.f, 0.f};
+                auto four = [&](int c, int jj, const uint32_t* v) {
+                    float x[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int e = c * 32 + jj + k;
+                        x[k] = e < a.E ? __expf(__uint_as_float(v[jj + k]) + bias_r[e] - m) : 0.f;
+                    }
+                    return (x[0] + x[1]) + (x[2] + x[3]);
+                };
 #pragma unroll 1
                 for (int c = 0; c < chunks; ++c) {
                     uint32_t v[32];
                     load_logits(c, v);
                     float lo = 0.f, hi = 0.f;  // a chunk of 32 is a quarter (PX = 128) or two (PX = 64)
 #pragma unroll
-                    for (int jj = 0; jj < 16; ++jj) {
-                        const int e = c * 32 + jj;
-                        if (e < a.E) lo += __expf(__uint_as_float(v[jj]) + bias_r[e] - m);
-                    }
+                    for (int jj = 0; jj < 16; jj += 4) lo += four(c, jj, v);
                     if (chunks > 2) hi = lo;
 #pragma unroll
-                    for (int jj = 16; jj < 32; ++jj) {
-                        const int e = c * 32 + jj;
-                        if (e < a.E) hi += __expf(__uint_as_float(v[jj]) + bias_r[e] - m);
-                    }
+                    for (int jj = 16; jj < 32; jj += 4) hi += four(c, jj, v);
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
                         if (chunks > 2 ? k == c : k == 2 * c + 1) quarter[k] = hi;
@@ -781,10 +784,10 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     }
                     __syncwarp();
                 }
-                float wsum = 0.f;
+                float w[KC];
 #pragma unroll
-                for (int j = 0; j < KC; ++j)
-                    if (j < K) wsum = fmaf(__expf(val[j] - m), inv, wsum);
+                for (int j = 0; j < KC; ++j) w[j] = j < K ? __fmul_rn(__expf(val[j] - m), inv) : 0.f;
+                const float wsum = pair_sum(w);
                 // probabilities, padding columns zero, one 16-byte store per eight experts
 #pragma unroll 1
                 for (int c = 0; c < chunks; ++c) {

@@ -415,26 +415,24 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 v.y = e0 + 1 < E ? __expf(v.y - m) : 0.f;
                 v.z = e0 + 2 < E ? __expf(v.z - m) : 0.f;
                 v.w = e0 + 3 < E ? __expf(v.w - m) : 0.f;
-                d += v.x;
-                d += v.y;
-                d += v.z;
-                d += v.w;
+                d += (v.x + v.y) + (v.z + v.w);
                 *reinterpret_cast<float4*>(l + i) = v;
             }
             d += __shfl_xor_sync(0xffffffffu, d, 1);
             d += __shfl_xor_sync(0xffffffffu, d, 2);
             const float inv = 1.f / d;
             if (sub == 0 && t < S && !*abort_flag) {
-                float wsum = 0.f;
+                float w[KC];
+#pragma unroll
+                for (int j = 0; j < KC; ++j) w[j] = j < K ? __fmul_rn(__expf(scr->sel_v[tok][j] - m), inv) : 0.f;
+                a.r.mcw[t] = pair_sum(w);
 #pragma unroll 1
                 for (int j = 0; j < K; ++j) {
-                    wsum = fmaf(__expf(scr->sel_v[tok][j] - m), inv, wsum);
                     const int e = scr->sel_i[tok][j];
                     a.r.topk[(size_t)t * K + j] = e;
                     ctl->top[tok * K + j] = e;
                     atomicAdd(&ctl->hist[e], 1);
                 }
-                a.r.mcw[t] = wsum;
             }
             // probabilities, padding columns zero
             TE* dst = static_cast<TE*>(a.r.probs) + (size_t)t * PXT + sub * PER;

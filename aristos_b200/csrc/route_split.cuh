@@ -52,11 +52,14 @@ struct Args {
     const char* ahead;         // expert weights to bring into L2 while the memory is idle, or null
     size_t ahead_bytes;        // ... a multiple of 16
     int parts;                 // blocks per cluster
-    int acc_slices;            // K slices that one accumulator sums before the next one takes over (0: all of a block's)
+    // kFine: K slices that one accumulator sums before the next one takes over.  When tensor memory is full of
+    // accumulators they are read, and the first ones start again.
+    int acc_slices;
 };
 
 struct Control {
-    unsigned long long full[8], empty[8], acc_full;
+    unsigned long long full[8], empty[8], acc_full;    // acc_full: once per filling of tensor memory
+    unsigned long long acc_read;                       // a filling's accumulators have been read, eight warps
     unsigned long long got;                            // the other blocks' parts of this block's logits have arrived
     uint32_t tmem_base;
     int abort;
@@ -150,8 +153,9 @@ __device__ __noinline__ void settle_near_ties(unsigned flagged, const float* log
 
 }  // namespace route_split
 
-// PXT: padded expert count; KT: compile-time top-k (0: read it from the arguments).
-template <typename TE, int PXT, int KT>
+// PXT: padded expert count; KT: compile-time top-k (0: read it from the arguments); kFine: Args::acc_slices
+// (a layer's router sums a block's slices in one accumulator: the code for more cost 256 tokens 0.6 of 30 us).
+template <typename TE, int PXT, int KT, bool kFine = false>
 __global__ void __launch_bounds__(route_split::kThreads, 1)
 route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_wg, route_split::Args a) {
     using namespace tc;
@@ -175,7 +179,7 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     const long long wait_cycles = a.place.wait_cycles;
     const uint32_t epoch = a.place.epoch;
     volatile int* abort_flag = &ctl->abort;
-    const uint32_t tmem_cols = a.acc_slices > 0 ? 512u : (uint32_t)PXT;
+    const uint32_t tmem_cols = kFine ? 512u : (uint32_t)PXT;
     uint32_t idesc;
     if constexpr (kWide) idesc = make_instr_desc_tf32(BM, PXT);
     else idesc = make_instr_desc_16b(BM, PXT, Pack2<TE>::kMmaFormat);
@@ -186,6 +190,7 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             mbar_init(&ctl->empty[s], 1);
         }
         mbar_init(&ctl->acc_full, 1);
+        mbar_init(&ctl->acc_read, 8);
         mbar_init(&ctl->got, 1);
         ctl->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -207,7 +212,9 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
     const int KS = H / BKE, kb0 = me * KS / C, kb1 = (me + 1) * KS / C;  // this block's part of K
     const int n_rt = (S + BM - 1) / BM, n_clusters = (int)gridDim.x / C, cluster_id = (int)blockIdx.x / C;
-    const int acc_slices = a.acc_slices > 0 ? a.acc_slices : KS, n_acc = (kb1 - kb0 + acc_slices - 1) / acc_slices;
+    const int acc_slices = kFine ? a.acc_slices : KS, n_acc = kFine ? (kb1 - kb0 + acc_slices - 1) / acc_slices : 1;
+    constexpr int kAccs = 512 / PXT, kSums = kFine ? PXT / 2 : 1;
+    const int fills = kFine ? (n_acc + kAccs - 1) / kAccs : 1;
     const uint32_t part_bytes = (uint32_t)own * LD * 4;
     const TE* A = static_cast<const TE*>(a.r.A);
     const TE* Wg = static_cast<const TE*>(a.r.Wg);
@@ -260,9 +267,19 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     tc_fence_after();
                     const uint32_t sa = smem_u32(tiles + s * Sh::STAGE_BYTES);
                     const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + W_BYTES);
-                    const int acc = (kb - kb0) / acc_slices;
+                    const int acc = kFine ? (kb - kb0) / acc_slices : 0;
                     const bool first = kb - kb0 == acc * acc_slices;
-                    const uint32_t d = tmem_base + (uint32_t)(acc * PXT);
+                    const uint32_t d = tmem_base + (uint32_t)(acc % kAccs * PXT);
+                    if (kFine && first && acc > 0 && acc % kAccs == 0) {
+                        umma_commit(&ctl->acc_full);
+                        if (!mbar_wait(&ctl->acc_read, (round * (fills - 1) + acc / kAccs - 1) & 1, wait_cycles, abort_flag)) {
+                            report_error(a.status, KLEOS_AT_GEMM_MMA, -300 - rt, (int)epoch);
+                            *abort_flag = 1;
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+                    }
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {  // four 32-byte steps per slice
                         if constexpr (kWide) umma_tf32(d, da + 2 * k, db + 2 * k, idesc, (!first || k != 0) ? 1u : 0u);
@@ -279,33 +296,57 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         // ---------------------------------------------------------- partial logits to the blocks that own the tokens
         if (warp >= 4 && warp < 12) {
             const int q = warp & 3, half = (warp - 4) >> 2;
-            const bool ok = mbar_wait(&ctl->acc_full, round & 1, wait_cycles, abort_flag);
-            if (!ok) {
-                if (lane == 0) report_error(a.status, KLEOS_AT_GEMM_EPILOGUE, -100 - rt, (int)epoch);
-                *abort_flag = 1;
-            }
-            tc_fence_after();
             const int row = q * 32 + lane, owner = row / own;
             // the rows of one owner lie one after the other on both sides
             float* dst = (owner == me ? recv + (size_t)me * own * LD : reinterpret_cast<float*>(tiles + kSendAt) + (size_t)owner * own * LD) +
                          (size_t)(row % own) * LD + half * (PXT / 2);
             const uint32_t taddr = tmem_base + half * (PXT / 2) + (static_cast<uint32_t>(q * 32) << 16);
-            if (__all_sync(0xffffffffu, ok)) {
+            float sum[kSums];  // of the fillings before the last
+#pragma unroll
+            for (int j = 0; j < kSums; ++j) sum[j] = 0.f;
+            bool ok = true;
 #pragma unroll 1
+            for (int f = 0; f < fills; ++f) {
+                ok = mbar_wait(&ctl->acc_full, (round * fills + f) & 1, wait_cycles, abort_flag);
+                if (!ok) {
+                    if (lane == 0) report_error(a.status, KLEOS_AT_GEMM_EPILOGUE, -100 - rt, (int)epoch);
+                    *abort_flag = 1;
+                }
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tc_fence_after();
+                const int accs = min(kAccs, n_acc - f * kAccs);
+                // (the operand stages, where the rows on their way out go, are free after the last filling only)
+                const bool last = f + 1 == fills;
+#pragma unroll (kFine ? PXT / 32 : 1)
                 for (int c = 0; c < PXT / 2; c += 16) {
                     uint32_t v[16];
                     tmem_ld_32x16(taddr + c, v);
                     tmem_ld_wait();
 #pragma unroll 1
-                    for (int acc = 1; acc < n_acc; ++acc) {
+                    for (int acc = 1; acc < accs; ++acc) {
                         uint32_t w[16];
                         tmem_ld_32x16(taddr + acc * PXT + c, w);
                         tmem_ld_wait();
 #pragma unroll
                         for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
                     }
+                    if (kSums > 1) {
 #pragma unroll
-                    for (int j = 0; j < 16; j += 4) *reinterpret_cast<uint4*>(dst + c + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                        for (int j = 0; j < 16; ++j) {
+                            sum[(c + j) % kSums] += __uint_as_float(v[j]);
+                            v[j] = __float_as_uint(sum[(c + j) % kSums]);
+                        }
+                    }
+                    if (last) {
+#pragma unroll
+                        for (int j = 0; j < 16; j += 4) *reinterpret_cast<uint4*>(dst + c + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                    }
+                }
+                if (!last) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&ctl->acc_read);
                 }
             }
             tc_fence_before();

@@ -75,8 +75,8 @@ extern "C" int kleos_route_static(const void* A, const void* Wg, const float* ga
         cudaError_t e = cudaGetSymbolAddress(&p, g_route_scratch);
         const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
         if (e == cudaSuccess) e = cudaFuncSetAttribute(route_kernel<float, 64>, dyn, route_fma::smem_bytes<float, 64>());
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(route_split_kernel<__nv_bfloat16, 64, 2>, dyn, route_split::Shape<64>::SMEM_BYTES);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(route_split_kernel<__nv_bfloat16, 64, 0>, dyn, route_split::Shape<64>::SMEM_BYTES);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(route_split_kernel<__nv_bfloat16, 64, 2, true>, dyn, route_split::Shape<64>::SMEM_BYTES);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(route_split_kernel<__nv_bfloat16, 64, 0, true>, dyn, route_split::Shape<64>::SMEM_BYTES);
         if (e != cudaSuccess || !p) {
             std::fprintf(stderr, "[kleos_b200] setting up kleos_route_static failed: %s\n",
                          cudaGetErrorString(e));
@@ -114,8 +114,8 @@ extern "C" int kleos_route_static(const void* A, const void* Wg, const float* ga
         refine_kernel<float><<<148, 256, 0, st>>>(ra);
     } else {
         // bf16 goes to the tensor cores (route_split.cuh): four blocks per 128 tokens, or as many as there
-        // are 64-wide slices of K.  mCw is a 32-bit result, so the running sums stay short: eight accumulators
-        // a block, added up in fp32 registers, each over an eighth of the block's slices.
+        // are 64-wide slices of K.  mCw is a 32-bit result, so the running sums stay short: an accumulator per
+        // slice, added up in fp32 registers eight at a time.
         CUtensorMap map_a, map_wg;
         const char* err = encode_map(&map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, (uint64_t)S, (uint64_t)H, route_split::BM, 64);
         if (!err) err = encode_map(&map_wg, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, Wg, 64, (uint64_t)H, 64, 64);
@@ -126,7 +126,7 @@ extern "C" int kleos_route_static(const void* A, const void* Wg, const float* ga
         sp.place.wait_cycles = 20000000000LL;
         const int slices = H / 64;
         sp.parts = slices >= 4 ? 4 : slices >= 2 ? 2 : 1;
-        sp.acc_slices = ((slices + sp.parts - 1) / sp.parts + 7) / 8;
+        sp.acc_slices = 1;
         cudaLaunchConfig_t lc{};
         lc.gridDim = dim3((unsigned)((S + route_split::BM - 1) / route_split::BM * sp.parts));
         lc.blockDim = dim3(route_split::kThreads);
@@ -138,8 +138,8 @@ extern "C" int kleos_route_static(const void* A, const void* Wg, const float* ga
         at.val.clusterDim.y = at.val.clusterDim.z = 1;
         lc.attrs = &at;
         lc.numAttrs = 1;
-        if (K == 2) cudaLaunchKernelEx(&lc, route_split_kernel<__nv_bfloat16, 64, 2>, map_a, map_wg, sp);
-        else cudaLaunchKernelEx(&lc, route_split_kernel<__nv_bfloat16, 64, 0>, map_a, map_wg, sp);
+        if (K == 2) cudaLaunchKernelEx(&lc, route_split_kernel<__nv_bfloat16, 64, 2, true>, map_a, map_wg, sp);
+        else cudaLaunchKernelEx(&lc, route_split_kernel<__nv_bfloat16, 64, 0, true>, map_a, map_wg, sp);
     }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {

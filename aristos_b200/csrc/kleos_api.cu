@@ -75,6 +75,7 @@ struct State {
     int route_parts = 1;                     // ... blocks per 128 tokens: parts of K whose logits are summed apart
     int route_grid = 0;                      // ... its blocks, no more than the device holds at once
     unsigned long long* place_hist = nullptr;  // see PlaceArgs
+    unsigned* place_launch = nullptr;          // ...
     int flow_grid = 0;                       // blocks of the persistent kernel (co-resident pairs x 2)
     flow::Counters* flow_ctr = nullptr;      // [2] scheduler state, see moe_flow.cuh
     long long* flow_stamps = nullptr;        // [flow_grid][kStampSlots] timeline of a timed forward
@@ -574,7 +575,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     int route_blocks = (c.S + route_fma::TM - 1) / route_fma::TM;
     PlaceArgs pl{};
     pl.topk = g.topk; pl.A = s.A; pl.slots = g.slots; pl.cell_tokens = g.cell_tokens; pl.counts = g.counts;
-    pl.hist = g.place_hist; pl.peers = g.peers; pl.cflag = g.lay.cflag; pl.row_chunks = (unsigned)((size_t)c.H * c.elem_bytes / 16);
+    pl.hist = g.place_hist; pl.launch = g.place_launch; pl.peers = g.peers; pl.cflag = g.lay.cflag; pl.row_chunks = (unsigned)((size_t)c.H * c.elem_bytes / 16);
     pl.status = g.status; pl.wait_cycles = g.wait_cycles; pl.S = c.S; pl.K = c.K; pl.E = c.E; pl.PX = c.PX; pl.EC = c.EC;
     pl.pEC = c.pEC; pl.nLx = g.nLx; pl.rank = g.rank; pl.epoch = g.epoch; pl.publish = !g.local;
     if (g.local) {
@@ -830,7 +831,7 @@ void release_all() {
     cudaFree(g.y1); cudaFree(g.topk); cudaFree(g.slots); cudaFree(g.cell_tokens);
     cudaFree(g.refine_list); cudaFree(g.refine_count); cudaFree(g.tile_hist); cudaFree(g.refine_done); cudaFree(g.refine_logits); cudaFree(g.le_start); cudaFree(g.mcw);
     cudaFree(g.bias); cudaFree(g.counts); cudaFree(g.done_dispatch); cudaFree(g.done_gemm2);
-    cudaFree(g.cell_counts); cudaFree(g.place_hist); cudaFree(g.flow_ctr); cudaFree(g.flow_stamps); cudaFree(g.flow_stalls); cudaFree(g.panels); cudaFree(g.tile_claims); cudaFree(g.status); cudaFree(g.gemm_stats);
+    cudaFree(g.cell_counts); cudaFree(g.place_hist); cudaFree(g.place_launch); cudaFree(g.flow_ctr); cudaFree(g.flow_stamps); cudaFree(g.flow_stalls); cudaFree(g.panels); cudaFree(g.tile_claims); cudaFree(g.status); cudaFree(g.gemm_stats);
     cudaFree(g.col_partial); cudaFree(g.gate_stats);
     for (auto& e : g.ev)
         if (e) cudaEventDestroy(e);
@@ -1027,6 +1028,7 @@ static int initialize_impl(const char* config_json_path, int rank, int world, co
         if (rc) return rc;
     }
     if (!dense && (rc = dev_alloc(&g.place_hist, (size_t)((cfg.S + kPlaceOwn - 1) / kPlaceOwn) * place_words(cfg.PX)))) return rc;
+    if (!dense && (rc = dev_alloc(&g.place_launch, 2))) return rc;
     if (g.use_tc) {
         if (cfg.torch_dtype == 2) rc = set_tc_attributes<__nv_bfloat16>();
         else rc = set_tc_attributes<__half>();

@@ -403,10 +403,13 @@ struct PlaceArgs {
     int* slots;             // [S,K] slot or kDropped
     int* cell_tokens;       // [E,pEC] token id held by each slot
     unsigned* counts;       // [E] unclamped
-    // [rows][place_words(PX)]: every block's histogram of chosen experts, four counts of 12 bits and 16 bits
-    // of the epoch in a word, so that a reader knows from the word itself that it is this forward's.  (A count
+    // [rows][place_words(PX)]: every block's histogram of chosen experts, four counts of 12 bits and a tag of 16 bits
+    // in a word, so that a reader knows from the word itself that it is this launch's.  (A count
     // reaches 128 * k = 1024: a token of NaN logits chooses expert 0 k times.)
     unsigned long long* hist;
+    // {launches so far, rows placed by this one}: the tag comes from here and not from the epoch, which is an
+    // argument and the same in every replay of a captured forward
+    unsigned* launch;
     // publish: count flags, cflag[owner][rank*nLx + le] = (epoch<<32)|routed, one 8-byte peer store
     // per expert (the reference's first-stage signal carries the same count, types.cuh:300-317)
     PeerTable peers;
@@ -433,6 +436,11 @@ struct PlaceScratch {
     int base[kPlaceMaxE], total[kPlaceMaxE], off[kPlaceMaxE + 1];
 };
 
+__device__ __forceinline__ unsigned ld_relaxed_u32(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
     unsigned long long v;
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
@@ -443,15 +451,19 @@ __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long
 // on, row `row` of n_rows: 512 threads, all of them.  top[own * K] and hist[PX] are the chosen experts and
 // their histogram, in shared memory.  The block publishes its histogram and adds up those of the rows
 // before it as they come, without a fence, a flag or a grid barrier: it only waits for blocks of lower
-// index.  A wait that runs out raises *abort_flag.
-__device__ __forceinline__ void place_tokens(const PlaceArgs& a, int row, int n_rows, int tok0, int own, int* top, const int* hist,
-                                             PlaceScratch* s, volatile int* abort_flag, DeviceStatus* status) {
+// index.  A wait that runs out raises *abort_flag.  `launch`: PlaceArgs::launch[0], read before.
+__device__ __forceinline__ void place_tokens(const PlaceArgs& a, unsigned launch, int row, int n_rows, int tok0, int own, int* top,
+                                             const int* hist, PlaceScratch* s, volatile int* abort_flag, DeviceStatus* status) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, K = a.K, E = a.E, words = place_words(a.PX);
+    const uint32_t tag = (launch + 1) & 0xffffu;  // (the words are zero at first)
     if (tid < words && !*abort_flag) {
-        unsigned long long w = (unsigned long long)(a.epoch & 0xffffu) << 48;
+        unsigned long long w = (unsigned long long)tag << 48;
         for (int j = 0; j < 4; ++j) w |= (unsigned long long)hist[4 * tid + j] << (12 * j);
         asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(a.hist + (size_t)row * words + tid), "l"(w) : "memory");
     }
+    // The row is counted, also after a failed wait: with the last one, every block has read launch[0].  (By a thread
+    // that has no row to wait for in a small layer: at the block's end the count took 0.3 of 31 us.)
+    if (tid == kPlaceThreads - 1 && atomicInc(a.launch + 1, (unsigned)n_rows - 1) == (unsigned)n_rows - 1) a.launch[0] = launch + 1;
     for (int i = tid; i < kPlaceWarps * kPlaceMaxE; i += kPlaceThreads) (&s->wcount[0][0])[i] = 0;
     // `width` threads per row, a word each; four rows in flight
     const int width = words <= 16 ? 16 : words <= 32 ? 32 : 64, groups = kPlaceThreads / width;
@@ -468,7 +480,7 @@ __device__ __forceinline__ void place_tokens(const PlaceArgs& a, int row, int n_
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 if (r0 + j * groups >= row) break;
-                while ((uint32_t)(v[j] >> 48) != (a.epoch & 0xffffu)) {
+                while ((uint32_t)(v[j] >> 48) != tag) {
                     __nanosleep(100);
                     v[j] = ld_relaxed_u64(a.hist + (size_t)(r0 + j * groups) * words + word);
                     if (*abort_flag) break;
@@ -569,18 +581,20 @@ constexpr int kPlaceOwn = 32;
 __global__ void __launch_bounds__(kPlaceThreads) place_kernel(PlaceArgs a) {
     __shared__ PlaceScratch s;
     __shared__ int hist[kPlaceMaxE], top[kPlaceOwn * kMaxTopK], abort;
+    __shared__ unsigned launch;
     pdl_wait();
     pdl_trigger();
     const int tid = threadIdx.x, tok0 = blockIdx.x * kPlaceOwn, own = min(kPlaceOwn, a.S - tok0);
     for (int e = tid; e < kPlaceMaxE; e += kPlaceThreads) hist[e] = 0;
     if (tid == 0) abort = 0;
+    if (tid == kPlaceThreads - 1) launch = ld_relaxed_u32(a.launch);
     __syncthreads();
     if (tid < own * a.K) {
         top[tid] = a.topk[(size_t)tok0 * a.K + tid];
         atomicAdd(&hist[top[tid]], 1);
     }
     __syncthreads();
-    place_tokens(a, blockIdx.x, gridDim.x, tok0, own, top, hist, &s, &abort, a.status);
+    place_tokens(a, launch, blockIdx.x, gridDim.x, tok0, own, top, hist, &s, &abort, a.status);
 }
 
 }  // namespace kleos

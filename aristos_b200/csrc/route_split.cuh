@@ -63,6 +63,7 @@ struct Control {
     unsigned long long got;                            // the other blocks' parts of this block's logits have arrived
     uint32_t tmem_base;
     int abort;
+    unsigned launch;                                   // PlaceArgs::launch[0]
     __align__(16) float bias[128];
     int hist[128];
     int top[BM * kMaxTopK];                            // chosen experts of this block's tokens
@@ -209,6 +210,7 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     cluster_sync_all();  // the cluster's blocks all run before anyone stores into their shared memory
     tc_fence_after();
     const uint32_t tmem_base = ctl->tmem_base;
+    if (tid == 64 && a.place.slots != nullptr) ctl->launch = ld_relaxed_u32(a.place.launch);  // (read after later barriers)
 
     const int KS = H / BKE, kb0 = me * KS / C, kb1 = (me + 1) * KS / C;  // this block's part of K
     const int n_rt = (S + BM - 1) / BM, n_clusters = (int)gridDim.x / C, cluster_id = (int)blockIdx.x / C;
@@ -521,7 +523,7 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             a.r.col_partial[(size_t)row * PXT + tid - 128] = sum;
         }
         if (a.place.slots != nullptr)
-            place_tokens(a.place, row, n_rt * C, rt * BM + me * own, own, ctl->top, ctl->hist, &scr->place, abort_flag, a.status);
+            place_tokens(a.place, ctl->launch, row, n_rt * C, rt * BM + me * own, own, ctl->top, ctl->hist, &scr->place, abort_flag, a.status);
         if (rt + n_clusters < n_rt) {
             // another round: every block of the cluster is done with the partial logits it received, and the
             // operand stages are handed back to the TMA

@@ -758,10 +758,10 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     }
                     __syncwarp();
                     if (lane == src) {
-                        int c_in = 0;
+                        int c_in = 0;  // the complement of the band above kth, by the same subtraction
 #pragma unroll
                         for (int j = 0; j < KC; ++j)
-                            if (j < K && val[j] > kth + eps) ++c_in;
+                            if (j < K && val[j] - kth > eps) ++c_in;
                         const int need = K - c_in;
                         for (int r = 0; r < need; ++r) {
                             int best = -1;
@@ -770,6 +770,11 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                                 if (best < 0 || band_v[b] > band_v[best] ||
                                     (band_v[b] == band_v[best] && band_id[b] < band_id[best]))
                                     best = b;
+                            }
+                            if (best < 0) {  // (the band holds every open place's expert)
+                                sel_id[r] = 0;
+                                sel_l[r] = kth;
+                                continue;
                             }
                             sel_id[r] = band_id[best];
                             sel_l[r] = band_l[best];

@@ -135,14 +135,17 @@ __device__ __noinline__ void settle_near_ties(unsigned flagged, const float* log
         }
         __syncwarp();
         if (lane == 0) {
-            int c_in = 0;  // chosen without doubt
-            for (int j = 0; j < K; ++j) c_in += scr->sel_v[tok_s][j] > kth_s + eps_s;
+            // Chosen without doubt: the same subtraction as above, so that every chosen expert is either here or in
+            // the band.  (kth + eps rounds to another value: an expert at 1.0001f with kth = 1 was in neither.)
+            int c_in = 0;
+            for (int j = 0; j < K; ++j) c_in += scr->sel_v[tok_s][j] - kth_s > eps_s;
             for (int j = c_in; j < K; ++j) {
                 int best = -1;
                 for (int b = 0; b < nb; ++b) {
                     if (band_id[b] < 0) continue;
                     if (best < 0 || band_v[b] > band_v[best]) best = b;  // (ids ascend)
                 }
+                if (best < 0) break;  // (the band holds every open place's expert)
                 scr->sel_i[tok_s][j] = band_id[best];
                 scr->sel_v[tok_s][j] = l[band_id[best]];
                 band_id[best] = -1;

@@ -107,11 +107,13 @@ __device__ __forceinline__ double dot64(const TE* x, const TE* w, int H, int lan
 // Near-ties, by a whole warp (eight tokens, four lanes each; rare, so it stays out of line): the experts
 // within eps of the k-th logit are re-evaluated in fp64 and the open places of the top-k are filled from
 // them (larger value first, equal values to the lower id).  Experts further above are in the set and
-// experts further below are out of it whatever the summation order.
+// experts further below are out of it whatever the summation order.  keep64: the band's logits are replaced by
+// the fp64 ones, from which the probabilities and mCw then come (all callers but the inference of 16-bit layers, which
+// gives the bits of the persistent kernel).
 template <typename TE>
-__device__ __noinline__ void settle_near_ties(unsigned flagged, const float* logits, int ld, int E, int K, float kth, float eps,
+__device__ __noinline__ void settle_near_ties(unsigned flagged, float* logits, int ld, int E, int K, float kth, float eps,
                                               const TE* A, int t, const TE* Wg, int H, const float* bias, Scratch* scr,
-                                              int tok) {
+                                              int tok, bool keep64) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     short* band_id = scr->band_id[warp];
     double* band_v = scr->band_v[warp];
@@ -120,7 +122,7 @@ __device__ __noinline__ void settle_near_ties(unsigned flagged, const float* log
         flagged &= flagged - 1;
         const float kth_s = __shfl_sync(0xffffffffu, kth, src), eps_s = __shfl_sync(0xffffffffu, eps, src);
         const int tok_s = __shfl_sync(0xffffffffu, tok, src), t_s = __shfl_sync(0xffffffffu, t, src);
-        const float* l = logits + (size_t)tok_s * ld;
+        float* l = logits + (size_t)tok_s * ld;
         int nb = 0;
         for (int e0 = 0; e0 < E; e0 += 32) {
             const unsigned in = __ballot_sync(0xffffffffu, e0 + lane < E && fabsf(l[e0 + lane] - kth_s) <= eps_s);
@@ -131,7 +133,10 @@ __device__ __noinline__ void settle_near_ties(unsigned flagged, const float* log
         for (int b = 0; b < nb; ++b) {
             const int e = band_id[b];
             const double dot = dot64<TE>(A + (size_t)t_s * H, Wg + (size_t)e * H, H, lane);
-            if (lane == 0) band_v[b] = dot + (double)bias[e];
+            if (lane == 0) {
+                band_v[b] = dot + (double)bias[e];
+                if (keep64) l[e] = (float)band_v[b];
+            }
         }
         __syncwarp();
         if (lane == 0) {
@@ -451,7 +456,9 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             __syncwarp();
             const float eps = a.r.tie_eps * fmaxf(1.f, fabsf(kth));
             const unsigned flagged = __ballot_sync(0xffffffffu, sub == 0 && t < S && K < E && (kth - next) < eps && !*abort_flag);
-            if (flagged) settle_near_ties<TE>(flagged, recv, LD, E, K, kth, eps, A, t, Wg, H, ctl->bias, scr, tok);
+            if (flagged)
+                settle_near_ties<TE>(flagged, recv, LD, E, K, kth, eps, A, t, Wg, H, ctl->bias, scr, tok,
+                                     kWide || kFine || a.r.col_partial != nullptr);
             float d = 0.f;
 #pragma unroll 1
             for (int i = 0; i < PER; i += 4) {

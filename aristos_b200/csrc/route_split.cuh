@@ -86,6 +86,12 @@ __device__ __forceinline__ void bulk_to_block(uint32_t dst_cluster, uint32_t src
                  : "memory");
 }
 
+// a + b - fl(a + b), exactly (Knuth's two-sum); 0 beside a sum that is not finite
+__device__ __forceinline__ float add_rest(float a, float b) {
+    const float s = a + b, t = s - a;
+    return fabsf(s) < INFINITY ? (a - (s - t)) + (b - t) : 0.f;
+}
+
 // fp64 dot product of a token row and a gate-weight row, by the whole warp
 template <typename TE>
 __device__ __forceinline__ double dot64(const TE* x, const TE* w, int H, int lane) {
@@ -459,7 +465,7 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             if (flagged)
                 settle_near_ties<TE>(flagged, recv, LD, E, K, kth, eps, A, t, Wg, H, ctl->bias, scr, tok,
                                      kWide || kFine || a.r.col_partial != nullptr);
-            float d = 0.f;
+            float d = 0.f, d_rest = 0.f;
 #pragma unroll 1
             for (int i = 0; i < PER; i += 4) {
                 const int e0 = sub * PER + i;
@@ -468,17 +474,28 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 v.y = e0 + 1 < E ? __expf(v.y - m) : 0.f;
                 v.z = e0 + 2 < E ? __expf(v.z - m) : 0.f;
                 v.w = e0 + 3 < E ? __expf(v.w - m) : 0.f;
-                d += (v.x + v.y) + (v.z + v.w);
+                const float four = (v.x + v.y) + (v.z + v.w);
+                if (kFine) d_rest += add_rest(d, four);
+                d += four;
                 *reinterpret_cast<float4*>(l + i) = v;
             }
-            d += __shfl_xor_sync(0xffffffffu, d, 1);
-            d += __shfl_xor_sync(0xffffffffu, d, 2);
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) {
+                const float other = __shfl_xor_sync(0xffffffffu, d, o);
+                if (kFine) d_rest += __shfl_xor_sync(0xffffffffu, d_rest, o) + add_rest(d, other);
+                d += other;
+            }
+            if (kFine) d += d_rest;  // (mCw is a 32-bit result: its sums and its quotient are rounded once each)
             const float inv = 1.f / d;
             if (sub == 0 && t < S && !*abort_flag) {
                 float w[KC];
 #pragma unroll
-                for (int j = 0; j < KC; ++j) w[j] = j < K ? __fmul_rn(__expf(scr->sel_v[tok][j] - m), inv) : 0.f;
-                a.r.mcw[t] = pair_sum(w);
+                for (int j = 0; j < KC; ++j) {
+                    const float x = j < K ? __expf(scr->sel_v[tok][j] - m) : 0.f;
+                    w[j] = kFine ? x : __fmul_rn(x, inv);
+                }
+                const float chosen = pair_sum(w);
+                a.r.mcw[t] = kFine ? __fdiv_rn(chosen, d) : chosen;
 #pragma unroll 1
                 for (int j = 0; j < K; ++j) {
                     const int e = scr->sel_i[tok][j];

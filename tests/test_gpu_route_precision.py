@@ -49,3 +49,25 @@ def test_layer(dtype, train):
     _, _, routing = hz.run_layer_single_gpu(cfg, packed[0])
     assert not routing["topk"].any()
     assert np.abs(routing["mcw"].astype(np.float64) - want).max() <= 2.0 ** -22
+
+
+@pytest.mark.parametrize("H,E,K", [(640, 24, 8), (512, 16, 4), (2048, 64, 2)])
+def test_mcw_is_no_less_exact_than_from_the_fp32_pipes(H, E, K):
+    """mCw of the tensor-core router against 64 bits, and that of the FP32-pipe router on the same values."""
+    import torch
+    S = 4096
+    rng = np.random.default_rng(H)
+    A = synth.round_to_dtype(rng.standard_normal((S, H), dtype=np.float32), 2)
+    W = np.zeros((64, H), np.float32)
+    W[:E] = synth.round_to_dtype(rng.standard_normal((E, H), dtype=np.float32) / np.float32(np.sqrt(H)), 2)
+    logits = A.astype(np.float64) @ W[:E].astype(np.float64).T
+    p = np.exp(logits - logits.max(1, keepdims=True))
+    want = -np.sort(-p, 1)[:, :K].sum(1) / p.sum(1)
+    off = {}
+    for dtype, tdt in ((0, torch.float32), (2, torch.bfloat16)):
+        a, w = (torch.from_numpy(x).cuda().to(tdt) for x in (A, W))
+        probs = torch.empty(S, 64, dtype=tdt, device="cuda")
+        topk, mcw = torch.empty(S, K, dtype=torch.int32, device="cuda"), torch.empty(S, device="cuda")
+        kleos.route_static(a, w, None, S, H, E, K, dtype, probs, topk, mcw)
+        off[dtype] = np.sqrt((((mcw.cpu().numpy() - want) / want) ** 2).mean())
+    assert off[2] <= off[0], off

@@ -55,6 +55,7 @@ struct Args {
     // kFine: K slices that one accumulator sums before the next one takes over.  When tensor memory is full of
     // accumulators they are read, and the first ones start again.
     int acc_slices;
+    int withhold;              // kFine, test hook: a cluster's first block keeps its partial logits, so that the others' waits run out
 };
 
 struct Control {
@@ -369,7 +370,7 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             asm volatile("bar.sync 1, 256;" ::: "memory");
-            if (tid == 128 && !*abort_flag)
+            if (tid == 128 && !*abort_flag && !(kFine && a.withhold && me == 0))
                 for (int p = 1; p < C; ++p) {
                     const int to = (me + p) % C;
                     bulk_to_block(map_to_cta(smem_u32(recv + (size_t)me * own * LD), (uint32_t)to),
@@ -503,6 +504,11 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     ctl->top[tok * K + j] = e;
                     atomicAdd(&ctl->hist[e], 1);
                 }
+            } else if (kFine && sub == 0 && t < S) {
+                // no host code asks for a status here: a token whose logits did not come says so itself
+                a.r.mcw[t] = __int_as_float(0x7fc00000);
+#pragma unroll 1
+                for (int j = 0; j < K; ++j) a.r.topk[(size_t)t * K + j] = -1;
             }
             // probabilities, padding columns zero
             TE* dst = static_cast<TE*>(a.r.probs) + (size_t)t * PXT + sub * PER;

@@ -4,9 +4,10 @@
 // decision: code running inside a framework's memory-pool callback, a real-time serving loop
 // that has pinned its memory budget up front, or a process whose allocator is owned by another
 // runtime.  The regular path (kleos_initialize + kleos_forward) allocates its bookkeeping once
-// at initialise time; this entry point needs no initialise call at all.  The router's scratch
-// (the list of near-tie tokens, their fp64 logits, completion counters, a zero bias) lives in
-// the fixed array below, which every GPU that loads the library holds until the process exits.
+// at initialise time; this entry point needs no initialise call at all.  The float router's scratch
+// (the list of near-tie tokens, their fp64 logits, completion counters) and a zero bias live in
+// the fixed array below, which every GPU that loads the library holds until the process exits.  The bf16
+// router keeps everything else on the chip.
 //
 // This file is compiled as part of kleos_api.cu (one translation unit), so the array, the
 // cudaGetSymbolAddress call and the launches below all see the same symbol.
@@ -16,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdio>
+#include <cstdlib>
 
 #include "route_split.cuh"
 
@@ -27,11 +29,11 @@ constexpr int kMaxDevices = 64;
 
 // Layout of the scratch array (byte offsets, all 256-byte aligned).
 constexpr size_t kOffCount = 0;                                                // int
-constexpr size_t kOffStatus = 64;                                              // DeviceStatus
+constexpr size_t kOffStatus = 64;                                              // DeviceStatus, bf16: the tokens say it too
 constexpr size_t kOffDone = 256;                                               // int[S]
 constexpr size_t kOffList = kOffDone + sizeof(int) * kStaticMaxTokens;         // int[S]
 constexpr size_t kOffZeroBias = kOffList + sizeof(int) * kStaticMaxTokens;     // float[E], stays 0
-constexpr size_t kClearBytes = kOffZeroBias + 256;                             // cleared every call
+constexpr size_t kClearBytes = kOffZeroBias + 256;                             // cleared by every float call
 constexpr size_t kOffLogits = kClearBytes;                                     // double[S*E]
 constexpr size_t kScratchBytes =
     kOffLogits + sizeof(double) * kStaticMaxTokens * kStaticMaxExperts;
@@ -40,7 +42,12 @@ static_assert(kScratchBytes == 2130432, "the size quoted in kleos_b200.h and in 
 // In host code this name is only a handle for cudaGetSymbolAddress, never a device address.
 static __device__ __align__(256) unsigned char g_route_scratch[kScratchBytes];
 
-unsigned char* g_scratch_ptr[kMaxDevices] = {};
+struct StaticDevice {
+    unsigned char* scratch = nullptr;
+    long long wait_cycles = 20000000000LL;  // about ten seconds; KLEOS_WAIT_MS at the first call
+    int withhold = 0;                       // KLEOS_DEBUG_STATIC_WITHHOLD=1 at the first call: see route_split::Args
+};
+StaticDevice g_static[kMaxDevices];
 
 int complain(int code, const char* what) {
     std::fprintf(stderr, "[kleos_b200] kleos_route_static: %s\n", what);
@@ -69,7 +76,8 @@ extern "C" int kleos_route_static(const void* A, const void* Wg, const float* ga
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices)
         return complain(KLEOS_E_CUDA, "no current CUDA device");
-    if (!g_scratch_ptr[dev]) {
+    StaticDevice& here = g_static[dev];
+    if (!here.scratch) {
         // one-time set-up for this device (do the first call outside any stream capture)
         void* p = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&p, g_route_scratch);
@@ -82,9 +90,16 @@ extern "C" int kleos_route_static(const void* A, const void* Wg, const float* ga
                          cudaGetErrorString(e));
             return KLEOS_E_CUDA;
         }
-        g_scratch_ptr[dev] = static_cast<unsigned char*>(p);
+        if (const char* w = std::getenv("KLEOS_WAIT_MS")) {
+            int khz = 0;
+            if (cudaDeviceGetAttribute(&khz, cudaDevAttrClockRate, dev) == cudaSuccess)
+                here.wait_cycles = (long long)(std::atof(w) * khz);
+        }
+        const char* wh = std::getenv("KLEOS_DEBUG_STATIC_WITHHOLD");
+        here.withhold = wh && wh[0] == '1';
+        here.scratch = static_cast<unsigned char*>(p);
     }
-    unsigned char* scratch = g_scratch_ptr[dev];
+    unsigned char* scratch = here.scratch;
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : cudaStreamPerThread;
 
     RouteArgs ra{};
@@ -123,7 +138,8 @@ extern "C" int kleos_route_static(const void* A, const void* Wg, const float* ga
         route_split::Args sp{};
         sp.r = ra;
         sp.status = reinterpret_cast<DeviceStatus*>(scratch + kOffStatus);
-        sp.place.wait_cycles = 20000000000LL;
+        sp.place.wait_cycles = here.wait_cycles;
+        sp.withhold = here.withhold;
         const int slices = H / 64;
         sp.parts = slices >= 4 ? 4 : slices >= 2 ? 2 : 1;
         sp.acc_slices = 1;

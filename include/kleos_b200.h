@@ -204,9 +204,11 @@ int kleos_debug_gemm_stats(long long* out, int max_values);
  *   Limits: S <= 4096, E <= 64, K <= min(E, 8), H a multiple of 64, torch_dtype 0 or 2; anything
  *   larger is refused with KLEOS_E_ARG and a message on stderr.
  * The first call on each device looks up the array's device address; make that call before any
- * stream capture.  All calls share the one array and each call first clears the part that must
- * start at zero, so two calls that overlap on the GPU (different streams, different threads)
- * race: serialise them.  Asynchronous on `stream` (NULL = per-thread default stream). */
+ * stream capture.  Float calls share the array, and each clears the part that must start at zero, so two
+ * float calls that overlap on the GPU (different streams, different threads) race: serialise them.
+ * bf16 calls only read the zero bias there and may overlap.  Asynchronous on `stream` (NULL = per-thread
+ * default stream).  The bf16 kernel's waits are bounded (KLEOS_WAIT_MS at the first call on the device, about ten
+ * seconds without it): a token whose logits did not come in time has topk = -1 and mcw = NaN. */
 int kleos_route_static(const void* A, const void* Wg, const float* gate_bias, int S, int H, int E,
                        int K, int torch_dtype, void* probs, int32_t* topk, float* mcw,
                        void* stream);

@@ -574,24 +574,24 @@ __device__ __forceinline__ void place_tokens(const PlaceArgs& a, unsigned launch
 }
 
 // The same on its own, behind the routers whose blocks do not have 512 threads or whose choices the near-tie
-// kernel may change: one block per 32 tokens.  Blocks wait for lower ones, which are placed on the chip first.
-// It stands for three kernels (histogram 2.8 us, slots 5.9, rows 3.9 at 256 tokens, 8 float experts, where the
-// forward went from 97.5 to 85 with the return flags gone too).
-constexpr int kPlaceOwn = 32;
-__global__ void __launch_bounds__(kPlaceThreads) place_kernel(PlaceArgs a) {
+// kernel may change: one block per 32, 64 or 128 tokens (place_own()).  Blocks wait for lower ones, which are placed on
+// the chip first.  It stands for three kernels (histogram 2.8 us, slots 5.9, rows 3.9 at 256 tokens, 8 float experts,
+// where the forward went from 97.5 to 85 with the return flags gone too).
+constexpr int kPlaceOwn = 32, kPlaceOwnMost = 128;
+__global__ void __launch_bounds__(kPlaceThreads) place_kernel(PlaceArgs a, int tokens) {
     __shared__ PlaceScratch s;
-    __shared__ int hist[kPlaceMaxE], top[kPlaceOwn * kMaxTopK], abort;
+    __shared__ int hist[kPlaceMaxE], top[kPlaceOwnMost * kMaxTopK], abort;
     __shared__ unsigned launch;
     pdl_wait();
     pdl_trigger();
-    const int tid = threadIdx.x, tok0 = blockIdx.x * kPlaceOwn, own = min(kPlaceOwn, a.S - tok0);
+    const int tid = threadIdx.x, tok0 = blockIdx.x * tokens, own = min(tokens, a.S - tok0);
     for (int e = tid; e < kPlaceMaxE; e += kPlaceThreads) hist[e] = 0;
     if (tid == 0) abort = 0;
     if (tid == kPlaceThreads - 1) launch = ld_relaxed_u32(a.launch);
     __syncthreads();
-    if (tid < own * a.K) {
-        top[tid] = a.topk[(size_t)tok0 * a.K + tid];
-        atomicAdd(&hist[top[tid]], 1);
+    for (int i = tid; i < own * a.K; i += kPlaceThreads) {
+        top[i] = a.topk[(size_t)tok0 * a.K + i];
+        atomicAdd(&hist[top[i]], 1);
     }
     __syncthreads();
     place_tokens(a, launch, blockIdx.x, gridDim.x, tok0, own, top, hist, &s, &abort, a.status);

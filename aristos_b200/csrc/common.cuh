@@ -159,6 +159,8 @@ __device__ __forceinline__ bool wait_flag(const unsigned long long* flag, uint32
 // kernel calls it, before it touches any global memory that a kernel writes, so that completion is
 // transitive along the stream; pdl_trigger() lets the next kernel's blocks start to arrive.  Both do
 // nothing in a kernel that was launched without the attribute.  (A launch boundary cost 2 to 3 us.)
+// For the same reason no kernel reads through the read-only path (__ldg, ld.global.nc): that is only defined on data
+// which no one writes while the kernel is resident, and the kernel in front, the caller's own among them, may still be.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

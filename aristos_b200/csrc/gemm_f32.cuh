@@ -442,7 +442,7 @@ ffn_gemm_f32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
                     }
                     __syncwarp();
                     const int j = lane & 7, col = c * 32 + 4 * j;
-                    const float4 bf = __ldg(reinterpret_cast<const float4*>(bq + col));
+                    const float4 bf = *reinterpret_cast<const float4*>(bq + col);
 #pragma unroll 1
                     for (int r = lane >> 3; r < 8 && hr + r < rows_w; r += 4) {
                         const uint4 raw = stg[r * 8 + (j ^ r)];

@@ -53,8 +53,8 @@ __global__ void __launch_bounds__(256) ffn_gemm_simt(GemmArgs g) {
             uint4 ra[NV], rb[NV];
 #pragma unroll
             for (int v = 0; v < NV; ++v) {
-                ra[v] = __ldg(reinterpret_cast<const uint4*>(arow + k0 + lk) + v);
-                rb[v] = brow_ok ? __ldg(reinterpret_cast<const uint4*>(brow + k0 + lk) + v)
+                ra[v] = reinterpret_cast<const uint4*>(arow + k0 + lk)[v];
+                rb[v] = brow_ok ? reinterpret_cast<const uint4*>(brow + k0 + lk)[v]
                                 : make_uint4(0u, 0u, 0u, 0u);
             }
             const T* ea = reinterpret_cast<const T*>(ra);

@@ -519,7 +519,7 @@ ffn_gemm_tc2(const __grid_constant__ gemm_tc2::RowMaps map_x, const __grid_const
             const bool mine = lane < per && at < x.half;
             const int row = (leader ? x.row_base[0] : x.row_base[1]) + at;
             int4 rows = make_int4(0, 0, 0, 0);
-            if (mine) rows = __ldg(reinterpret_cast<const int4*>(g.row_token + row));  // (past the last row: some earlier forward's tokens)
+            if (mine) rows = *reinterpret_cast<const int4*>(g.row_token + row);  // (past the last row: some earlier forward's tokens)
             bool ok = true;
             for (int kb = 0; kb < KS; ++kb, ++it) {
                 const int s = it % kSlices;

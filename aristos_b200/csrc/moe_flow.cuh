@@ -420,8 +420,8 @@ __device__ __forceinline__ double warp_dot64(const T* x, const T* w, int H, int 
     double s = 0.0;
 #pragma unroll 4
     for (int h = lane * VEC; h < H; h += 32 * VEC) {
-        const uint4 xr = __ldg(reinterpret_cast<const uint4*>(x + h));
-        const uint4 wr = __ldg(reinterpret_cast<const uint4*>(w + h));
+        const uint4 xr = *reinterpret_cast<const uint4*>(x + h);
+        const uint4 wr = *reinterpret_cast<const uint4*>(w + h);
         const T* xv = reinterpret_cast<const T*>(&xr);
         const T* wv = reinterpret_cast<const T*>(&wr);
 #pragma unroll
@@ -1587,7 +1587,7 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 const int nb = ti.nt * BN + 8 * lane;
                 float* bs = &ctl->bias_s[q][8 * lane];
                 if (nb < N) {
-                    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(bias + (size_t)ti.le * N + nb));
+                    const uint4 raw = *reinterpret_cast<const uint4*>(bias + (size_t)ti.le * N + nb);
                     const TE2* h2 = reinterpret_cast<const TE2*>(&raw);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
@@ -1705,8 +1705,8 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
                         if (c0 + 32 * k < row_chunks) {
-                            v0[k] = __ldg(src0 + c0 + 32 * k);
-                            if (two) v1[k] = __ldg(src1 + c0 + 32 * k);
+                            v0[k] = src0[c0 + 32 * k];
+                            if (two) v1[k] = src1[c0 + 32 * k];
                         }
 #pragma unroll
                     for (int k = 0; k < 8; ++k)

@@ -558,7 +558,7 @@ __device__ __forceinline__ void place_tokens(const PlaceArgs& a, unsigned launch
                 uint4 v[8];
 #pragma unroll
                 for (int q = 0; q < 8; ++q)
-                    if (c0 + 32 * q < a.row_chunks) v[q] = __ldg(src + c0 + 32 * q);
+                    if (c0 + 32 * q < a.row_chunks) v[q] = src[c0 + 32 * q];
 #pragma unroll 1
                 for (int j = 0; j < K; ++j) {
                     const int to = top[tk * K + j];

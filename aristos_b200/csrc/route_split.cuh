@@ -100,7 +100,7 @@ __device__ __forceinline__ double dot64(const TE* x, const TE* w, int H, int lan
     double s = 0.0;
 #pragma unroll 4
     for (int h = lane * VEC; h < H; h += 32 * VEC) {
-        const uint4 xr = __ldg(reinterpret_cast<const uint4*>(x + h)), wr = __ldg(reinterpret_cast<const uint4*>(w + h));
+        const uint4 xr = *reinterpret_cast<const uint4*>(x + h), wr = *reinterpret_cast<const uint4*>(w + h);
         const TE* xv = reinterpret_cast<const TE*>(&xr);
         const TE* wv = reinterpret_cast<const TE*>(&wr);
 #pragma unroll

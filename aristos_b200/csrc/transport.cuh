@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(256) dispatch_kernel(DispatchArgs a) {
             uint4 v[8];
 #pragma unroll
             for (int q = 0; q < 8; ++q)
-                if (c0 + 32 * q < row_chunks) v[q] = __ldg(src + c0 + 32 * q);
+                if (c0 + 32 * q < row_chunks) v[q] = src[c0 + 32 * q];
 #pragma unroll
             for (int q = 0; q < 8; ++q)
                 if (c0 + 32 * q < row_chunks) dst[c0 + 32 * q] = v[q];

@@ -68,7 +68,7 @@ struct State {
     bool fuse_route = false;                 // ... and the router runs inside it too (KLEOS_FUSE_ROUTE=0: separate launches)
     // One rank, separate launches: it owns every expert, so the rows only move inside this GPU's memory, with
     // no plan, and no flags to raise or to wait for (KLEOS_DISPATCH_KERNELS=1: the dispatch and plan
-    // kernels of several ranks instead)
+    // kernels of several ranks instead, and GEMMs that work through the panel list)
     bool local = false;
     bool gather = false;                     // GEMM1 fetches the token rows from the activations by index
     bool split_route = false;                // the router is route_split_kernel (KLEOS_ROUTE_KERNELS=1: the kernels of route.cuh)
@@ -689,7 +689,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
     const int flags = g.local && !g.suppress_return_flag ? 0 : g.world;  // (the test hook needs something to wait for)
     ga.ret.rank = g.rank; ga.ret.world = flags; ga.ret.epoch = g.epoch;
     ga.ret.suppress = g.suppress_return_flag ? 1 : 0;
-    ga.contiguous = g.world == 1; ga.next_tile = g.tile_claims; ga.counts = g.counts; ga.EC = c.EC;
+    ga.contiguous = g.local; ga.next_tile = g.tile_claims; ga.counts = g.counts; ga.EC = c.EC;
     GemmArgs g1 = ga;
     g1.row_token = g.cell_tokens;
     g1.A = g.arena + g.lay.xcell; g1.B = s.W1; g1.bias = s.b1; g1.N = c.I; g1.Kd = c.H; g1.mode = 0;

@@ -72,7 +72,8 @@ struct State {
     bool local = false;
     bool gather = false;                     // GEMM1 fetches the token rows from the activations by index
     bool split_route = false;                // the router is route_split_kernel (KLEOS_ROUTE_KERNELS=1: the kernels of route.cuh)
-    int route_parts = 1;                     // ... blocks per 128 tokens: parts of K whose logits are summed apart
+    int route_own = 128;                     // ... tokens that a block decides on
+    int route_parts = 0;                     // ... TF32: blocks per 128 tokens (a cluster), parts of K whose logits are summed apart
     int route_grid = 0;                      // ... its blocks, no more than the device holds at once
     unsigned long long* place_hist = nullptr;  // see PlaceArgs
     unsigned* place_launch = nullptr;          // ...
@@ -285,6 +286,9 @@ int make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, u
     return err ? fail(KLEOS_E_CUDA, "%s", err) : KLEOS_OK;
 }
 
+// Token rows of a box of the router's operand: 128 where a cluster or a block of the persistent kernel loads them
+uint32_t route_rows() { return g.fuse_route || g.use_tf32_tc ? route_split::BM : (uint32_t)g.route_own; }
+
 // The boxes of token rows that ffn_gemm_tc2 loads
 int make_row_maps(gemm_tc2::RowMaps* m, const void* base, uint64_t rows, uint64_t cols) {
     const uint32_t bk = 128 / (uint32_t)g.cfg.elem_bytes;
@@ -336,7 +340,7 @@ int ensure_maps(const Sections& s) {
         if ((rc = make_map(&g.map_w1h, s.W1, (uint64_t)g.nLx * c.I, c.H, gemm_tc2::BM, bk))) return rc;
         if ((rc = make_map(&g.map_w2h, s.W2, (uint64_t)g.nLx * c.H, c.I, gemm_tc2::BM, bk))) return rc;
         if (c.PX <= 128 && !g.dense) {
-            if ((rc = make_map(&g.map_act, s.A, c.S, c.H, route_split::BM, bk))) return rc;
+            if ((rc = make_map(&g.map_act, s.A, c.S, c.H, route_rows(), bk))) return rc;
             if ((rc = make_map(&g.map_wg, s.Wg, c.PX, c.H, c.PX, bk))) return rc;
         }
         g.maps_for_iP = s.A;
@@ -347,7 +351,7 @@ int ensure_maps(const Sections& s) {
     if ((rc = make_map(&g.map_w1h, s.W1, (uint64_t)g.nLx * c.I, c.H, gemm_tc2::BM))) return rc;
     if ((rc = make_map(&g.map_w2h, s.W2, (uint64_t)g.nLx * c.H, c.I, gemm_tc2::BM))) return rc;
     if (c.PX <= 128 && !g.dense) {
-        if ((rc = make_map(&g.map_act, s.A, c.S, c.H, route_split::BM))) return rc;
+        if ((rc = make_map(&g.map_act, s.A, c.S, c.H, route_rows()))) return rc;
         if ((rc = make_map(&g.map_wg, s.Wg, c.PX, c.H, c.PX))) return rc;
         // the half of the gate weight each block of a pair loads when the router runs inside the
         // persistent kernel
@@ -395,12 +399,26 @@ int with_route_split(F f) {
 // Every block of the chip issues its share: left to the four with tokens it took the router 98 us.
 constexpr size_t kAheadBytes = (size_t)64 << 20;
 
-// How the router's work is spread: as many blocks per 128 tokens (1, 2 or 4 in a cluster) as find room
-// on the chip beside those of the other tokens, none without a slice of K, and no more than the
-// persistent kernel's routing phase has accumulator columns for.
+// How the router's work is spread.  16-bit layers: 32, 64 or 128 tokens a block, the fewest with which the chip holds
+// all blocks at once.  TF32 layers: as many blocks per 128 tokens (1, 2 or 4 in a cluster, with a part of K each) as find
+// room on the chip beside those of the other tokens, none without a slice of K, and 256 columns at most.
 template <typename T>
 int prepare_route_split() {
     const LayerConfig& c = g.cfg;
+    if constexpr (sizeof(T) == 2) {
+        g.route_own = 32;
+        while (g.route_own < route_split::BM && c.S > g.route_own * g.sm_count) g.route_own *= 2;
+        int per_sm = 0;
+        const int rc = with_route_split<T>([&](auto kernel, int smem) -> int {
+            KLEOS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            KLEOS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, route_split::kThreads, (size_t)smem));
+            return KLEOS_OK;
+        });
+        if (rc) return rc;
+        if (per_sm < 1) return fail(KLEOS_E_CUDA, "the router does not fit the device");
+        g.route_grid = g.sm_count;  // (those beyond the tokens only bring weights into L2)
+        return KLEOS_OK;
+    }
     const int tiles = c.S / route_split::BM, slices = c.H * c.elem_bytes / 128;
     for (int parts = route_split::kMaxParts;; parts >>= 1) {
         if (parts > 1 && (parts * c.PX > 256 || parts > slices || tiles * parts > g.sm_count)) continue;
@@ -424,6 +442,7 @@ int prepare_route_split() {
         if (parts > 1 && clusters < tiles) continue;
         if (clusters < 1) return fail(KLEOS_E_CUDA, "the router does not fit the device");
         g.route_parts = parts;
+        g.route_own = route_split::BM / parts;
         g.route_grid = clusters * parts;  // (those beyond the tokens only bring weights into L2)
         return KLEOS_OK;
     }
@@ -596,7 +615,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
         // gate GEMM, top-k, near-ties, slots, counts and the panel list in one launch
         if constexpr (!std::is_same<T, float>::value) {
             route_split::Args sp{};
-            sp.r = ra; sp.place = pl; sp.status = g.status; sp.parts = g.route_parts;
+            sp.r = ra; sp.place = pl; sp.status = g.status; sp.own = g.route_own; sp.parts = g.route_parts;
             // (an expert is likely to get a token at all)
             if ((long long)c.S * c.K * g.world >= 2LL * c.E) {
                 sp.ahead = s.W1;
@@ -606,7 +625,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
                 launch_clusters(g.route_parts, kernel, g.route_grid, route_split::kThreads, smem, st, *act_map, g.map_wg, sp);
                 return KLEOS_OK;
             });
-            route_blocks = c.S / route_split::BM * g.route_parts;
+            route_blocks = c.S / g.route_own;
         }
     } else if (routed_in_kernel) {
         // nothing to launch here
@@ -647,7 +666,6 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
             fa.unit_rows = g.flow_unit_rows;
             fa.fuse_route = routed_in_kernel ? 1 : 0;
             fa.Wg = s.Wg; fa.gate_bias = g.bias; fa.tile_hist = g.tile_hist; fa.tie_eps = 1e-4f;
-            fa.parts = g.route_parts;
             if (timed) {
                 KLEOS_CUDA(cudaMemsetAsync(g.flow_stamps, 0,
                                            sizeof(long long) * g.flow_grid * flow::kStampSlots, st));
@@ -815,11 +833,11 @@ int ensure_host_pipe() {
         KLEOS_CUDA(cudaEventCreateWithFlags(&hp.comp_done[b], cudaEventDisableTiming));
         KLEOS_CUDA(cudaEventCreateWithFlags(&hp.out_done[b], cudaEventDisableTiming));
         if (g.use_tc && c.PX <= 128) {
-            int rc = make_map(&hp.map_act[b], hp.act[b], c.S, c.H, route_split::BM);
+            int rc = make_map(&hp.map_act[b], hp.act[b], c.S, c.H, route_rows());
             if (rc) return rc;
-        } else if ((g.use_tf32_tc && (g.dense || c.PX <= 128)) || (g.use_f32_tc && g.dense)) {
-            // same box (128 rows x 32 words) serves the tf32 router and the dense layers' GEMM1
-            int rc = make_map(&hp.map_act[b], hp.act[b], c.S, c.H, gemm_f32::BM, 32);
+        } else if ((g.use_tf32_tc && !g.dense && c.PX <= 128) || (g.use_f32_tc && g.dense)) {
+            // the TF32 router's tokens, or those of the dense float layer's GEMM1
+            int rc = make_map(&hp.map_act[b], hp.act[b], c.S, c.H, g.dense ? gemm_f32::BM : route_rows(), 32);
             if (rc) return rc;
         }
         if (g.dense && (g.use_tc || g.use_tf32_tc)) {

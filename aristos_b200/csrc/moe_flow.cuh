@@ -173,7 +173,6 @@ struct Args {
     const float* gate_bias;  // [E]
     int* tile_hist;          // [S/128][E] per-tile histogram of the chosen experts
     float tie_eps;
-    int parts;               // parts of K whose gate logits are summed apart, as route_split.cuh does it
 };
 
 struct Tile {
@@ -567,14 +566,9 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                         break;
                     }
                     tc_fence_after();
+                    const uint32_t d_tmem = tmem_r + buf * BN;
                     bool ok = true;
-                    int part = 0, part_kb = 0;  // part of K the slice belongs to, and its first slice
                     for (int kb = 0; kb < KSr; ++kb, ++it) {
-                        if (kb == (part + 1) * KSr / a.parts) {
-                            ++part;
-                            part_kb = kb;
-                        }
-                        const uint32_t d_tmem = tmem_r + buf * BN + (uint32_t)(part * a.PX);
                         const int s = it % kSlices;
                         const uint32_t ph = (it / kSlices) & 1;
                         if (!mbar_wait(&ctl->full[s], ph, budget, abort_flag)) {
@@ -589,7 +583,7 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                         const uint64_t db = make_smem_desc(sa + A_STAGE_BYTES);
 #pragma unroll
                         for (int k = 0; k < BK / UMMA_K; ++k)
-                            umma_bf16_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb != part_kb || k != 0) ? 1u : 0u);
+                            umma_bf16_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
                         const uint32_t e_local = smem_u32(&ctl->empty[s]);
                         umma_commit_pair(map_to_cta(e_local, 0));
                         umma_commit_pair(map_to_cta(e_local, 1));
@@ -635,19 +629,6 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 const int row = row_w + lane;
                 const bool valid = row < a.S;
                 const uint32_t taddr = tmem_r + buf * BN + (static_cast<uint32_t>(q * 32) << 16);
-                // 32 logits, without their bias: the parts of K in order
-                auto load_logits = [&](int c, uint32_t* v) {
-                    tmem_ld_32x32(taddr + c * 32, v);
-                    tmem_ld_wait();
-#pragma unroll 1
-                    for (int p = 1; p < a.parts; ++p) {
-                        uint32_t w[32];
-                        tmem_ld_32x32(taddr + p * a.PX + c * 32, w);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
-                    }
-                };
                 float val[KC + 1];
                 int idx[KC + 1];
 #pragma unroll
@@ -658,7 +639,8 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
 #pragma unroll 1
                 for (int c = 0; c < chunks; ++c) {
                     uint32_t v[32];
-                    load_logits(c, v);
+                    tmem_ld_32x32(taddr + c * 32, v);
+                    tmem_ld_wait();
 #pragma unroll
                     for (int jj = 0; jj < 32; ++jj) {
                         const int e = c * 32 + jj;
@@ -681,35 +663,18 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 }
                 if (stamp && q == 0 && lane == 0) stamp[kTopkPass1] = global_ns();
                 const float m = val[0];
-                // sum of the exponentials by quarters of the PX experts, then (q0 + q1) + (q2 + q3): the order
-                // in which the four threads per token of route_split.cuh add them
-                float quarter[4] = {0.f, 0.f, 0.f, 0.f};
-                auto four = [&](int c, int jj, const uint32_t* v) {
-                    float x[4];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const int e = c * 32 + jj + k;
-                        x[k] = e < a.E ? __expf(__uint_as_float(v[jj + k]) + bias_r[e] - m) : 0.f;
-                    }
-                    return (x[0] + x[1]) + (x[2] + x[3]);
-                };
+                float d = 0.f;  // in the order of the experts, as route_split.cuh adds them
 #pragma unroll 1
                 for (int c = 0; c < chunks; ++c) {
                     uint32_t v[32];
-                    load_logits(c, v);
-                    float lo = 0.f, hi = 0.f;  // a chunk of 32 is a quarter (PX = 128) or two (PX = 64)
+                    tmem_ld_32x32(taddr + c * 32, v);
+                    tmem_ld_wait();
 #pragma unroll
-                    for (int jj = 0; jj < 16; jj += 4) lo += four(c, jj, v);
-                    if (chunks > 2) hi = lo;
-#pragma unroll
-                    for (int jj = 16; jj < 32; jj += 4) hi += four(c, jj, v);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        if (chunks > 2 ? k == c : k == 2 * c + 1) quarter[k] = hi;
-                        else if (chunks <= 2 && k == 2 * c) quarter[k] = lo;
+                    for (int jj = 0; jj < 32; ++jj) {
+                        const int e = c * 32 + jj;
+                        if (e < a.E) d += __expf(__uint_as_float(v[jj]) + bias_r[e] - m);
                     }
                 }
-                const float d = (quarter[0] + quarter[1]) + (quarter[2] + quarter[3]);
                 const float inv = 1.f / d;
                 if (stamp && q == 0 && lane == 0) stamp[kTopkDone] = global_ns();
                 float kth = 0.f, next = -INFINITY;
@@ -734,7 +699,8 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
 #pragma unroll 1
                     for (int c = 0; c < chunks; ++c) {
                         uint32_t v[32];
-                        load_logits(c, v);
+                        tmem_ld_32x32(taddr + c * 32, v);
+                        tmem_ld_wait();
                         if (lane == src) {
 #pragma unroll
                             for (int jj = 0; jj < 32; ++jj) {
@@ -789,15 +755,16 @@ moe_flow_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     }
                     __syncwarp();
                 }
-                float w[KC];
+                float wsum = 0.f;
 #pragma unroll
-                for (int j = 0; j < KC; ++j) w[j] = j < K ? __fmul_rn(__expf(val[j] - m), inv) : 0.f;
-                const float wsum = pair_sum(w);
+                for (int j = 0; j < KC; ++j)
+                    if (j < K) wsum = __fmaf_rn(__expf(val[j] - m), inv, wsum);
                 // probabilities, padding columns zero, one 16-byte store per eight experts
 #pragma unroll 1
                 for (int c = 0; c < chunks; ++c) {
                     uint32_t v[32];
-                    load_logits(c, v);
+                    tmem_ld_32x32(taddr + c * 32, v);
+                    tmem_ld_wait();
                     if (c + 1 == chunks) {
                         // last read of this accumulator: hand it back to the MMA issuer
                         tc_fence_before();

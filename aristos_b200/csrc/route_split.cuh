@@ -33,7 +33,7 @@
 namespace kleos {
 namespace route_split {
 
-constexpr int BM = 128, kThreads = 512, kWarps = kThreads / 32, kMaxParts = 4;
+constexpr int BM = 128, kThreads = 512, kWarps = kThreads / 32, kMaxParts = 4, kMaxStages = 14;
 constexpr int W_BYTES = BM * 128;  // one 128-byte K slice of the tokens
 
 template <int PXT>
@@ -51,7 +51,8 @@ struct Args {
     DeviceStatus* status;
     const char* ahead;         // expert weights to bring into L2 while the memory is idle, or null
     size_t ahead_bytes;        // ... a multiple of 16
-    int parts;                 // blocks per cluster
+    int own;                   // layers: tokens per block, 32, 64 or 128
+    int parts;                 // kFine: blocks per cluster
     // kFine: K slices that one accumulator sums before the next one takes over.  When tensor memory is full of
     // accumulators they are read, and the first ones start again.
     int acc_slices;
@@ -59,7 +60,7 @@ struct Args {
 };
 
 struct Control {
-    unsigned long long full[8], empty[8], acc_full;    // acc_full: once per filling of tensor memory
+    unsigned long long full[kMaxStages], empty[kMaxStages], acc_full;  // acc_full: once per filling of tensor memory
     unsigned long long acc_read;                       // a filling's accumulators have been read, eight warps
     unsigned long long got;                            // the other blocks' parts of this block's logits have arrived
     uint32_t tmem_base;
@@ -181,6 +182,7 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     constexpr int KC = KT > 0 ? KT : kMaxTopK;
     static_assert(sizeof(Control) <= 8192 && sizeof(Scratch) <= kSendAt && kSendAt + Sh::RECV_BYTES <= STAGES * Sh::STAGE_BYTES, "shared memory set aside");
     constexpr bool kWide = sizeof(TE) == 4;            // tf32: fp32 words
+    constexpr bool kSplit = kWide || kFine;            // K split over a cluster
     constexpr int BKE = 128 / (int)sizeof(TE);         // elements per K slice
     extern __shared__ uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>(
@@ -190,7 +192,11 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     Scratch* scr = reinterpret_cast<Scratch*>(tiles);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int C = a.parts, me = (int)cluster_ctarank(), own = BM / C;  // tokens this block decides on
+    // own: tokens this block decides on, all alone or (kSplit) after its part of K for the 128 of its cluster
+    const int C = kSplit ? a.parts : 1, me = kSplit ? (int)cluster_ctarank() : 0, own = a.own;
+    const uint32_t rows = kSplit ? BM : own;           // token rows of a K slice
+    const uint32_t stage_bytes = rows * 128 + PXT * 128;
+    const int stages = min(kMaxStages, (int)(STAGES * Sh::STAGE_BYTES / stage_bytes));
     const int S = a.r.S, E = a.r.E, H = a.r.H, K = KT > 0 ? KT : a.r.K;
     const long long wait_cycles = a.place.wait_cycles;
     const uint32_t epoch = a.place.epoch;
@@ -201,7 +207,7 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     else idesc = make_instr_desc_16b(BM, PXT, Pack2<TE>::kMmaFormat);
 
     if (tid == 0) {
-        for (int s = 0; s < STAGES; ++s) {
+        for (int s = 0; s < stages; ++s) {
             mbar_init(&ctl->full[s], 1);
             mbar_init(&ctl->empty[s], 1);
         }
@@ -228,7 +234,7 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     if (tid == 64 && a.place.slots != nullptr) ctl->launch = ld_relaxed_u32(a.place.launch);  // (read after later barriers)
 
     const int KS = H / BKE, kb0 = me * KS / C, kb1 = (me + 1) * KS / C;  // this block's part of K
-    const int n_rt = (S + BM - 1) / BM, n_clusters = (int)gridDim.x / C, cluster_id = (int)blockIdx.x / C;
+    const int n_rt = (S + (int)rows - 1) / (int)rows, n_clusters = (int)gridDim.x / C, cluster_id = (int)blockIdx.x / C;
     const int acc_slices = kFine ? a.acc_slices : KS, n_acc = kFine ? (kb1 - kb0 + acc_slices - 1) / acc_slices : 1;
     constexpr int kAccs = 512 / PXT, kSums = kFine ? PXT / 2 : 1;
     const int fills = kFine ? (n_acc + kAccs - 1) / kAccs : 1;
@@ -246,44 +252,45 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                          : "memory");
     };
     if (tid == 96 && a.ahead != nullptr && cluster_id >= n_rt) bring_ahead();
-    uint32_t it0 = 0, round = 0;
-    for (int rt = cluster_id; rt < n_rt; rt += n_clusters, ++round, it0 += (uint32_t)(kb1 - kb0)) {
+    uint32_t round = 0, s = 0, ph = 0;  // s, ph: stage and parity of the producer, and of the MMA issuer
+    for (int rt = cluster_id; rt < n_rt; rt += n_clusters, ++round) {
         if (tid < PXT) ctl->hist[tid] = 0;
         if (tid == 0 && C > 1) mbar_expect_tx(&ctl->got, (uint32_t)(C - 1) * part_bytes);
         // (after a failed wait the block still runs through its barriers, with the abort flag up, so that
         // the blocks of a cluster meet at the same ones)
         if (warp == 0) {
             if (lane == 0 && !*abort_flag) {
-                uint32_t it = it0;
-                for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (!mbar_wait(&ctl->empty[s], ((it / STAGES) & 1) ^ 1, wait_cycles, abort_flag)) {
+                for (int kb = kb0; kb < kb1; ++kb) {
+                    if (!mbar_wait(&ctl->empty[s], ph ^ 1, wait_cycles, abort_flag)) {
                         report_error(a.status, KLEOS_AT_GEMM_PRODUCER, -100 - rt, (int)epoch);
                         *abort_flag = 1;
                         break;
                     }
-                    mbar_expect_tx(&ctl->full[s], Sh::STAGE_BYTES);
-                    uint8_t* sa = tiles + s * Sh::STAGE_BYTES;
-                    tma_load_2d(sa, &map_a, kb * BKE, rt * BM, &ctl->full[s]);
-                    tma_load_2d(sa + W_BYTES, &map_wg, kb * BKE, 0, &ctl->full[s]);
+                    mbar_expect_tx(&ctl->full[s], stage_bytes);
+                    uint8_t* sa = tiles + s * stage_bytes;
+                    tma_load_2d(sa, &map_a, kb * BKE, rt * (int)rows, &ctl->full[s]);
+                    tma_load_2d(sa + rows * 128, &map_wg, kb * BKE, 0, &ctl->full[s]);
+                    if (++s == (uint32_t)stages) {
+                        s = 0;
+                        ph ^= 1;
+                    }
                 }
             }
             __syncwarp();
         } else if (warp == 1) {
             if (lane == 0 && !*abort_flag) {
-                uint32_t it = it0;
                 bool ok = true;
-                for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (!mbar_wait(&ctl->full[s], (it / STAGES) & 1, wait_cycles, abort_flag)) {
+                for (int kb = kb0; kb < kb1; ++kb) {
+                    if (!mbar_wait(&ctl->full[s], ph, wait_cycles, abort_flag)) {
                         report_error(a.status, KLEOS_AT_GEMM_MMA, -100 - rt, (int)epoch);
                         *abort_flag = 1;
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t sa = smem_u32(tiles + s * Sh::STAGE_BYTES);
-                    const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + W_BYTES);
+                    // (the instruction has 128 token rows; those after `rows` are whatever lies there, and so are their logits)
+                    const uint32_t sa = smem_u32(tiles + s * stage_bytes);
+                    const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + rows * 128);
                     const int acc = kFine ? (kb - kb0) / acc_slices : 0;
                     const bool first = kb - kb0 == acc * acc_slices;
                     const uint32_t d = tmem_base + (uint32_t)(acc % kAccs * PXT);
@@ -303,6 +310,10 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         else umma_bf16(d, da + 2 * k, db + 2 * k, idesc, (!first || k != 0) ? 1u : 0u);
                     }
                     umma_commit(&ctl->empty[s]);
+                    if (++s == (uint32_t)stages) {
+                        s = 0;
+                        ph ^= 1;
+                    }
                 }
                 if (ok) umma_commit(&ctl->acc_full);
             }
@@ -310,7 +321,7 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         }
         if (tid == 96 && round == 0 && a.ahead != nullptr && mbar_wait(&ctl->acc_full, 0, wait_cycles, abort_flag)) bring_ahead();
         __syncwarp();
-        // ---------------------------------------------------------- partial logits to the blocks that own the tokens
+        // ---------------------------------------------------------- logits, or partial ones to the blocks that own the tokens
         if (warp >= 4 && warp < 12) {
             const int q = warp & 3, half = (warp - 4) >> 2;
             const int row = q * 32 + lane, owner = row / own;
@@ -336,7 +347,7 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 // (the operand stages, where the rows on their way out go, are free after the last filling only)
                 const bool last = f + 1 == fills;
 #pragma unroll (kFine ? PXT / 32 : 1)
-                for (int c = 0; c < PXT / 2; c += 16) {
+                for (int c = 0; c < PXT / 2 && (kSplit || q * 32 < own); c += 16) {
                     uint32_t v[16];
                     tmem_ld_32x16(taddr + c, v);
                     tmem_ld_wait();
@@ -367,9 +378,11 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 }
             }
             tc_fence_before();
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            asm volatile("bar.sync 1, 256;" ::: "memory");
+            if (kSplit) {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+            }
             if (tid == 128 && !*abort_flag && !(kFine && a.withhold && me == 0))
                 for (int p = 1; p < C; ++p) {
                     const int to = (me + p) % C;
@@ -388,7 +401,7 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         // (Loops that are short in code: this runs once per launch, and the time of straight-line code
         // is that of fetching it.  With the four threads' logits in registers and all loops unrolled
         // the step took 4.0 us at 64 experts and 8.5 at 128.)
-        const int tok = tid >> 2, sub = tid & 3, t = rt * BM + me * own + tok;
+        const int tok = tid >> 2, sub = tid & 3, tok0 = rt * (int)rows + me * own, t = tok0 + tok;
         if (warp < own / 8) {  // whole warps: eight tokens each
             float* l = recv + (size_t)tok * LD + sub * PER;  // first part of K; the token's logits from here on
             float val[KC + 1];
@@ -475,28 +488,41 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 v.y = e0 + 1 < E ? __expf(v.y - m) : 0.f;
                 v.z = e0 + 2 < E ? __expf(v.z - m) : 0.f;
                 v.w = e0 + 3 < E ? __expf(v.w - m) : 0.f;
-                const float four = (v.x + v.y) + (v.z + v.w);
-                if (kFine) d_rest += add_rest(d, four);
-                d += four;
+                if (kSplit) {
+                    const float four = (v.x + v.y) + (v.z + v.w);
+                    if (kFine) d_rest += add_rest(d, four);
+                    d += four;
+                }
                 *reinterpret_cast<float4*>(l + i) = v;
             }
+            if (kSplit) {
 #pragma unroll
-            for (int o = 1; o < 4; o <<= 1) {
-                const float other = __shfl_xor_sync(0xffffffffu, d, o);
-                if (kFine) d_rest += __shfl_xor_sync(0xffffffffu, d_rest, o) + add_rest(d, other);
-                d += other;
+                for (int o = 1; o < 4; o <<= 1) {
+                    const float other = __shfl_xor_sync(0xffffffffu, d, o);
+                    if (kFine) d_rest += __shfl_xor_sync(0xffffffffu, d_rest, o) + add_rest(d, other);
+                    d += other;
+                }
+                if (kFine) d += d_rest;  // (mCw is a 32-bit result: its sums and its quotient are rounded once each)
+            } else {
+                // in the order of the experts, as the persistent kernel adds them
+                __syncwarp();
+                const float* x = l - sub * PER;
+#pragma unroll 4
+                for (int i = 0; i < PXT; i += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(x + i);
+                    d += v.x; d += v.y; d += v.z; d += v.w;
+                }
             }
-            if (kFine) d += d_rest;  // (mCw is a 32-bit result: its sums and its quotient are rounded once each)
             const float inv = 1.f / d;
             if (sub == 0 && t < S && !*abort_flag) {
-                float w[KC];
+                float w[KC], in_order = 0.f;
 #pragma unroll
                 for (int j = 0; j < KC; ++j) {
-                    const float x = j < K ? __expf(scr->sel_v[tok][j] - m) : 0.f;
-                    w[j] = kFine ? x : __fmul_rn(x, inv);
+                    w[j] = j < K ? __expf(scr->sel_v[tok][j] - m) : 0.f;
+                    if (!kSplit && j < K) in_order = __fmaf_rn(w[j], inv, in_order);
+                    if (kWide) w[j] = __fmul_rn(w[j], inv);
                 }
-                const float chosen = pair_sum(w);
-                a.r.mcw[t] = kFine ? __fdiv_rn(chosen, d) : chosen;
+                a.r.mcw[t] = kFine ? __fdiv_rn(pair_sum(w), d) : kWide ? pair_sum(w) : in_order;
 #pragma unroll 1
                 for (int j = 0; j < K; ++j) {
                     const int e = scr->sel_i[tok][j];
@@ -556,7 +582,7 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             a.r.col_partial[(size_t)row * PXT + tid - 128] = sum;
         }
         if (a.place.slots != nullptr)
-            place_tokens(a.place, ctl->launch, row, n_rt * C, rt * BM + me * own, own, ctl->top, ctl->hist, &scr->place, abort_flag, a.status);
+            place_tokens(a.place, ctl->launch, row, n_rt * C, tok0, own, ctl->top, ctl->hist, &scr->place, abort_flag, a.status);
         if (rt + n_clusters < n_rt) {
             // another round: every block of the cluster is done with the partial logits it received, and the
             // operand stages are handed back to the TMA

@@ -142,6 +142,7 @@ extern "C" int kleos_route_static(const void* A, const void* Wg, const float* ga
         sp.withhold = here.withhold;
         const int slices = H / 64;
         sp.parts = slices >= 4 ? 4 : slices >= 2 ? 2 : 1;
+        sp.own = route_split::BM / sp.parts;
         sp.acc_slices = 1;
         cudaLaunchConfig_t lc{};
         lc.gridDim = dim3((unsigned)((S + route_split::BM - 1) / route_split::BM * sp.parts));

@@ -109,7 +109,7 @@ __device__ __forceinline__ float apply_act(float z, int hidden_act) {
     return 0.5f * z * (1.f + erff(z * 0.70710678118654752f));
 }
 
-// w[0] + .. + w[N - 1], halves onto halves: the order in which the routers add the winning probabilities
+// w[0] + .. + w[N - 1], halves onto halves
 template <int N>
 __device__ __forceinline__ float pair_sum(float (&w)[N]) {
     static_assert((N & (N - 1)) == 0, "a power of two");

@@ -4,11 +4,13 @@
 // thousands of columns; the rows an expert gets are any number, and N takes any multiple of 32.  So
 // the work done for padding is below 32 rows of an expert, and an expert's weights are read once for
 // every 256 or 288 of its rows.  With the rows on M, 128 a block, every tile cost as much as one of 256 rows.
+// (That is with one source rank.  With several, a tile is two panels of up to 128 rows of one or two sources, and takes
+// twice the rows of the larger one; an expert's odd last panel is one tile, half of which is discarded.)
 // What bounds it: the weight stream from HBM up to about 256 rows an expert (128 tokens, 64 experts,
 // H = I = 2048: 537 MB of weights in 85 us = 6.3 TB/s, where plain loads reach 6.2; before 106 and 115 us
 // a launch), above that the tensor pipe, in steady state at the clock the power limit leaves (4096 tokens,
-// H = 4096, I = 14336, 8 experts: 614 us = 1.57 PFLOP/s alone, both GEMMs and the rest 1538 us one after the
-// other, before 1565).  16384 tokens on 128 experts of Zipf popularity: 135 + 143 us -> 103 + 112.
+// H = 4096, I = 14336, 8 experts: 600 us = 1.6 PFLOP/s alone; forwards one after the other take 1520 to 1580, as
+// they did with the rows on M).  16384 tokens on 128 experts of Zipf popularity: 135 + 143 us -> 96 + 95.
 //
 // Tile = (local expert, 256 columns, up to 288 rows).  Each block TMA-loads 128 weight rows (A) and half
 // of the token rows (B), 64 wide K slices through a ring of six.  Accumulators are a ring in
@@ -31,9 +33,9 @@
 //               16 rows at a time in turn; arrive on the LEADER's `slot_empty`
 //   warps 12..15  gathering form only: token rows by index
 // Work and epilogue semantics follow the reference's tile worker (os/processor/processor.cuh:
-// 350-489,706-741).  Every wait is bounded.  This kernel runs one GEMM over a finished panel
-// list (the dense single-expert layer, and the routed layer when its phases are launched one
-// by one).
+// 350-489,706-741).  Every wait is bounded.  This kernel runs one GEMM over rows whose places are
+// known when it starts: those of each expert by count (one source rank, and the dense single-expert layer, whose
+// rows are all of one expert), or a list of panels (several ranks).
 //
 // Element types: bf16, fp16, and TF32 words (kind::tf32, torch_dtype 1; the reference's mma.sync
 // m16n8k8 block GEMM, os/processor/mmaConfig.cuh:73-81).  A K slice is 128 bytes of a row and four
@@ -242,7 +244,8 @@ __device__ __forceinline__ void arrive_relaxed(uint32_t cluster_addr) {
 // the cells, so that on one rank nobody copies them there (a layer of 8192 tokens, k = 2, 4 KiB rows: 13 us
 // of the router's 43, and 64 MB written and read back).  Four warps issue the copies: 128 rows take 0.33 us,
 // which a weight stream from HBM hides (0.4 us a slice) and the tensor pipe at 256 rows a tile does not
-// (0.26 us); one warp took 1.06.
+// (0.26 us); one warp took 1.06.  Up to 256 rows an expert it pays all the same, by what the router then does not copy:
+// see State::gather.
 template <typename TE, int kEpi, bool kGather>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_tc2::kBlock<kGather>, 1)
 ffn_gemm_tc2(const __grid_constant__ gemm_tc2::RowMaps map_x, const __grid_constant__ CUtensorMap map_w, GemmArgs g) {

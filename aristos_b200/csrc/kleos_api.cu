@@ -396,7 +396,8 @@ int with_route_split(F f) {
 
 // Expert weights that the router brings into L2 (126 MB, which also holds the layer's rows): 64 MB are ten
 // microseconds of HBM.  GEMM1 of a decode step of 128 tokens, 64 experts, took 102 us without and 88 with.
-// Every block of the chip issues its share: left to the four with tokens it took the router 98 us.
+// Every block of the chip issues its share: left to the four with tokens it took the router 98 us.  (They are those
+// of the first experts, whatever the gate bias: of an expert that gets no token they are brought in vain.)
 constexpr size_t kAheadBytes = (size_t)64 << 20;
 
 // How the router's work is spread.  16-bit layers: 32, 64 or 128 tokens a block, the fewest with which the chip holds
@@ -521,8 +522,8 @@ struct Staging {
 };
 
 // num_experts == 1: out = (act(A W1^T + b1)) W2^T + b2 over this rank's S tokens, both GEMMs by
-// the expert-FFN kernels in their local-output mode over a fixed panel list (one panel per 128
-// tokens, written once at initialisation).  Follows the reference's dense kernel
+// the expert-FFN kernels in their local-output mode (the float ones over a panel list of 128 tokens each,
+// written once at initialisation).  Follows the reference's dense kernel
 // (moe/fffn.cuh:31-167): intermediate rounded to the element type, identity epilogue on the
 // second GEMM, no gate, no scaling.
 template <typename T>
@@ -612,7 +613,7 @@ int forward_typed(const void* iP, void* oP, cudaStream_t st, bool timed, const S
         if (!g.use_tc && !g.use_tf32_tc) { pl.panels = g.panels; pl.le_start = g.le_start; }
     }
     if (split) {
-        // gate GEMM, top-k, near-ties, slots, counts and the panel list in one launch
+        // gate GEMM, top-k, near-ties, slots and counts in one launch
         if constexpr (!std::is_same<T, float>::value) {
             route_split::Args sp{};
             sp.r = ra; sp.place = pl; sp.status = g.status; sp.own = g.route_own; sp.parts = g.route_parts;
@@ -1086,7 +1087,12 @@ static int initialize_impl(const char* config_json_path, int rank, int world, co
     const char* dk = std::getenv("KLEOS_DISPATCH_KERNELS");
     g.local = world == 1 && !g.use_flow && !(dk && dk[0] == '1');
     // The rows are fetched by index where the weights' way from HBM hides it (see ffn_gemm_tc2): up to 256 rows
-    // an expert on average.  KLEOS_GATHER=0 copies them to the cells there too.
+    // an expert on average.  KLEOS_GATHER=0 copies them to the cells there too.  us per forward, bf16 unless said
+    // otherwise, fetched / copied: H = I = 2048, 128 rows an expert 231 / 241, 192 rows 283 to 299 / 291, 256 rows
+    // 158 to 172 / 166 to 174 (32 experts), 322 to 333 / 307 to 335 (64); H = 4096, I = 1024: 260 / 285, 320 / 349,
+    // 188 / 200, 371 / 392; H = 1024, I = 4096: 245 / 260, 276 / 288, 167 / 167, 336 / 323; TF32, H = I = 2048: 456 / 478,
+    // 540 / 562, 329 / 341.  So at 256 rows the two are about even, and above, a tile's copies take
+    // longer than its MMAs.
     const char* gt = std::getenv("KLEOS_GATHER");
     g.gather = g.local && g.split_route && (long long)cfg.S * cfg.K <= 256LL * cfg.E && !(gt && gt[0] == '0');
     const char* fr = std::getenv("KLEOS_FUSE_ROUTE");

@@ -32,75 +32,6 @@ struct RouteArgs {
     float* col_partial;
 };
 
-// One token's routing decision from its fp32 logits (in shared memory):
-// a single ascending pass keeps the K+1 largest logits in order (strict '>' on insertion, so
-// equal values keep the lower expert id in front -- the reference's tie rule,
-// moe/gate.cuh:662-667), a second pass sums the exponentials.  Writes top-k ids and the sum of
-// the k winning probabilities, and returns the softmax statistics and the k-th / (k+1)-th
-// margin used to decide whether the token needs the fp64 re-evaluation.
-struct RowDecision {
-    float max, inv_den, kth, margin;
-};
-
-// KT is a compile-time bound on K: the insertion chain is KT+1 registers long, so a top-2
-// layer does not pay for the eight-deep chain of the largest supported k.
-template <int KT>
-__device__ __forceinline__ RowDecision decide_row_k(const float* l, int E, int K, int* topk_out,
-                                                    float* mcw_out) {
-    float val[KT + 1];
-    int idx[KT + 1];
-#pragma unroll
-    for (int j = 0; j <= KT; ++j) {
-        val[j] = -INFINITY;
-        idx[j] = 0;
-    }
-    for (int e = 0; e < E; ++e) {
-        float v = l[e];
-        int id = e;
-#pragma unroll
-        for (int j = 0; j <= KT; ++j) {
-            if (j <= K && v > val[j]) {
-                const float tv = val[j];
-                const int ti = idx[j];
-                val[j] = v;
-                idx[j] = id;
-                v = tv;
-                id = ti;
-            }
-        }
-    }
-    const float m = val[0];
-    float d = 0.f;
-    for (int e = 0; e < E; ++e) d += __expf(l[e] - m);
-    const float inv = 1.f / d;
-    float w = 0.f, kth = 0.f, next = -INFINITY;
-#pragma unroll
-    for (int j = 0; j <= KT; ++j) {
-        if (j < K) {
-            topk_out[j] = idx[j];
-            w += __expf(val[j] - m) * inv;
-            kth = val[j];
-        } else if (j == K) {
-            next = val[j];
-        }
-    }
-    *mcw_out = w;
-    RowDecision r;
-    r.max = m;
-    r.inv_den = inv;
-    r.kth = kth;
-    r.margin = (K < E) ? kth - next : INFINITY;
-    return r;
-}
-
-__device__ __forceinline__ RowDecision decide_row(const float* l, int E, int K, int* topk_out,
-                                                  float* mcw_out) {
-    if (K <= 1) return decide_row_k<1>(l, E, K, topk_out, mcw_out);
-    if (K <= 2) return decide_row_k<2>(l, E, K, topk_out, mcw_out);
-    if (K <= 4) return decide_row_k<4>(l, E, K, topk_out, mcw_out);
-    return decide_row_k<kMaxTopK>(l, E, K, topk_out, mcw_out);
-}
-
 // ---------------------------------------------------------------- router on the FP32 pipes
 // Float layers, layers of more than 128 experts, and kleos_route_static on float.  Bound by the FP32
 // FMA rate and L2: S * H * PX multiply-adds (4096 tokens, H = 2048, 64 experts: 15 us on all SMs).  One

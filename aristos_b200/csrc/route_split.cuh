@@ -2,27 +2,31 @@
 // softmax, top-k, near-tie re-evaluation, slots, counts and, on one rank, the rows' way into the cells.
 //
 // What bounds it is latency: the bytes and multiply-adds take 5 us at most on the largest layers and
-// next to nothing on the others, while one block that walks all of K, then thread by thread
-// over the experts of its tokens, then through grid barriers, takes 30 to 40.  So every step is spread:
-//   * a cluster of C = 1, 2 or 4 blocks shares 128 tokens, each block multiplying its part of K (the most
-//     blocks that the chip holds at once, Args::parts), and exchanges partial logits through
-//     distributed shared memory, one bulk copy per pair of blocks (16-byte stores from tensor memory to
-//     the other block took 4 us): block r gets all parts of the tokens [r, r + 1) * 128 / C and adds
-//     them in order of K;
+// next to nothing on the others, while 128 tokens a block, then thread by thread over the experts of its tokens,
+// then through grid barriers, take 30 to 40.  So every step is spread:
+//   * 16-bit layers: a block has 32, 64 or 128 tokens to itself, the fewest with which the chip holds all blocks, and
+//     walks all of K for them with up to fourteen slices in flight.  Every logit is one sum over K, and the
+//     softmax sum goes by experts, so a token's results do not depend on the size of the layer, and they are the bits
+//     of the persistent kernel (moe_flow.cuh);
+//   * TF32 layers and kleos_route_static (kSplit): a cluster of C = 1, 2 or 4 blocks shares 128 tokens, each block
+//     multiplying its part of K (Args::parts), and exchanges partial logits through distributed shared memory,
+//     one bulk copy per pair of blocks (16-byte stores from tensor memory to the other block took 4 us): block r
+//     gets all parts of the tokens [r, r + 1) * 128 / C and adds them in order of K.  (16-bit layers did so
+//     too, and took 20.9 instead of 23.9 us in a decode step, 47.5 instead of 54.1 at H = 4096, 30.2 instead of
+//     29.4 at 8192 tokens, H = 2048: with bits that changed with the number of tokens.)
 //   * four threads per token, each with a quarter of the experts, do softmax and top-k;
 //   * slots without a grid barrier: place_tokens(), route.cuh.
-// Measured, router and row copy, alone and cold: 256 tokens, 8 experts 28 us -> 15; 8192 tokens, 64 experts
-// 54 -> 43 (29 where GEMM1 gathers the rows); 16384 tokens, 128 experts 67 -> 61 (45); of the 128 tokens of a
-// decode step, 64 experts, 39 -> 25 with 64 MB of weights brought into L2 meanwhile.
+// Measured, router and row copy, alone and cold (before: the persistent kernel's routing phase and a copy kernel): 256
+// tokens, 8 experts 28 us -> 15; 8192 tokens, 64 experts 54 -> 43 (29 where GEMM1 gathers the rows); 16384 tokens,
+// 128 experts 67 -> 60 (40); of the 128 tokens of a decode step, 64 experts, 39 -> 24 with 64 MB of weights brought
+// into L2 meanwhile.
 // A block only waits for blocks of lower index and for its own cluster; the host launches no more
-// clusters than the device holds at once.
+// blocks than the device holds at once.
 //
 // Selection rules are those of route.cuh / moe/gate.cuh:556-718: softmax over the E real experts, the k
 // largest with ties to the lowest id, mCw = sum of the k winning probabilities; tokens whose k-th and
 // (k+1)-th logits are closer than fp32 summation error can move them have the experts in that
-// distance of the k-th re-evaluated in fp64.  The routing phase of the persistent kernel (moe_flow.cuh)
-// adds the same parts of K, and the exponentials by the same quarters, in the same order: the two give
-// the same bits.
+// distance of the k-th re-evaluated in fp64.
 #pragma once
 
 #include <cuda.h>
@@ -34,11 +38,10 @@ namespace kleos {
 namespace route_split {
 
 constexpr int BM = 128, kThreads = 512, kWarps = kThreads / 32, kMaxParts = 4, kMaxStages = 14;
-constexpr int W_BYTES = BM * 128;  // one 128-byte K slice of the tokens
 
 template <int PXT>
 struct Shape {
-    static constexpr int STAGE_BYTES = W_BYTES + PXT * 128;
+    static constexpr int STAGE_BYTES = BM * 128 + PXT * 128;  // one 128-byte K slice of 128 tokens and of the gate weight
     static constexpr int STAGES = PXT == 64 ? 7 : 4;
     static constexpr int LD = PXT + 4;                          // floats of a row of partial logits
     static constexpr int RECV_BYTES = BM * LD * 4;              // [parts][128 / parts][LD]
@@ -116,8 +119,8 @@ __device__ __forceinline__ double dot64(const TE* x, const TE* w, int H, int lan
 // within eps of the k-th logit are re-evaluated in fp64 and the open places of the top-k are filled from
 // them (larger value first, equal values to the lower id).  Experts further above are in the set and
 // experts further below are out of it whatever the summation order.  keep64: the band's logits are replaced by
-// the fp64 ones, from which the probabilities and mCw then come (all callers but the inference of 16-bit layers, which
-// gives the bits of the persistent kernel).
+// the fp64 ones, from which the probabilities and mCw then come (kleos_route_static and 16-bit training layers; 16-bit
+// inference gives the bits of the persistent kernel, and TF32 layers keep the fp32 logits' too).
 template <typename TE>
 __device__ __noinline__ void settle_near_ties(unsigned flagged, float* logits, int ld, int E, int K, float kth, float eps,
                                               const TE* A, int t, const TE* Wg, int H, const float* bias, Scratch* scr,
@@ -170,8 +173,9 @@ __device__ __noinline__ void settle_near_ties(unsigned flagged, float* logits, i
 
 }  // namespace route_split
 
-// PXT: padded expert count; KT: compile-time top-k (0: read it from the arguments); kFine: Args::acc_slices
-// (a layer's router sums a block's slices in one accumulator: the code for more cost 256 tokens 0.6 of 30 us).
+// PXT: padded expert count; KT: compile-time top-k (0: read it from the arguments); kFine: kleos_route_static, whose
+// mCw is a 32-bit result: Args::acc_slices, compensated sums (a layer's router sums a block's slices in one accumulator: the
+// code for more cost 256 tokens 0.6 of 30 us).
 template <typename TE, int PXT, int KT, bool kFine = false>
 __global__ void __launch_bounds__(route_split::kThreads, 1)
 route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_wg, route_split::Args a) {
@@ -478,7 +482,7 @@ route_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             const unsigned flagged = __ballot_sync(0xffffffffu, sub == 0 && t < S && K < E && (kth - next) < eps && !*abort_flag);
             if (flagged)
                 settle_near_ties<TE>(flagged, recv, LD, E, K, kth, eps, A, t, Wg, H, ctl->bias, scr, tok,
-                                     kWide || kFine || a.r.col_partial != nullptr);
+                                     kFine || (!kWide && a.r.col_partial != nullptr));
             float d = 0.f, d_rest = 0.f;
 #pragma unroll 1
             for (int i = 0; i < PER; i += 4) {

@@ -1,4 +1,5 @@
-"""Near-tie tokens: probabilities and mCw come from 64-bit logits.  Two experts, whose gate rows are alike but for one
+"""Near-tie tokens of kleos_route_static on bf16 and of 16-bit training layers: probabilities and mCw come from 64-bit
+logits.  Two experts, whose gate rows are alike but for one
 small entry, and products of 2^8 that cancel: the fp32 sum loses about 2^-16 of the small difference, while the 64-bit
 one keeps it.  mCw is the larger of two probabilities next to 1/2, so a 32-bit softmax of exact logits of
 magnitude below 2^-7 is right to 2^-22: logits and their difference are exact to 2^-31, the exponentials near 1, their
@@ -40,7 +41,7 @@ def test_static():
     assert np.abs(mcw.cpu().numpy().astype(np.float64) - want).max() <= 2.0 ** -22
 
 
-@pytest.mark.parametrize("dtype,train", [(1, 0), (2, 1), (3, 1)], ids=["tf32", "bf16-training", "fp16-training"])
+@pytest.mark.parametrize("dtype,train", [(2, 1), (3, 1)], ids=["bf16-training", "fp16-training"])
 def test_layer(dtype, train):
     cfg = KleosConfig(sequence_len=256, hidden_size=256, intermediate_size=64, num_experts=2, expert_top_k=1,
                       torch_dtype=dtype, is_training=train, drop_tokens=0)

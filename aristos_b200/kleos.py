@@ -197,7 +197,8 @@ def gemm_stats():
 
 def route_static(A, Wg, gate_bias, S, H, E, K, torch_dtype, probs, topk, mcw, stream=None) -> None:
     """Router without any device allocation (fixed scratch inside the library): see
-    kleos_route_static in include/kleos_b200.h for limits and the no-overlap rule."""
+    kleos_route_static in include/kleos_b200.h for limits, the float calls' no-overlap rule and what a
+    wait that runs out leaves in topk and mcw."""
     lib = load_library()
     lib.kleos_route_static.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p] + \
         [ctypes.c_int] * 5 + [ctypes.c_void_p] * 4
